@@ -372,8 +372,9 @@ int mg_shape_box_levelset(mg_grid phi, const float* p0, const float* p1);
  * pressure solve is the reference's GridCg with PcMIC: MIC(0) for 3D scenes
  * with (int)(cgMaxIterFac * max size) iterations at most, no preconditioner
  * for 2D scenes with 4 times as many (conjugategrad.cpp:315-321,
- * pressure.cpp:407-419).  Once the CG tile height is tuned, the sweeps run
- * as CUDA graphs of 8 sweeps between convergence polls. */
+ * pressure.cpp:407-419).  A 2D scene that fits a thread-block cluster (up to
+ * 512 x 512 cells) is solved by one launch of its own; the other scenes'
+ * sweeps run as CUDA graphs of 8 sweeps between convergence polls. */
 typedef struct mg_batch_s* mg_batch;
 typedef struct {
   int sweeps;                  /* CG iterations launched (the slowest scene's count) */
@@ -415,7 +416,7 @@ int mg_batch_download(mg_batch b, int scene, int what, void* host, size_t bytes)
  * cell (host computation, for feeding the same inflow to a single scene) */
 int mg_batch_noise(unsigned long long seed, int step, long long cells, float* out);
 int mg_batch_info(mg_batch b, int* count, long long* cells, long long* tiles, size_t* bytes);
-/* the CG sweep tile height the batch's autotuner chose on its first solve
+/* the CG sweep tile height the batch's autotuner chose over its first solves
  * (0 before) and the four timings (ms per lag sweeps, 8/16/32/64 rows) */
 int mg_batch_tuning(mg_batch b, int* sweepRows, float* ms);
 int mg_batch_sync(mg_batch b);

@@ -93,6 +93,14 @@ struct GraphKey {
   }
 };
 
+// scenes solved by cluster launches of one shape
+struct ClusterGroup {
+  CgClusterPlan plan;
+  bool a0;
+  int first, count;  // their entries in the table of cluster scenes
+};
+constexpr int kSideStreams = 4;
+
 struct Engine {
   cudaStream_t stream = nullptr;
   float dt = 1.f;
@@ -131,6 +139,15 @@ struct Engine {
   GraphKey graphKey{};
   unsigned long long graphNodes = 0;
   long long graphLaunches = 0;
+  // 2D scenes whose solve is one cluster launch (cgcluster.cu), by launch
+  // shape; the launches run beside the sweeps of the other scenes
+  std::vector<char> onCluster;  // per member
+  std::vector<ClusterGroup> groups;
+  std::vector<CgClusterScene> hCluster;
+  CgClusterScene* dCluster = nullptr;
+  size_t clusterCap = 0;
+  cudaStream_t side[kSideStreams] = {};
+  cudaEvent_t fork = nullptr, join[kSideStreams] = {};
   std::vector<BTile> tiles1;
   std::vector<BTile> tilesDam;  // the 32 x 8 tiles of the dam-break scenes
   BTile* dTilesDam = nullptr;
@@ -142,13 +159,17 @@ struct Engine {
   BTile* dActive = nullptr;
   size_t activeCap = 0;
   bool dirty = true;
-  int rowsK = -1;
+  int rowsK = -1;      // the tuned tile height; -1 while tuning
+  int tuneK = 0;       // the height timed next
+  int tuneSpoilt = 0;  // timings dropped because a scene finished during them
   float tuneMs[4] = {0.f, 0.f, 0.f, 0.f};
   cudaEvent_t ev[2] = {nullptr, nullptr};
   int* dDone = nullptr;
 
   ~Engine() {
     if (stream) cudaStreamSynchronize(stream);
+    for (auto st : side)
+      if (st) cudaStreamSynchronize(st);
     for (auto* m : members) {
       cudaFree(m->mem);
       cudaFree(m->refMem);
@@ -165,6 +186,12 @@ struct Engine {
     cudaFree(dOrder2);
     cudaFree(dMicScene);
     cudaFree(dMicCounter);
+    cudaFree(dCluster);
+    for (int q = 0; q < kSideStreams; q++) {
+      if (join[q]) cudaEventDestroy(join[q]);
+      if (side[q]) cudaStreamDestroy(side[q]);
+    }
+    if (fork) cudaEventDestroy(fork);
     if (sweepGraph) cudaGraphExecDestroy(sweepGraph);
     if (ev[0]) cudaEventDestroy(ev[0]);
     if (ev[1]) cudaEventDestroy(ev[1]);
@@ -177,6 +204,11 @@ int engine_init(Engine& e, float dt) {
   CKB(cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking));
   CKB(cudaEventCreate(&e.ev[0]));
   CKB(cudaEventCreate(&e.ev[1]));
+  CKB(cudaEventCreateWithFlags(&e.fork, cudaEventDisableTiming));
+  for (int q = 0; q < kSideStreams; q++) {
+    CKB(cudaStreamCreateWithFlags(&e.side[q], cudaStreamNonBlocking));
+    CKB(cudaEventCreateWithFlags(&e.join[q], cudaEventDisableTiming));
+  }
   CKB(cudaMalloc(&e.dDone, sizeof(int)));
   CKB(cudaMalloc(&e.dMicCounter, 3 * sizeof(int)));
   CKB(cudaMemset(e.dMicCounter, 0, 3 * sizeof(int)));
@@ -441,6 +473,34 @@ int engine_tables(Engine& e) {
     CKB(cudaMemcpyAsync(e.dMicScene, e.hMicScene.data(), sizeof(int) * e.hMicScene.size(), cudaMemcpyHostToDevice,
                         e.stream));
   }
+  // 2D scenes that fit a cluster, grouped by launch shape, the longest
+  // strips first
+  e.onCluster.assign(nm, 0);
+  e.groups.clear();
+  e.hCluster.clear();
+  std::map<std::pair<int, int>, std::vector<std::pair<size_t, CgClusterPlan>>> shapes;
+  for (size_t q = 0; q < nm; q++) {
+    const BScene& b = e.hScenes[q];
+    CgClusterPlan pl;
+    if (b.mic || !cg_cluster_plan(b.d, b.A0f != nullptr, &pl)) continue;
+    e.onCluster[q] = 1;
+    shapes[{-pl.k, -(2 * pl.ctas + (b.A0f ? 1 : 0))}].push_back({q, pl});
+  }
+  for (auto& kv : shapes) {
+    ClusterGroup g{kv.second[0].second, e.hScenes[kv.second[0].first].A0f != nullptr, (int)e.hCluster.size(),
+                   (int)kv.second.size()};
+    for (auto& m : kv.second) {
+      const BScene& b = e.hScenes[m.first];
+      g.plan.smem = std::max(g.plan.smem, m.second.smem);
+      e.hCluster.push_back(CgClusterScene{b.d.nx, b.d.ny, m.second.rows, 0.f, b.code, b.A0f, b.rhs, b.pres, b.sc});
+    }
+    e.groups.push_back(g);
+  }
+  if (!e.hCluster.empty()) {
+    if (ensure_cap(&e.dCluster, &e.clusterCap, e.hCluster.size())) return MG_ERR_CUDA;
+    CKB(cudaMemcpyAsync(e.dCluster, e.hCluster.data(), sizeof(CgClusterScene) * e.hCluster.size(),
+                        cudaMemcpyHostToDevice, e.stream));
+  }
   if (ensure_cap(&e.dTiles, &e.tilesCap, e.tiles1.size()) || ensure_cap(&e.dActive, &e.activeCap, e.tiles1.size()))
     return MG_ERR_CUDA;
   CKB(cudaMemcpyAsync(e.dTiles, e.tiles1.data(), sizeof(BTile) * e.tiles1.size(), cudaMemcpyHostToDevice, e.stream));
@@ -491,29 +551,36 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
     c.maxIter = (int)(e.cgMaxIterFac * (float)std::max(d.nx, std::max(d.ny, d.nz))) * (d.is3d ? 1 : 4);
     c.resNorm = 1e20f;
     c.refNorm = e.hSc[q].refNorm;
-    if (skip[q]) {
-      c.done = 1;
-      nskip++;
-    }
+    if (skip[q]) c.done = 1;
+    if (skip[q] || e.onCluster[q]) nskip++;
     e.hSc[q] = c;
-    if (!skip[q]) maxIterAll = std::max(maxIterAll, c.maxIter);
+    if (!skip[q] && !e.onCluster[q]) maxIterAll = std::max(maxIterAll, c.maxIter);
   }
   CKB(cudaMemcpyAsync(e.dSc, e.hSc.data(), sizeof(CgScalars) * nm, cudaMemcpyHostToDevice, st));
   CKB(cudaMemcpyAsync(e.dDone, &nskip, sizeof(int), cudaMemcpyHostToDevice, st));
   launch_b_pcg_init(e.dTiles, nt, e.dScenes, st);
+  // the cluster scenes' solves, beside everything below
+  const int nside = std::min((int)e.groups.size(), kSideStreams);
+  if (nside) CKB(cudaEventRecord(e.fork, st));
+  for (int q = 0; q < nside; q++) CKB(cudaStreamWaitEvent(e.side[q], e.fork, 0));
+  for (size_t q = 0; q < e.groups.size(); q++) {
+    const ClusterGroup& g = e.groups[q];
+    CKB(launch_cg_cluster(g.plan, e.dCluster + g.first, CgClusterScene{}, g.count, g.a0, e.side[q % kSideStreams]));
+  }
+  for (int q = 0; q < nside; q++) CKB(cudaEventRecord(e.join[q], e.side[q]));
   if (mic.nscenes > 0) launch_b_mic_init(e.dTiles, nt, e.dScenes, mic, st);
-  // CG sweeps over the tiles of the scenes still iterating.  Autotuner: the
-  // first solve runs its first 4 x lag sweeps with tiles 8, 16, 32 and 64
-  // rows tall (lag sweeps each, timed with events) and keeps the fastest;
-  // results do not depend on the choice.
-  int kk = e.rowsK >= 0 ? e.rowsK : 0;
+  // CG sweeps over the tiles of the scenes still iterating.  Autotuner: runs
+  // of lag sweeps in which no scene finishes are timed with events, one with
+  // tiles 8, 16, 32 and 64 rows tall each, over as many solves as that takes,
+  // and the fastest is kept; results do not depend on the choice.
+  int kk = e.rowsK >= 0 ? e.rowsK : e.tuneK;
   int active = 0, doneSeen = -1, sweeps = 0;
   (void)nt;
   std::vector<BTile> list;
   auto rebuild = [&](bool all) -> int {
     list.clear();
     for (int q = 0; q < nm; q++)
-      if (all || !e.hSc[q].done)
+      if (!e.onCluster[q] && (all || !e.hSc[q].done))
         list.insert(list.end(), e.tilesR[kk].begin() + e.startR[kk][q], e.tilesR[kk].begin() + e.startR[kk][q + 1]);
     active = (int)list.size();
     if (active) CKB(cudaMemcpyAsync(e.dActive, list.data(), sizeof(BTile) * active, cudaMemcpyHostToDevice, st));
@@ -521,11 +588,10 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
   };
   if (rebuild(false)) return MG_ERR_CUDA;
   const bool tuning = e.rowsK < 0;
-  if (tuning) CKB(cudaEventRecord(e.ev[0], st));
   while (active > 0 && sweeps < maxIterAll) {
-    // once the tile height is tuned, `lag` sweeps run as one CUDA graph,
-    // captured for the current sweep list and captured again when it changes
-    const bool useGraph = !(tuning && e.rowsK < 0) && sweeps % e.lag == 0 && sweeps + e.lag <= maxIterAll;
+    // `lag` sweeps run as one CUDA graph, captured for the current sweep list
+    // and captured again when it changes
+    const bool useGraph = sweeps % e.lag == 0 && sweeps + e.lag <= maxIterAll;
     if (useGraph) {
       const GraphKey key{e.dActive, active, kk, e.dScenes, mic.flow, mic.order, mic.ntiles, mic.nscenes};
       if (!e.sweepGraph || !(key == e.graphKey)) {
@@ -549,6 +615,7 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
         }
         e.graphKey = key;
       }
+      if (tuning && e.rowsK < 0) CKB(cudaEventRecord(e.ev[0], st));  // after the capture, which is host time
       CKB(cudaGraphLaunch(e.sweepGraph, st));
       g_launches.fetch_add(e.graphNodes, std::memory_order_relaxed);
       e.graphLaunches++;
@@ -559,27 +626,26 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
     }
     if (sweeps % e.lag == 0 || sweeps == maxIterAll) {
       bool relist = false;
-      if (tuning && e.rowsK < 0 && sweeps <= 4 * e.lag) {
-        CKB(cudaEventRecord(e.ev[1], st));
-        CKB(cudaEventSynchronize(e.ev[1]));
-        float ms = 0.f;
-        CKB(cudaEventElapsedTime(&ms, e.ev[0], e.ev[1]));
-        e.tuneMs[kk] = ms;
-        if (kk < 3) {
-          kk++;
-          relist = true;
-        } else {
-          int best = 0;
-          for (int q = 1; q < 4; q++)
-            if (e.tuneMs[q] < e.tuneMs[best]) best = q;
-          e.rowsK = best;
-          relist = kk != best;
-          kk = best;
-        }
-      }
+      const bool timing = tuning && e.rowsK < 0 && useGraph;
+      if (timing) CKB(cudaEventRecord(e.ev[1], st));
       int nd = 0;
       CKB(cudaMemcpyAsync(&nd, e.dDone, sizeof(int), cudaMemcpyDeviceToHost, st));
       CKB(cudaStreamSynchronize(st));
+      if (timing && nd == (doneSeen < 0 ? nskip : doneSeen)) {
+        CKB(cudaEventElapsedTime(&e.tuneMs[kk], e.ev[0], e.ev[1]));
+        if (e.tuneK < 3) {
+          kk = ++e.tuneK;
+          relist = true;
+        } else {
+          e.rowsK = (int)(std::min_element(e.tuneMs, e.tuneMs + 4) - e.tuneMs);
+        }
+      } else if (timing && ++e.tuneSpoilt >= 16) {
+        e.rowsK = 0;  // scenes that never run lag sweeps together
+      }
+      if (e.rowsK >= 0 && kk != e.rowsK) {
+        kk = e.rowsK;
+        relist = true;
+      }
       if (nd >= nm) break;
       if (nd != doneSeen || relist) {
         doneSeen = nd;
@@ -587,10 +653,10 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
         CKB(cudaStreamSynchronize(st));
         if (rebuild(false)) return MG_ERR_CUDA;
       }
-      if (tuning && e.rowsK < 0) CKB(cudaEventRecord(e.ev[0], st));
     }
   }
   *sweepsOut = sweeps;
+  for (int q = 0; q < nside; q++) CKB(cudaStreamWaitEvent(st, e.join[q], 0));
   CKB(cudaStreamSynchronize(st));
   return MG_OK;
 }
@@ -664,7 +730,6 @@ int engine_step(Engine& e, mg_batch_stats* stats) {
     m->step++;
   }
   if (stats) {
-    stats->sweeps = sweeps;
     stats->graphLaunches = e.graphLaunches - graphLaunches0;
     int mx = 0, diverged = 0;
     long long sum = 0;
@@ -673,6 +738,7 @@ int engine_step(Engine& e, mg_batch_stats* stats) {
       sum += c.iterations;
       diverged += c.status == 2;
     }
+    stats->sweeps = std::max(sweeps, mx);  // a cluster launch runs its scenes' sweeps itself
     stats->maxIterations = mx;
     stats->totalIterations = sum;
     stats->diverged = diverged;

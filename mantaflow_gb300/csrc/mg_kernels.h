@@ -206,6 +206,30 @@ int pcg_prepare(int sms);
 // sum of nparts per-block dot partials -> beta/sigma (init: sigma only)
 void launch_mic_finish(const PcgBuffers& b, int nparts, bool init, cudaStream_t s);
 
+// unpreconditioned CG of 2D scenes, one thread-block cluster each
+// (cgcluster.cu): rhs -> p, iterations and status in sc (accuracy, maxIter
+// and resNorm set by the caller; a scene with sc->done set is left alone)
+struct CgClusterScene {
+  int nx, ny, rows;  // rows: grid rows per CTA
+  float nanNorm;     // residual norm reported when no residual is a number
+  const code_t* code;
+  const float* A0f;  // ghost-fluid diagonal (launches with a0)
+  const float* rhs;
+  float* p;
+  CgScalars* sc;
+};
+struct CgClusterPlan {
+  int ctas, k, rows;  // CTAs of the cluster, cells per thread, rows per CTA
+  size_t smem;
+};
+int cg_cluster_prepare();
+// the split of a scene, by its size alone; false: it does not fit a cluster
+bool cg_cluster_plan(const Dims& d, bool a0, CgClusterPlan* pl);
+// scenes of one plan (ctas, k; smem the largest): tab in device memory, or
+// one scene by value when tab is null
+cudaError_t launch_cg_cluster(const CgClusterPlan& pl, const CgClusterScene* tab, const CgClusterScene& one, int scenes,
+                              bool a0, cudaStream_t s);
+
 // precision form (refine.cu): FP64 residual refinement around the FP32 PCG
 void launch_to_double(long long n, const float* a, double* b, cudaStream_t s);
 void launch_to_float(long long n, const double* a, float* b, cudaStream_t s);

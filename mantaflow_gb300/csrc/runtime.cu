@@ -3,6 +3,7 @@
 // Owns the CUDA device state of every FluidSolver-equivalent (stream, grid
 // storage pool, CG/MIC state) and translates each mantaflow plugin call into
 // kernel launches on the solver's stream.
+#include <cfloat>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -313,7 +314,7 @@ extern "C" int mg_init(int device) {
   g_ctx.sms = prop.multiProcessorCount;
   g_ctx.micCtasPerSm = mic_ctas_per_sm();
   if (mic_col_prepare() || mic_wave_prepare(&g_ctx.waveCtasPerSm4, &g_ctx.waveCtasPerSm8) ||
-      mic_flow_prepare(&g_ctx.flowCtasPerSm) || pcg_prepare(g_ctx.sms))
+      mic_flow_prepare(&g_ctx.flowCtasPerSm) || pcg_prepare(g_ctx.sms) || cg_cluster_prepare())
     return fail(MG_ERR_CUDA, "mg_init: cannot configure the MIC kernels");
   g_ctx.device = device;
   g_ctx.init = true;
@@ -1339,6 +1340,18 @@ static int mg_iteration_graph(mg_solver s, const PcgBuffers& b) {
   return MG_OK;
 }
 
+// iterations and residual norm of the finished solve (scHost), and its
+// divergence as the reference reports it
+static int solve_outcome(mg_solver s, mg_pressure_result* out) {
+  if (out) {
+    out->iterations = s->scHost->iterations;
+    out->resNorm = s->scHost->resNorm;
+  }
+  if (s->scHost->status == 2)
+    return fail(MG_ERR_SOLVER, "GridCg::iterate: The CG solver diverged, residual norm > 1e30, stopping.");
+  return MG_OK;
+}
+
 extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressure, mg_grid flags,
                                         const mg_pressure_params* p, mg_grid phi, mg_grid perCellCorr, mg_grid fractions,
                                         mg_grid curv, mg_pressure_result* out) {
@@ -1433,6 +1446,19 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
   init.maxIter = maxIter;
   init.resNorm = 1e20f;
   CK(cudaMemcpyAsync(s->sc, &init, sizeof(CgScalars), cudaMemcpyHostToDevice, s->stream));
+  // a 2D scene's whole solve in one cluster launch where it fits one (the
+  // max-abs norm, links of 0 or -1: the other forms take the loop below)
+  CgClusterPlan cc;
+  if (pc == kPcNone && !b.Aif && !p->useL2Norm && cg_cluster_plan(d, b.A0f != nullptr, &cc)) {
+    {
+      ProfScope ps(s, "pcg_cluster");
+      const CgClusterScene one{d.nx, d.ny, cc.rows, FLT_MAX, b.code, b.A0f, b.rhs, b.pressure, b.sc};
+      CK(launch_cg_cluster(cc, nullptr, one, 1, b.A0f != nullptr, s->stream));
+    }
+    CK(cudaMemcpyAsync(s->scHost, s->sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    return solve_outcome(s, out);
+  }
   {
     ProfScope ps(s, "pcg_init");
     launch_pcg_init(b, s->stream);
@@ -1532,12 +1558,8 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
     CK(cudaMemcpy(&err, s->mic.error, sizeof(int), cudaMemcpyDeviceToHost));
     if (err) return fail(MG_ERR_TIMEOUT, "MIC wavefront: a tile wait exceeded its spin limit");
   }
-  if (out) {
-    out->iterations = s->scHost->iterations;
-    out->resNorm = s->scHost->resNorm;
-  }
-  if (s->scHost->status == 2)
-    return fail(MG_ERR_SOLVER, "GridCg::iterate: The CG solver diverged, residual norm > 1e30, stopping.");
+  st = solve_outcome(s, out);
+  if (st) return st;
   if (s->scHost->status == 4) return fail(MG_ERR_TIMEOUT, "PCG: a plane copy of the streamed SpMV exceeded its wait limit");
   if (s->mg && preconditioner == MG_PC_MG_DYNAMIC) mg_hierarchy_reset(s->mg);
   return MG_OK;
