@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -55,17 +56,41 @@ int tiles_of(int nx, int ny, int nz, int rows) { return ((nx + kBTX - 1) / kBTX)
 constexpr int kMicTile = 16;  // edge of the MIC dataflow tiles
 int mic_tiles(int n) { return (n + kMicTile - 1) / kMicTile; }
 
+Dims dims_of(int nx, int ny, int nz) {
+  Dims d;
+  d.nx = nx;
+  d.ny = ny;
+  d.nz = nz;
+  d.is3d = nz > 1;
+  d.n = (long long)nx * ny * nz;
+  d.sy = nx;
+  d.sz = d.is3d ? (long long)nx * ny : 0;
+  return d;
+}
+// bytes of a 3D scene's MIC buffers: what the cluster sweeps need, or the
+// diagonal and face words of the tile sweeps
+size_t mic_bytes(int nx, int ny, int nz) {
+  MicClusterScene m;
+  const size_t n = (size_t)nx * ny * nz;
+  if (!mic_cluster_plan(dims_of(nx, ny, nz), &m))
+    return align256(n * sizeof(float)) +
+           align256(mic_flow_face_words(mic_tiles(nx) * mic_tiles(ny) * mic_tiles(nz)) * sizeof(unsigned long long));
+  const size_t f = mic_cluster_floats(m);
+  size_t b = align256(f * sizeof(float)) + align256(f / 2 * sizeof(unsigned)) + align256(mic_cluster_flag_bytes(m)) +
+             align256(mic_cluster_face_words(m) * sizeof(unsigned));
+  if (2 * f > 4 * n) b += 2 * align256(f * sizeof(float));  // else r and z share advection's scratch
+  return b;
+}
+
 // bytes of one scene's device block (3D scenes also hold the MIC diagonal
-// and the face words of the dataflow sweeps; dam-break scenes the
+// and the words between its sweeps' parts; dam-break scenes the
 // ghost-fluid diagonal and the extrapolation marks)
 size_t scene_bytes(int nx, int ny, int nz, int kind = 0) {
   const size_t n = (size_t)nx * ny * nz;
   size_t b = align256(n * sizeof(int)) + 2 * align256(3 * n * sizeof(float)) + 2 * align256(n * sizeof(float)) +
              align256(4 * n * sizeof(float)) + 6 * align256(n * sizeof(float)) + align256(n * sizeof(code_t)) +
              align256(2 * (size_t)tiles_of(nx, ny, nz, kBTY) * sizeof(double));
-  if (nz > 1)
-    b += align256(n * sizeof(float)) +
-         align256(mic_flow_face_words(mic_tiles(nx) * mic_tiles(ny) * mic_tiles(nz)) * sizeof(unsigned long long));
+  if (nz > 1) b += mic_bytes(nx, ny, nz);
   if (kind == 1) b += align256(n * sizeof(float)) + align256(n * sizeof(int));
   return b;
 }
@@ -75,6 +100,7 @@ struct SceneRec {
   void* mem = nullptr;
   void* refMem = nullptr;  // p64 | b64 of the FP64 refinement, allocated when first used
   size_t bytes = 0;
+  MicClusterScene mc{};    // cluster sweeps (s.mcl)
   int step = 0;  // steps taken: the inflow noise index
   int cur = 0;   // which ping-pong buffers are current
 };
@@ -82,14 +108,17 @@ struct SceneRec {
 // the kernel arguments a captured sweep graph depends on
 struct GraphKey {
   const void* tiles;
-  int active, rowsK;
+  int active, byTile, rowsK;
   const void* scenes;
   const void* flow;
   const void* order;
   int micTiles, micScenes;
+  const void *mc, *jobs;
+  int njobs, mcScenes, mcBlocks, mcLevels;
   bool operator==(const GraphKey& o) const {
-    return tiles == o.tiles && active == o.active && rowsK == o.rowsK && scenes == o.scenes && flow == o.flow &&
-           order == o.order && micTiles == o.micTiles && micScenes == o.micScenes;
+    return tiles == o.tiles && active == o.active && byTile == o.byTile && rowsK == o.rowsK && scenes == o.scenes &&
+           flow == o.flow && order == o.order && micTiles == o.micTiles && micScenes == o.micScenes && mc == o.mc &&
+           jobs == o.jobs && njobs == o.njobs && mcScenes == o.mcScenes && mcBlocks == o.mcBlocks && mcLevels == o.mcLevels;
   }
 };
 
@@ -124,6 +153,17 @@ struct Engine {
   bool refine = false;
   double refineAccuracy = 1e-5, innerAccuracy = 1e-2;
   int maxRefine = 10;
+  // 3D scenes whose MIC(0) runs as cluster sweeps (miccluster.cu): the scene
+  // table, its members, and the jobs of the scenes still iterating
+  std::vector<MicClusterScene> hMc;
+  std::vector<int> mcMember;
+  std::vector<int2> hJobs;
+  MicClusterScene* dMc = nullptr;
+  size_t mcCap = 0;
+  int2* dJobs = nullptr;
+  size_t jobsCap = 0;
+  int mcBlocks = 0, mcLevels = 0;
+  // the others: tile sweeps (micflow.cu)
   std::vector<FlowScene> hFlow;
   std::vector<int2> hOrder2;
   std::vector<int> hMicScene;
@@ -133,7 +173,7 @@ struct Engine {
   size_t orderCap = 0;
   int* dMicScene = nullptr;
   size_t micSceneCap = 0;
-  int* dMicCounter = nullptr;  // [0] tile counter, [1] wait error, [2] sweep epoch
+  int* dMicCounter = nullptr;  // [0] tile counter, [1] wait error, [2] sweep epoch, [3] cluster ticket
   // `lag` CG sweeps captured as a CUDA graph, and what it was captured with
   cudaGraphExec_t sweepGraph = nullptr;
   GraphKey graphKey{};
@@ -187,6 +227,8 @@ struct Engine {
     cudaFree(dMicScene);
     cudaFree(dMicCounter);
     cudaFree(dCluster);
+    cudaFree(dMc);
+    cudaFree(dJobs);
     for (int q = 0; q < kSideStreams; q++) {
       if (join[q]) cudaEventDestroy(join[q]);
       if (side[q]) cudaStreamDestroy(side[q]);
@@ -210,8 +252,8 @@ int engine_init(Engine& e, float dt) {
     CKB(cudaEventCreateWithFlags(&e.join[q], cudaEventDisableTiming));
   }
   CKB(cudaMalloc(&e.dDone, sizeof(int)));
-  CKB(cudaMalloc(&e.dMicCounter, 3 * sizeof(int)));
-  CKB(cudaMemset(e.dMicCounter, 0, 3 * sizeof(int)));
+  CKB(cudaMalloc(&e.dMicCounter, 4 * sizeof(int)));
+  CKB(cudaMemset(e.dMicCounter, 0, 4 * sizeof(int)));
   return MG_OK;
 }
 
@@ -255,13 +297,7 @@ int scene_add(Engine& e, int nx, int ny, int nz, const float* gravity, unsigned 
   e.liveBytes += r->bytes;
   CKB(cudaMemsetAsync(r->mem, 0, r->bytes, e.stream));
   BScene& s = r->s;
-  s.d.nx = nx;
-  s.d.ny = ny;
-  s.d.nz = nz;
-  s.d.is3d = nz > 1;
-  s.d.n = (long long)nx * ny * nz;
-  s.d.sy = nx;
-  s.d.sz = s.d.is3d ? (long long)nx * ny : 0;
+  s.d = dims_of(nx, ny, nz);
   const size_t n = (size_t)s.d.n;
   unsigned char* p = (unsigned char*)r->mem;
   auto take = [&](size_t bytes) {
@@ -289,9 +325,28 @@ int scene_add(Engine& e, int nx, int ny, int nz, const float* gravity, unsigned 
   s.tx = mic_tiles(nx);
   s.ty = mic_tiles(ny);
   s.tz = mic_tiles(nz);
+  s.mcl = 0;
   if (nz > 1) {
-    s.P = (float*)take(n * sizeof(float));
-    s.face = (unsigned long long*)take(mic_flow_face_words(s.tx * s.ty * s.tz) * sizeof(unsigned long long));
+    MicClusterScene& m = r->mc;
+    if (mic_cluster_plan(s.d, &m)) {
+      const size_t f = mic_cluster_floats(m);
+      s.mcl = 1;
+      m.P = (float*)take(f * sizeof(float));
+      m.cw = (unsigned*)take(f / 2 * sizeof(unsigned));
+      m.regular = (unsigned char*)take(mic_cluster_flag_bytes(m));
+      m.gface = (unsigned*)take(mic_cluster_face_words(m) * sizeof(unsigned));
+      if (2 * f > 4 * n) {
+        m.r = (float*)take(f * sizeof(float));
+        m.z = (float*)take(f * sizeof(float));
+      } else {
+        m.r = s.fwd;
+        m.z = s.fwd + f;
+      }
+      CKB(cudaMemsetAsync(m.gface, 0xff, mic_cluster_face_words(m) * sizeof(unsigned), e.stream));
+    } else {
+      s.P = (float*)take(n * sizeof(float));
+      s.face = (unsigned long long*)take(mic_flow_face_words(s.tx * s.ty * s.tz) * sizeof(unsigned long long));
+    }
   }
   s.mic = (nz > 1 && e.micFor3D) ? 1 : 0;
   s.kind = kind;
@@ -437,7 +492,7 @@ int engine_tables(Engine& e) {
   int maxLevel = 0;
   for (size_t q = 0; q < nm; q++) {
     const BScene& b = e.hScenes[q];
-    if (!b.mic) continue;
+    if (!b.mic || b.mcl) continue;
     FlowScene f;
     f.d = b.d;
     f.code = b.code;
@@ -472,6 +527,32 @@ int engine_tables(Engine& e) {
     CKB(cudaMemcpyAsync(e.dOrder2, e.hOrder2.data(), sizeof(int2) * e.hOrder2.size(), cudaMemcpyHostToDevice, e.stream));
     CKB(cudaMemcpyAsync(e.dMicScene, e.hMicScene.data(), sizeof(int) * e.hMicScene.size(), cudaMemcpyHostToDevice,
                         e.stream));
+  }
+  // MIC scenes of the cluster sweeps
+  e.hMc.clear();
+  e.mcMember.clear();
+  e.mcBlocks = e.mcLevels = 0;
+  for (size_t q = 0; q < nm; q++) {
+    const BScene& b = e.hScenes[q];
+    if (!b.mic || !b.mcl) continue;
+    MicClusterScene m = e.members[q]->mc;
+    m.code = b.code;
+    m.A0f = b.A0f;
+    m.rhs = b.rhs;
+    m.p = b.pres;
+    m.s = b.search;
+    m.t = b.tmp;
+    m.part = b.part;
+    m.sc = b.sc;
+    m.nanNorm = 0.f;
+    e.hMc.push_back(m);
+    e.mcMember.push_back((int)q);
+    e.mcBlocks = std::max(e.mcBlocks, m.nby * m.nbz);
+    e.mcLevels = std::max(e.mcLevels, m.nlp);
+  }
+  if (!e.hMc.empty()) {
+    if (ensure_cap(&e.dMc, &e.mcCap, e.hMc.size())) return MG_ERR_CUDA;
+    CKB(cudaMemcpyAsync(e.dMc, e.hMc.data(), sizeof(MicClusterScene) * e.hMc.size(), cudaMemcpyHostToDevice, e.stream));
   }
   // 2D scenes that fit a cluster, grouped by launch shape, the longest
   // strips first
@@ -538,7 +619,7 @@ int engine_refine_buffers(Engine& e) {
 // skipped, each to its own accuracy: PcMIC in 3D with (int)(cgMaxIterFac *
 // max size) iterations at most; in 2D GridCg drops MIC (conjugategrad.cpp:
 // 315-321) and allows 4 times as many.  The right-hand side is in rhs.
-int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, const std::vector<char>& skip,
+int engine_cg(Engine& e, BatchMic& mic, const std::vector<float>& acc, const std::vector<char>& skip,
               int* sweepsOut) {
   const int nm = (int)e.members.size();
   const int nt = (int)e.tiles1.size();
@@ -568,7 +649,36 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
     CKB(launch_cg_cluster(g.plan, e.dCluster + g.first, CgClusterScene{}, g.count, g.a0, e.side[q % kSideStreams]));
   }
   for (int q = 0; q < nside; q++) CKB(cudaEventRecord(e.join[q], e.side[q]));
+  // the jobs of the cluster sweeps: a scene's z-blocks in order, the scenes
+  // taking turns, for those still iterating
+  auto jobs = [&]() -> int {
+    e.hJobs.clear();
+    for (int k = 0, more = 1; more; k++) {
+      more = 0;
+      for (size_t m = 0; m < e.hMc.size(); m++) {
+        const MicClusterScene& c = e.hMc[m];
+        if (e.hSc[e.mcMember[m]].done || k * c.zper >= c.nbz) continue;
+        e.hJobs.push_back(make_int2((int)m, k * c.zper));
+        more = 1;
+      }
+    }
+    mic.mc.njobs = (int)e.hJobs.size();
+    if (e.hJobs.empty()) return MG_OK;
+    if (ensure_cap(&e.dJobs, &e.jobsCap, e.hJobs.size())) return MG_ERR_CUDA;
+    mic.mc.jobs = e.dJobs;
+    CKB(cudaMemcpyAsync(e.dJobs, e.hJobs.data(), sizeof(int2) * e.hJobs.size(), cudaMemcpyHostToDevice, st));
+    return MG_OK;
+  };
+  if (jobs()) return MG_ERR_CUDA;
   if (mic.nscenes > 0) launch_b_mic_init(e.dTiles, nt, e.dScenes, mic, st);
+  if (mic.mc.njobs > 0) {
+    CKB(launch_mic_level(mic.mc, kMicInit, st));
+    CKB(launch_mic_cluster_order(mic.mc, st));
+    CKB(launch_mic_cluster(mic.mc, 0, st));
+    CKB(launch_mic_cluster(mic.mc, 1, st));
+    CKB(launch_mic_cluster(mic.mc, 3, st));
+    CKB(launch_mic_level(mic.mc, kMicSearch, st));
+  }
   // CG sweeps over the tiles of the scenes still iterating.  Autotuner: runs
   // of lag sweeps in which no scene finishes are timed with events, one with
   // tiles 8, 16, 32 and 64 rows tall each, over as many solves as that takes,
@@ -576,31 +686,40 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
   int kk = e.rowsK >= 0 ? e.rowsK : e.tuneK;
   int active = 0, doneSeen = -1, sweeps = 0;
   (void)nt;
+  // sweep list: the tiles of the scenes still iterating, first those whose
+  // vectors are updated tile by tile, then those of the cluster sweeps
   std::vector<BTile> list;
-  auto rebuild = [&](bool all) -> int {
+  int byTile = 0;
+  auto rebuild = [&]() -> int {
     list.clear();
-    for (int q = 0; q < nm; q++)
-      if (!e.onCluster[q] && (all || !e.hSc[q].done))
-        list.insert(list.end(), e.tilesR[kk].begin() + e.startR[kk][q], e.tilesR[kk].begin() + e.startR[kk][q + 1]);
+    for (int pass = 0; pass < 2; pass++) {
+      for (int q = 0; q < nm; q++) {
+        const bool cluster = e.hScenes[q].mic && e.hScenes[q].mcl;
+        if (!e.onCluster[q] && !e.hSc[q].done && cluster == (pass == 1))
+          list.insert(list.end(), e.tilesR[kk].begin() + e.startR[kk][q], e.tilesR[kk].begin() + e.startR[kk][q + 1]);
+      }
+      if (pass == 0) byTile = (int)list.size();
+    }
     active = (int)list.size();
     if (active) CKB(cudaMemcpyAsync(e.dActive, list.data(), sizeof(BTile) * active, cudaMemcpyHostToDevice, st));
-    return MG_OK;
+    return jobs();
   };
-  if (rebuild(false)) return MG_ERR_CUDA;
+  if (rebuild()) return MG_ERR_CUDA;
   const bool tuning = e.rowsK < 0;
   while (active > 0 && sweeps < maxIterAll) {
     // `lag` sweeps run as one CUDA graph, captured for the current sweep list
     // and captured again when it changes
     const bool useGraph = sweeps % e.lag == 0 && sweeps + e.lag <= maxIterAll;
     if (useGraph) {
-      const GraphKey key{e.dActive, active, kk, e.dScenes, mic.flow, mic.order, mic.ntiles, mic.nscenes};
+      const GraphKey key{e.dActive, active, byTile, kk, e.dScenes, mic.flow, mic.order, mic.ntiles, mic.nscenes,
+                         e.dMc, e.dJobs, mic.mc.njobs, mic.mc.nscenes, mic.mc.maxBlocks, mic.mc.nlpMax};
       if (!e.sweepGraph || !(key == e.graphKey)) {
         if (e.sweepGraph) cudaGraphExecDestroy(e.sweepGraph);
         e.sweepGraph = nullptr;
         const unsigned long long before = t_launches;
         cudaGraph_t g = nullptr;
         CKB(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        for (int q = 0; q < e.lag; q++) launch_b_pcg_iteration(e.dActive, active, e.dScenes, 1 << kk, e.dDone, &mic, st);
+        for (int q = 0; q < e.lag; q++) launch_b_pcg_iteration(e.dActive, active, byTile, e.dScenes, 1 << kk, e.dDone, &mic, st);
         const cudaError_t ce = cudaStreamEndCapture(st, &g);
         e.graphNodes = uncount_captured(before);
         if (ce != cudaSuccess) {
@@ -621,7 +740,7 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
       e.graphLaunches++;
       sweeps += e.lag;
     } else {
-      launch_b_pcg_iteration(e.dActive, active, e.dScenes, 1 << kk, e.dDone, &mic, st);
+      launch_b_pcg_iteration(e.dActive, active, byTile, e.dScenes, 1 << kk, e.dDone, &mic, st);
       sweeps++;
     }
     if (sweeps % e.lag == 0 || sweeps == maxIterAll) {
@@ -651,7 +770,7 @@ int engine_cg(Engine& e, const BatchMic& mic, const std::vector<float>& acc, con
         doneSeen = nd;
         CKB(cudaMemcpyAsync(e.hSc.data(), e.dSc, sizeof(CgScalars) * nm, cudaMemcpyDeviceToHost, st));
         CKB(cudaStreamSynchronize(st));
-        if (rebuild(false)) return MG_ERR_CUDA;
+        if (rebuild()) return MG_ERR_CUDA;
       }
     }
   }
@@ -686,7 +805,18 @@ int engine_step(Engine& e, mg_batch_stats* stats) {
   mic.error = e.dMicCounter + 1;
   mic.epochDev = (unsigned int*)(e.dMicCounter + 2);
   mic.spinLimit = 200000000LL;
-  if (mic.nscenes > 0) CKB(cudaMemsetAsync(mic.error, 0, sizeof(int), st));
+  mic.mc = MicClusterLaunch{};
+  mic.mc.scenes = e.dMc;
+  mic.mc.nscenes = (int)e.hMc.size();
+  mic.mc.maxBlocks = e.mcBlocks;
+  mic.mc.nlpMax = e.mcLevels;
+  mic.mc.maxParts = INT_MAX;  // every scene's part has a slot per tile
+  mic.mc.counter = (unsigned*)(e.dMicCounter + 3);
+  mic.mc.error = mic.error;
+  mic.mc.ndone = e.dDone;
+  mic.mc.waitNs = mic.spinLimit;
+  const bool anyMic = mic.nscenes > 0 || mic.mc.nscenes > 0;
+  if (anyMic) CKB(cudaMemsetAsync(mic.error, 0, sizeof(int), st));
   std::vector<char> skip(nm, 0);
   std::vector<float> acc(nm, e.cgAccuracy);
   const long long graphLaunches0 = e.graphLaunches;
@@ -743,9 +873,12 @@ int engine_step(Engine& e, mg_batch_stats* stats) {
     stats->totalIterations = sum;
     stats->diverged = diverged;
   }
-  if (mic.nscenes > 0) {
+  if (anyMic) {
     int err = 0;
     CKB(cudaMemcpy(&err, mic.error, sizeof(int), cudaMemcpyDeviceToHost));
+    if (err)  // words that nobody fetched: empty again for the next solve
+      for (const MicClusterScene& m : e.hMc)
+        CKB(cudaMemsetAsync(m.gface, 0xff, mic_cluster_face_words(m) * sizeof(unsigned), st));
     if (err) return set_error(MG_ERR_TIMEOUT, "MIC wavefront (batched): a tile wait exceeded its spin limit");
   }
   for (auto& c : e.hSc)

@@ -61,6 +61,7 @@ struct BScene {
   float* P;
   unsigned long long* face;
   int mic, tx, ty, tz;
+  int mcl;         // MIC(0) by cluster sweeps (miccluster.cu): P and face are null
   // kind 0: smoke plume.  kind 1: dam break (free-surface liquid; dens[]
   // holds the levelset phi, A0f the ghost-fluid diagonal, itmp the marks of
   // the MAC extrapolation)
@@ -111,6 +112,7 @@ struct BatchMic {
   int* error;
   unsigned int* epochDev;  // device word, advanced on the device before each sweep
   long long spinLimit;
+  MicClusterLaunch mc;  // the scenes of the cluster sweeps
 };
 // doInit's preconditioner application for the MIC scenes: P, z = M^-1 r,
 // sigma = dot(z, r), search = z
@@ -118,7 +120,9 @@ void launch_b_mic_init(const BTile* t, int nt, const BScene* s, const BatchMic& 
 // one CG sweep over tiles 32 x 8*rows cells tall (rows 1, 2, 4 or 8); with
 // mic, the MIC scenes apply their preconditioner between the residual
 // update and the search-vector update
-void launch_b_pcg_iteration(const BTile* t, int nt, const BScene* s, int rows, int* ndone, const BatchMic* mic,
+// the first byTile tiles belong to scenes whose vectors are updated tile by
+// tile, the others to the scenes of the cluster sweeps
+void launch_b_pcg_iteration(const BTile* t, int nt, int byTile, const BScene* s, int rows, int* ndone, const BatchMic* mic,
                             cudaStream_t st);
 void launch_b_correct(const BTile* t, int nt, const BScene* s, int nxt, cudaStream_t st);
 // dam-break scenes (over their own tiles): extrapolateMACSimple(vel, 4),

@@ -206,6 +206,61 @@ int pcg_prepare(int sms);
 // sum of nparts per-block dot partials -> beta/sigma (init: sigma only)
 void launch_mic_finish(const PcgBuffers& b, int nparts, bool init, cudaStream_t s);
 
+// MIC(0) sweeps in thread-block clusters (miccluster.cu).  Level order: the
+// cells of 8 x 8 line bundles by level x + y + z within the bundle.
+struct MicClusterScene {
+  Dims d;
+  const code_t* code;
+  const float* A0f;   // ghost-fluid diagonal or null
+  // in level order (mic_cluster_floats each; cw half of it)
+  unsigned* cw;       // stencil bits
+  float* P;           // MIC diagonal
+  float* r;           // residual
+  float* z;           // M^-1 r
+  unsigned char* regular;  // per 8 levels of a bundle: links follow from the fluid (mic_cluster_flag_bytes)
+  // grids of the iteration
+  const float* rhs;
+  float* p;           // pressure
+  float* s;           // search vector
+  const float* t;     // A s
+  double* part;       // partial sums and norms
+  CgScalars* sc;
+  unsigned* gface;    // words between clusters (mic_cluster_face_words), all ones between sweeps
+  float nanNorm;      // residual norm reported when no residual is a number
+  int nby, nbz;       // blocks of 16 x 16 lines
+  int zper;           // z-blocks per cluster
+  int nlp;            // levels of a bundle, whole chunks
+};
+struct MicClusterLaunch {
+  MicClusterScene one;            // the scene when scenes is null
+  const MicClusterScene* scenes;  // device table of nscenes, with their jobs
+  const int2* jobs;               // (scene, first z-block), a scene's in z order
+  int njobs, nscenes;
+  int maxBlocks, nlpMax;          // the largest nby * nbz and nlp
+  int maxParts;                   // CTAs of a level launch per scene (part has at least as many slots)
+  unsigned* counter;              // ticket: zero before the first launch, back at zero after each
+  int* error;
+  int* ndone;                     // finished scenes of a batch, or null
+  long long waitNs;
+  bool stall;                     // the waits run out (failure-path tests)
+  bool l2;                        // residual norm: sum of squares instead of max-abs
+};
+int mic_cluster_prepare();
+// geometry (d, nby, nbz, zper, nlp) of a scene; false: the tile sweeps run it
+bool mic_cluster_plan(const Dims& d, MicClusterScene* s);
+size_t mic_cluster_floats(const MicClusterScene& s);
+size_t mic_cluster_flag_bytes(const MicClusterScene& s);
+size_t mic_cluster_face_words(const MicClusterScene& s);
+int mic_cluster_jobs(const MicClusterScene& s);
+// once per solve, before the factorisation: codes (and A0f) into level order
+cudaError_t launch_mic_cluster_order(const MicClusterLaunch& m, cudaStream_t s);
+// between grid and level order: r = rhs, p = 0; p += alpha s, r -= alpha t and
+// the residual norm with the convergence test; s = z + beta s; s = z
+enum { kMicInit = 0, kMicAxpy = 1, kMicUpdate = 2, kMicSearch = 3 };
+cudaError_t launch_mic_level(const MicClusterLaunch& m, int op, cudaStream_t s);
+// mode 0 factor, 1 forward r -> z, 2 backward z -> z (+ beta), 3 backward for doInit (+ sigma)
+cudaError_t launch_mic_cluster(const MicClusterLaunch& m, int mode, cudaStream_t s);
+
 // unpreconditioned CG of 2D scenes, one thread-block cluster each
 // (cgcluster.cu): rhs -> p, iterations and status in sc (accuracy, maxIter
 // and resNorm set by the caller; a scene with sc->done set is left alone)

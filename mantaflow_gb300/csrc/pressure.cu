@@ -1884,7 +1884,7 @@ __global__ void __launch_bounds__(256) k_b_correct(const BTile* __restrict__ til
 // search = z for the MIC scenes after doInit's preconditioner application
 __global__ void __launch_bounds__(256) k_b_mic_search(const BTile* __restrict__ tiles, const BScene* __restrict__ S) {
   BATCH_TILE
-  if (!in || !sc.mic) return;
+  if (!in || !sc.mic || sc.mcl) return;
   sc.search[idx] = sc.tmp[idx];
 }
 
@@ -2036,12 +2036,20 @@ void launch_b_pcg_init(const BTile* t, int nt, const BScene* s, cudaStream_t st)
   k_b_pcg_init<<<nt, dim3(kBTX, kBTY, 1), 0, st>>>(t, s);
 }
 template <int R>
-static void pcg_iteration(const BTile* t, int nt, const BScene* s, int* ndone, const BatchMic* mic, cudaStream_t st) {
+static void pcg_iteration(const BTile* t, int nt, int byTile, const BScene* s, int* ndone, const BatchMic* mic,
+                          cudaStream_t st) {
   const dim3 b(kBTX, kBTY, 1);
   count_launch();
   k_b_pcg_spmv<R><<<nt, b, 0, st>>>(t, s);
+  if (mic && mic->mc.njobs > 0) {
+    launch_mic_level(mic->mc, kMicAxpy, st);
+    launch_mic_cluster(mic->mc, 1, st);
+    launch_mic_cluster(mic->mc, 2, st);
+    launch_mic_level(mic->mc, kMicUpdate, st);
+  }
+  if (byTile == 0) return;
   count_launch();
-  k_b_pcg_axpy<R><<<nt, b, 0, st>>>(t, s, ndone);
+  k_b_pcg_axpy<R><<<byTile, b, 0, st>>>(t, s, ndone);
   if (mic && mic->nscenes > 0) {
     launch_mic_flow_batch(mic->flow, mic->order, mic->ntiles, mic->ctas, mic->counter, mic->error, 1, mic->epochDev,
                           mic->spinLimit, st);
@@ -2051,15 +2059,15 @@ static void pcg_iteration(const BTile* t, int nt, const BScene* s, int* ndone, c
     k_b_mic_finish<false><<<mic->nscenes, 256, 0, st>>>(s, mic->sceneOf, mic->flow, ndone);
   }
   count_launch();
-  k_b_pcg_update<R><<<nt, b, 0, st>>>(t, s);
+  k_b_pcg_update<R><<<byTile, b, 0, st>>>(t, s);
 }
-void launch_b_pcg_iteration(const BTile* t, int nt, const BScene* s, int rows, int* ndone, const BatchMic* mic,
+void launch_b_pcg_iteration(const BTile* t, int nt, int byTile, const BScene* s, int rows, int* ndone, const BatchMic* mic,
                             cudaStream_t st) {
   switch (rows) {
-    case 1: pcg_iteration<1>(t, nt, s, ndone, mic, st); break;
-    case 2: pcg_iteration<2>(t, nt, s, ndone, mic, st); break;
-    case 4: pcg_iteration<4>(t, nt, s, ndone, mic, st); break;
-    default: pcg_iteration<8>(t, nt, s, ndone, mic, st); break;
+    case 1: pcg_iteration<1>(t, nt, byTile, s, ndone, mic, st); break;
+    case 2: pcg_iteration<2>(t, nt, byTile, s, ndone, mic, st); break;
+    case 4: pcg_iteration<4>(t, nt, byTile, s, ndone, mic, st); break;
+    default: pcg_iteration<8>(t, nt, byTile, s, ndone, mic, st); break;
   }
 }
 void launch_b_correct(const BTile* t, int nt, const BScene* s, int nxt, cudaStream_t st) {

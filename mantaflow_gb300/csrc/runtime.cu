@@ -124,6 +124,8 @@ struct mg_solver_s {
   bool useMicWave = false;
   unsigned long long* micFace = nullptr;  // tile-dataflow sweeps: face words
   bool useMicFlow = false;
+  MicClusterLaunch micCluster{};  // cluster sweeps: geometry and buffers
+  bool useMicCluster = false;
   unsigned int epoch = 0;
   long long waitNs = kWaitNs;  // limit of each device-side MIC wait
   bool stallNext = false;      // the next MIC solve's waits run out (test of the timeout path)
@@ -314,7 +316,8 @@ extern "C" int mg_init(int device) {
   g_ctx.sms = prop.multiProcessorCount;
   g_ctx.micCtasPerSm = mic_ctas_per_sm();
   if (mic_col_prepare() || mic_wave_prepare(&g_ctx.waveCtasPerSm4, &g_ctx.waveCtasPerSm8) ||
-      mic_flow_prepare(&g_ctx.flowCtasPerSm) || pcg_prepare(g_ctx.sms) || cg_cluster_prepare())
+      mic_flow_prepare(&g_ctx.flowCtasPerSm) || pcg_prepare(g_ctx.sms) || cg_cluster_prepare() ||
+      mic_cluster_prepare())
     return fail(MG_ERR_CUDA, "mg_init: cannot configure the MIC kernels");
   g_ctx.device = device;
   g_ctx.init = true;
@@ -389,6 +392,12 @@ static void free_cg_state(mg_solver s) {
   cudaFree(s->micWave.order); cudaFree(s->micWave.counter); cudaFree(s->micWave.exchange);
   cudaFree(s->micFace);
   s->micFace = nullptr;
+  // micCluster.error aliases mic.error
+  cudaFree(s->micCluster.one.cw); cudaFree(s->micCluster.one.P); cudaFree(s->micCluster.one.r);
+  cudaFree(s->micCluster.one.z); cudaFree(s->micCluster.one.gface);
+  cudaFree(s->micCluster.one.regular);
+  cudaFree(s->micCluster.counter);
+  s->micCluster = MicClusterLaunch{};
   cudaFree(s->Aoff);
   s->Aoff = nullptr;
   cudaGetLastError();  // a failed free must not surface as a later launch error
@@ -1115,7 +1124,6 @@ static int ensure_cg_state(mg_solver s) {
   CK(cudaMallocHost(&s->scHost, sizeof(CgScalars)));
   CK(cudaMalloc(&s->intScratch, 16 * sizeof(int)));
   if (s->d.is3d) {
-    CK(cudaMalloc(&s->P, n * sizeof(float)));
     MicPlan& m = s->mic;
     m.tx = tx; m.ty = ty; m.tz = tz;
     m.ntiles = (int)ntiles;
@@ -1129,14 +1137,38 @@ static int ensure_cg_state(mg_solver s) {
     CK(cudaMalloc(&m.error, sizeof(int)));
     CK(cudaMemset(m.error, 0, sizeof(int)));
     m.ctas = g_ctx.sms * g_ctx.micCtasPerSm;
-    // tile-dataflow sweeps (micflow.cu) by default; MANTA_GB300_MIC selects
-    // the whole-tile sweeps ("tile", pressure.cu), the column-block sweeps
-    // ("column", mic.cu) or the warp wavefronts ("wave", micwave.cu)
+    // cluster sweeps (miccluster.cu) where the grid fits them, else
+    // tile-dataflow sweeps (micflow.cu); MANTA_GB300_MIC selects the latter
+    // ("flow"), the whole-tile sweeps ("tile", pressure.cu), the column-block
+    // sweeps ("column", mic.cu) or the warp wavefronts ("wave", micwave.cu)
     const char* ev = getenv("MANTA_GB300_MIC");
-    const std::string mk = ev ? std::string(ev) : std::string("flow");
+    const std::string mk = ev ? std::string(ev) : std::string("cluster");
     s->useMicCol = mic_col_supported(s->d) && mk == "column";
     s->useMicWave = mic_wave_supported(s->d) && mk == "wave";
-    s->useMicFlow = !s->useMicCol && !s->useMicWave && mk != "tile";
+    MicClusterLaunch& mc = s->micCluster;
+    s->useMicCluster = !s->useMicCol && !s->useMicWave && mk != "tile" && mk != "flow" && mic_cluster_plan(s->d, &mc.one);
+    s->useMicFlow = !s->useMicCol && !s->useMicWave && !s->useMicCluster && mk != "tile";
+    if (s->useMicCluster) {
+      const size_t words = mic_cluster_face_words(mc.one);
+      const size_t nl = mic_cluster_floats(mc.one);
+      CK(cudaMalloc(&mc.one.cw, nl / 2 * sizeof(unsigned)));
+      CK(cudaMalloc(&mc.one.P, nl * sizeof(float)));
+      CK(cudaMalloc(&mc.one.r, nl * sizeof(float)));
+      CK(cudaMalloc(&mc.one.z, nl * sizeof(float)));
+      CK(cudaMalloc(&mc.one.regular, mic_cluster_flag_bytes(mc.one)));
+      CK(cudaMalloc(&mc.one.gface, words * sizeof(unsigned)));
+      CK(cudaMemset(mc.one.gface, 0xff, words * sizeof(unsigned)));
+      CK(cudaMalloc(&mc.counter, sizeof(unsigned)));
+      CK(cudaMemset(mc.counter, 0, sizeof(unsigned)));
+      mc.njobs = mic_cluster_jobs(mc.one);
+      mc.nscenes = 1;
+      mc.maxBlocks = mc.one.nby * mc.one.nbz;
+      mc.nlpMax = mc.one.nlp;
+      mc.maxParts = s->nblocks;
+      mc.one.nanNorm = FLT_MAX;
+      mc.error = m.error;
+      if ((size_t)mc.maxBlocks > s->partCount) return fail(MG_ERR_STATE, "MIC: partial buffer too small");
+    }
     if (s->useMicFlow) {
       const size_t words = mic_flow_face_words(m.ntiles);
       CK(cudaMalloc(&s->micFace, words * sizeof(unsigned long long)));
@@ -1187,6 +1219,31 @@ static MicPlan flow_plan(mg_solver s) {
 static int wave_ctas(mg_solver s) {
   return g_ctx.sms * (s->micWave.zw == 4 ? g_ctx.waveCtasPerSm4 : g_ctx.waveCtasPerSm8);
 }
+
+// the diagonal P in grid layout, which every MIC(0) but the cluster sweeps uses
+static int ensure_grid_p(mg_solver s) {
+  if (!s->P) CK(cudaMalloc(&s->P, (size_t)s->d.n * sizeof(float)));
+  return MG_OK;
+}
+
+// the cluster sweeps of this solve
+static MicClusterLaunch mic_cluster_launch(mg_solver s, const PcgBuffers& b, bool l2 = false) {
+  MicClusterLaunch m = s->micCluster;
+  m.one.code = b.code;
+  m.one.A0f = b.A0f;
+  m.one.rhs = b.rhs;
+  m.one.p = b.pressure;
+  m.one.s = b.search;
+  m.one.t = b.tmp;
+  m.one.part = b.part;
+  m.one.sc = b.sc;
+  m.waitNs = s->waitNs;
+  m.stall = s->stall;
+  m.l2 = l2;
+  return m;
+}
+// whether this solve's MIC(0) runs as cluster sweeps (fractions run plane by plane)
+static bool mic_cluster_on(mg_solver s, const PcgBuffers& b) { return s->useMicCluster && !b.Aif; }
 
 static PcgBuffers cg_buffers(mg_solver s, mg_grid flags, float* rhs, mg_grid pressure) {
   PcgBuffers b;
@@ -1272,14 +1329,16 @@ static int apply_precond(mg_solver s, const PcgBuffers& b, int pc, bool init) {
   } else if (pc == kPcMic) {
     {
       ProfScope ps(s, "mic_forward");
-      if (s->useMicFlow) launch_mic_flow(b, flow_plan(s), s->micFace, 1, ++s->epoch, s->waitNs, s->stream, s->stall);
+      if (s->useMicCluster) CK(launch_mic_cluster(mic_cluster_launch(s, b), 1, s->stream));
+      else if (s->useMicFlow) launch_mic_flow(b, flow_plan(s), s->micFace, 1, ++s->epoch, s->waitNs, s->stream, s->stall);
       else if (s->useMicWave) launch_mic_wave(b, s->micWave, 1, ++s->epoch, s->waitNs, wave_ctas(s), s->stream);
       else if (s->useMicCol) launch_mic_col(b, s->micCol, 1, ++s->epoch, s->waitNs, g_ctx.sms, s->stream);
       else launch_mic(b, s->mic, 1, ++s->epoch, s->waitNs, s->stream);
     }
     {
       ProfScope ps(s, "mic_backward");
-      if (s->useMicFlow) launch_mic_flow(b, flow_plan(s), s->micFace, init ? 3 : 2, ++s->epoch, s->waitNs, s->stream, s->stall);
+      if (s->useMicCluster) CK(launch_mic_cluster(mic_cluster_launch(s, b), init ? 3 : 2, s->stream));
+      else if (s->useMicFlow) launch_mic_flow(b, flow_plan(s), s->micFace, init ? 3 : 2, ++s->epoch, s->waitNs, s->stream, s->stall);
       else if (s->useMicWave)
         launch_mic_wave(b, s->micWave, init ? 3 : 2, ++s->epoch, s->waitNs, wave_ctas(s), s->stream);
       else if (s->useMicCol) launch_mic_col(b, s->micCol, init ? 3 : 2, ++s->epoch, s->waitNs, g_ctx.sms, s->stream);
@@ -1439,6 +1498,11 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
     const int e = mg_setup(s->mg, b, (float)((double)p->cgAccuracy * 1E-4), s->stream);
     if (e) return fail(MG_ERR_CUDA, std::string("multigrid setup failed: ") + cudaGetErrorString(cudaGetLastError()));
   }
+  if (pc == kPcMic && (b.Aif || !s->useMicCluster)) {
+    st = ensure_grid_p(s);
+    if (st) return st;
+    b.P = s->P;
+  }
   // GridCg::doInit
   CgScalars init{};
   init.accuracy = p->cgAccuracy;
@@ -1461,7 +1525,8 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
   }
   {
     ProfScope ps(s, "pcg_init");
-    launch_pcg_init(b, s->stream);
+    if (pc == kPcMic && mic_cluster_on(s, b)) CK(launch_mic_level(mic_cluster_launch(s, b), kMicInit, s->stream));
+    else launch_pcg_init(b, s->stream);
   }
   CKL();
   if (pc == kPcMic) {
@@ -1470,12 +1535,18 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
     s->stallNext = false;
     CK(cudaMemsetAsync(s->mic.error, 0, sizeof(int), s->stream));
     if (b.Aif) launch_mic_planes(b, 0, s->stream);
+    else if (s->useMicCluster) {
+      const MicClusterLaunch m = mic_cluster_launch(s, b);
+      CK(launch_mic_cluster_order(m, s->stream));
+      CK(launch_mic_cluster(m, 0, s->stream));
+    }
     else if (s->useMicFlow) launch_mic_flow(b, flow_plan(s), s->micFace, 0, ++s->epoch, s->waitNs, s->stream, s->stall);
     else if (s->useMicWave) launch_mic_wave(b, s->micWave, 0, ++s->epoch, s->waitNs, wave_ctas(s), s->stream);
     else if (s->useMicCol) launch_mic_col(b, s->micCol, 0, ++s->epoch, s->waitNs, g_ctx.sms, s->stream);
     else launch_mic(b, s->mic, 0, ++s->epoch, s->waitNs, s->stream);
     CKL();
   }
+  const bool micLevels = pc == kPcMic && mic_cluster_on(s, b);
   if (pc != kPcNone) {
     st = apply_precond(s, b, pc, true);
     if (st) return st;
@@ -1485,7 +1556,8 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
   }
   {
     ProfScope ps(s, "pcg_set_search");
-    launch_pcg_set_search(b, s->stream);
+    if (micLevels) CK(launch_mic_level(mic_cluster_launch(s, b), kMicSearch, s->stream));  // sigma: from the sweep
+    else launch_pcg_set_search(b, s->stream);
   }
   CKL();
   // GridCg::iterate until converged or maxIter; the host polls the device
@@ -1522,7 +1594,8 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
     }
     {
       ProfScope ps(s, "pcg_axpy");
-      launch_pcg_axpy(b, s->stream);
+      if (micLevels) CK(launch_mic_level(mic_cluster_launch(s, b, p->useL2Norm != 0), kMicAxpy, s->stream));
+      else launch_pcg_axpy(b, s->stream);
     }
     if (s->prof) {
       // the axpy's residual norm may have converged the solve, after which
@@ -1540,7 +1613,8 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
     if (st) return st;
     {
       ProfScope ps(s, "pcg_update");
-      launch_pcg_update(b, s->stream);
+      if (micLevels) CK(launch_mic_level(mic_cluster_launch(s, b), kMicUpdate, s->stream));
+      else launch_pcg_update(b, s->stream);
     }
     CKL();
     it++;
@@ -1556,6 +1630,10 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
     s->stall = false;
     int err = 0;
     CK(cudaMemcpy(&err, s->mic.error, sizeof(int), cudaMemcpyDeviceToHost));
+    if (err && s->useMicCluster) {
+      // words that nobody fetched: empty again for the next solve
+      CK(cudaMemsetAsync(s->micCluster.one.gface, 0xff, mic_cluster_face_words(s->micCluster.one) * sizeof(unsigned), s->stream));
+    }
     if (err) return fail(MG_ERR_TIMEOUT, "MIC wavefront: a tile wait exceeded its spin limit");
   }
   st = solve_outcome(s, out);
