@@ -41,6 +41,8 @@
 // solves against the tile sweeps of micflow.cu: 64^3 smoke (50 iterations)
 // 9.2 -> 4.0 ms, 128^3 dam break (53) 21.3 -> 8.0 ms.  Grids with more than
 // 256 rows or more than about 400 cells along x do not fit and keep the tiles.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
