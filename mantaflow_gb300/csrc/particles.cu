@@ -12,12 +12,17 @@
 // transfers (the reference's single-threaded setInterpolated loops,
 // knMapLinearVec3ToMACGrid and knMapLinear) add every particle's weighted
 // value into the 8 faces or cells around it, in particle order, so a face's
-// float sums depend on that order.  Here each face gathers instead of each
-// particle scattering: the particles are sorted, stably, by the cell their
-// interpolation stencil starts at (one LSD radix sort per MAC component),
-// and a face merges the up to 8 sorted buckets that reach it by particle
-// index, adding the same float products in the same order as the reference.
-// The result is the reference's bit for bit, with no atomics.
+// float sums depend on that order.  The results here are the reference's bit
+// for bit:
+//
+//  * MAC faces in 3D (mapPartsToMAC): the particles are listed, in particle
+//    order, by the tiles of 4^3 or 8^3 cells they reach, and one warp per tile
+//    adds them up one after another, a particle's 24 faces at a time, in
+//    shared memory (k_tile_*).
+//  * Cells (mapPartsToGrid), 2D, and systems too large for the lists: the
+//    particles are sorted, stably, by the cell their interpolation stencil
+//    starts at (one LSD radix sort per MAC component), and each face or cell
+//    merges the up to 8 sorted buckets that reach it by particle index.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -341,7 +346,7 @@ __global__ void __launch_bounds__(256) k_p2g_gather(Dims d, int comp, SortedPart
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
   if (i >= d.nx || j >= d.ny) return;
-  constexpr unsigned kNone = 0xffffffffu;
+  constexpr unsigned kEnd = 0xffffffffu;
   unsigned cur[8], end[8], head[8];
 #pragma unroll
   for (int q = 0; q < 8; q++) {
@@ -354,7 +359,7 @@ __global__ void __launch_bounds__(256) k_p2g_gather(Dims d, int comp, SortedPart
       cur[q] = starts[key];
       end[q] = starts[key + 1];
     }
-    head[q] = cur[q] < end[q] ? sorted[cur[q]] : kNone;
+    head[q] = cur[q] < end[q] ? sorted[cur[q]] : kEnd;
   }
   const bool zFirst0 = comp == 2;  // 2D: which z layer the reference adds first
   float sum = 0.f, r0 = 0.f, r1 = 0.f, r2 = 0.f;
@@ -367,7 +372,7 @@ __global__ void __launch_bounds__(256) k_p2g_gather(Dims d, int comp, SortedPart
         best = head[q];
         bq = q;
       }
-    if (best == kNone) break;
+    if (best == kEnd) break;
     unsigned at = cur[0];  // the particle's slot in bucket order
 #pragma unroll
     for (int q = 1; q < 8; q++)
@@ -402,7 +407,7 @@ __global__ void __launch_bounds__(256) k_p2g_gather(Dims d, int comp, SortedPart
     for (int q = 0; q < 8; q++)
       if (q == bq) {
         cur[q]++;
-        head[q] = cur[q] < end[q] ? sorted[cur[q]] : kNone;
+        head[q] = cur[q] < end[q] ? sorted[cur[q]] : kEnd;
       }
   }
   const long long o = ix(d, i, j, k);
@@ -424,6 +429,409 @@ __global__ void __launch_bounds__(256) k_p2g_gather(Dims d, int comp, SortedPart
       o1[o] = r1 / sum;
       o2[o] = r2 / sum;
     }
+  }
+}
+
+// ---------------------------------------------- particles -> MAC faces
+// The serial sums of the faces of a tile of cells depend on nothing but the
+// particles that reach the tile, in particle order.  So: list those (a
+// particle near a tile's border is in up to eight lists: 1.9 on average with
+// 8 x 8 x 4 cells, 2.6 with 4^3), put every list into particle order, and let
+// one warp per tile walk its list.  Lane 8 c + k of it holds corner k of
+// component c: it reads the particle's three weights and value of that
+// component, forms its corner's weight as the reference does, and adds to its
+// face in shared memory, about 20 instructions for a particle's 24 faces.  The
+// weights come from a batch of 32 particles whose lanes prepared one each.
+//
+// At 128^3 with 16.8 M particles mapPartsToMAC took 5.5 ms with a radix sort
+// and eight-way merges per component (3.2 ms of it in the merges, about 100
+// instructions per contribution); FIGURES
+template <int X, int Y, int Z>
+struct TileShape {
+  static constexpr int x = X, y = Y, z = Z;
+};
+using TileLarge = TileShape<8, 8, 4>;
+using TileSmall = TileShape<4, 4, 4>;
+constexpr int kLine = 32;  // words of 128 bytes
+constexpr int kSortThreads = 256, kSortWarps = kSortThreads / 32;
+constexpr int kSortShort = 4608, kSortLong = 24576;  // list entries sorted in shared memory, by two kernels
+constexpr int kDigit = 10;                           // most bits of a sort pass
+struct Tiles {
+  Dims d;
+  long long n;
+  int tx, ty, tz;
+  bool large;         // TileLarge, not TileSmall
+  unsigned* starts;   // [tiles + 1]: the lists' first entries
+  unsigned* cursor;   // [tiles][kLine]: counts, then next entries
+  unsigned* list;     // particles by tile
+  const float* v[3];  // velocity components
+  __host__ __device__ int count() const { return tx * ty * tz; }
+  __device__ unsigned* counter(int t) const { return cursor + (size_t)t * kLine; }
+};
+
+// one axis of BUILD_INDEX / BUILD_INDEX_SHIFT: first sample and upper weight
+// (the lower one is 1 minus it, in the border clamps too)
+__device__ __forceinline__ int axis_sample(float q, int n, float& w1) {
+  int i = (int)q;
+  w1 = q - (float)i;
+  if (q < 0.f) {
+    i = 0;
+    w1 = 0.f;
+  }
+  if (i >= n - 1) {
+    i = n - 2;
+    w1 = 1.f;
+  }
+  return i;
+}
+__device__ __forceinline__ int axis_sample(float q, int n) {
+  float w;
+  return axis_sample(q, n, w);
+}
+
+// Counts of a tile's particles, or their entries (kFill).  A particle's faces
+// of all three components lie in at most 2 x 2 x 2 tiles.  The lanes of a warp
+// with the same tile take it with one atomic; particles in flight are mostly
+// neighbours, so each tile's counter has a line of its own (side by side, the
+// atomics queue at a few L2 slices: 295 and 361 us at 128^3, now FIGURES2).
+template <class T, bool kFill>
+__global__ void __launch_bounds__(256) k_tile_lists(Tiles s, PartView p) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  float x = 0.f, y = 0.f, z = 0.f;
+  bool live = i < s.n;
+  if (live) {  // before the flag is known
+    x = p.x[i];
+    y = p.y[i];
+    z = p.z[i];
+    live = !part_skip(p, i);
+  }
+  const int a0 = axis_sample(x - 0.5f, s.d.nx) / T::x, a1 = (axis_sample(x, s.d.nx) + 1) / T::x;
+  const int b0 = axis_sample(y - 0.5f, s.d.ny) / T::y, b1 = (axis_sample(y, s.d.ny) + 1) / T::y;
+  const int c0 = axis_sample(z - 0.5f, s.d.nz) / T::z, c1 = (axis_sample(z, s.d.nz) + 1) / T::z;
+  const int t0 = a0 + s.tx * (b0 + s.ty * c0);
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const bool in = live && (!(q & 1) || a1 > a0) && (!(q & 2) || b1 > b0) && (!(q & 4) || c1 > c0);
+    if (!__any_sync(0xffffffffu, in)) continue;
+    const int t = in ? t0 + (q & 1) + s.tx * ((q >> 1 & 1) + s.ty * (q >> 2)) : -1;
+    const unsigned act = __ballot_sync(0xffffffffu, in);
+    if (!in) continue;
+    const unsigned peers = __match_any_sync(act, t);
+    const int first = __ffs(peers) - 1;
+    if (!kFill) {
+      if (lane == first) atomicAdd(s.counter(t), (unsigned)__popc(peers));
+    } else {
+      unsigned at = 0;
+      if (lane == first) at = atomicAdd(s.counter(t), (unsigned)__popc(peers));
+      at = __shfl_sync(peers, at, first) + __popc(peers & ((1u << lane) - 1u));
+      s.list[at] = (unsigned)i;
+    }
+  }
+}
+
+// counts to first entries; one CTA, eight tiles per thread at a time
+__global__ void __launch_bounds__(1024) k_tile_starts(Tiles s) {
+  __shared__ unsigned sh[32];
+  const int tiles = s.count();
+  unsigned carry = 0;
+  for (int t0 = threadIdx.x * 8; t0 - (int)threadIdx.x * 8 < tiles; t0 += 8192) {
+    unsigned c[8], sum = 0, total;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      c[q] = t0 + q < tiles ? *s.counter(t0 + q) : 0u;
+      sum += c[q];
+    }
+    unsigned at = carry + block_excl_scan(sum, sh, &total);
+    carry += total;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      if (t0 + q < tiles) s.starts[t0 + q] = *s.counter(t0 + q) = at;
+      at += c[q];
+    }
+  }
+  if (threadIdx.x == 0) s.starts[tiles] = carry;
+}
+
+// A tile's list into particle order.  Up to kCap entries: an LSD radix sort in
+// shared memory over the bits in which the list's entries can differ, eight
+// warps on consecutive pieces of the list (digit counts per warp, scanned
+// digit by digit, keep it stable).  A first kernel takes a CTA for every list
+// and sorts the short ones with four CTAs per SM; in a second one few CTAs
+// walk over all lists for those that were too long, and sort what does not
+// fit into shared memory either (crowded tiles) by a bitonic network in place.
+__device__ void sort_in_place(unsigned* list, unsigned n) {
+  unsigned long long top = 1;
+  while (top < n) top <<= 1;
+  for (unsigned long long g = 2; g <= top; g <<= 1)
+    for (unsigned long long h = g >> 1; h > 0; h >>= 1) {
+      for (unsigned long long e = threadIdx.x; e < top / 2; e += blockDim.x) {
+        // every comparison upward: the first step of a merge pairs an
+        // entry with its mirror image; places past the end count as larger
+        const unsigned long long b = e / h * 2 * h, x = b + e % h, y = h == g >> 1 ? b + 2 * h - 1 - e % h : x + h;
+        if (y < n && list[y] < list[x]) {
+          const unsigned v = list[x];
+          list[x] = list[y];
+          list[y] = v;
+        }
+      }
+      __syncthreads();
+    }
+}
+
+template <int kCap>
+__device__ __forceinline__ void sort_list(unsigned* list, unsigned n, unsigned* sm) {
+  __shared__ unsigned sh[32], range[2];
+  unsigned *in = sm, *out = sm + kCap;
+  unsigned short* const cnt = (unsigned short*)(sm + 2 * kCap);  // [warps][1 << width]
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  if (t == 0) {
+    range[0] = 0xffffffffu;
+    range[1] = 0u;
+  }
+  unsigned least = 0xffffffffu, most = 0u;
+  for (unsigned e = t; e < n; e += kSortThreads) {
+    const unsigned v = list[e];
+    in[e] = v;
+    least = min(least, v);
+    most = max(most, v);
+  }
+  least = __reduce_min_sync(0xffffffffu, least);
+  most = __reduce_max_sync(0xffffffffu, most);
+  __syncthreads();
+  if (lane == 0) {
+    atomicMin(range, least);
+    atomicMax(range + 1, most);
+  }
+  __syncthreads();
+  least = range[0];
+  const int bits = 32 - __clz(range[1] - least), passes = (bits + kDigit - 1) / kDigit;
+  const int width = max(8, (bits + passes - 1) / max(passes, 1)), digits = 1 << width, each = digits / kSortThreads;
+  const unsigned mask = digits - 1;
+  const unsigned per = ((n + kSortWarps - 1) / kSortWarps + 31) & ~31u;
+  const unsigned from = min(n, w * per), to = min(n, from + per);
+  unsigned short* const mine = cnt + w * digits;
+  for (int pass = 0, shift = 0; pass < passes; pass++, shift += width) {
+    for (int q = lane; q < digits / 2; q += 32) ((unsigned*)mine)[q] = 0u;
+    __syncwarp();
+    for (unsigned e = from + lane; e < to; e += 32) {
+      const unsigned dig = (in[e] - least) >> shift & mask;
+      atomicAdd((unsigned*)mine + (dig >> 1), 1u << (dig & 1) * 16);
+    }
+    __syncthreads();
+    unsigned sum = 0, total;
+    for (int g = t * each; g < (t + 1) * each; g++)
+#pragma unroll
+      for (int q = 0; q < kSortWarps; q++) sum += cnt[q * digits + g];
+    unsigned at = block_excl_scan(sum, sh, &total);
+    for (int g = t * each; g < (t + 1) * each; g++)
+#pragma unroll
+      for (int q = 0; q < kSortWarps; q++) {
+        const unsigned c = cnt[q * digits + g];
+        cnt[q * digits + g] = (unsigned short)at;
+        at += c;
+      }
+    __syncthreads();
+    for (unsigned e0 = from; e0 < to; e0 += 32) {
+      const bool ok = e0 + lane < to;
+      const unsigned v = ok ? in[e0 + lane] : 0u, dig = (v - least) >> shift & mask;
+      // lanes with the same digit, by one vote per bit: __match_any_sync takes
+      // far longer when all digits differ
+      unsigned peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+      for (int q = 0; q < kDigit; q++)
+        if (q < width) {
+          const unsigned ones = __ballot_sync(0xffffffffu, dig >> q & 1u);
+          peers &= dig >> q & 1u ? ones : ~ones;
+        }
+      const unsigned rank = __popc(peers & ((1u << lane) - 1u)), at = mine[dig];
+      __syncwarp();
+      if (ok) {
+        out[at + rank] = v;
+        if (rank == 0) mine[dig] = (unsigned short)(at + __popc(peers));
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    unsigned* const x = in;
+    in = out;
+    out = x;
+  }
+  for (unsigned e = t; e < n; e += kSortThreads) list[e] = in[e];
+  __syncthreads();
+}
+constexpr size_t sort_smem(int cap) { return 2 * (size_t)cap * 4 + (kSortWarps << kDigit) * 2; }
+
+__global__ void __launch_bounds__(kSortThreads) k_tile_sort(Tiles s) {
+  extern __shared__ __align__(16) unsigned sm[];
+  const unsigned lo = s.starts[blockIdx.x], n = s.starts[blockIdx.x + 1] - lo;
+  if (n > 1 && n <= kSortShort) sort_list<kSortShort>(s.list + lo, n, sm);
+}
+__global__ void __launch_bounds__(kSortThreads) k_tile_sort_long(Tiles s) {
+  extern __shared__ __align__(16) unsigned sm[];
+  __shared__ unsigned many[kSortThreads], found;
+  for (int t0 = blockIdx.x * kSortThreads; t0 < s.count(); t0 += gridDim.x * kSortThreads) {
+    if (threadIdx.x == 0) found = 0;
+    __syncthreads();
+    const int t = t0 + threadIdx.x;
+    if (t < s.count() && s.starts[t + 1] - s.starts[t] > kSortShort) many[atomicAdd(&found, 1u)] = t;
+    __syncthreads();
+    for (unsigned q = 0; q < found; q++) {
+      const unsigned lo = s.starts[many[q]], n = s.starts[many[q] + 1] - lo;
+      if (n <= kSortLong) sort_list<kSortLong>(s.list + lo, n, sm);
+      else sort_in_place(s.list + lo, n);
+    }
+    __syncthreads();
+  }
+}
+
+// A tile's accumulators in shared memory, {weight, weighted value} per face.
+// A lane owns the faces of one component and one parity along x, y and z: a
+// particle has one face of each, and no two lanes ever add to the same one.
+template <class T>
+struct TileAcc {
+  static constexpr int kRow = 32;  // lanes: no bank conflicts (with 24, the lanes that add: 20 % fewer tiles' worth of memory, 9 % slower)
+  static constexpr int kY = T::x / 2, kZ = kY * (T::y / 2), kAll = kZ * (T::z / 2);
+  float2 acc[kAll][kRow];
+  // A batch of 32 particles.  Weights of the odd faces and value of particles
+  // 2 i and 2 i + 1 by component, {x, x, y, y}, {z, z, value, value}:
+  float4 w[16][7];
+  uint4 in[3][8];  // 5-bit fields: first sample - tile's first cell + 8 per axis
+  uint4 at[3][8];  // from bit 16: byte offset of the first sample's row of acc; below, the rows' steps along axes with an odd sample
+};
+
+// two floats at once, each rounded as by itself
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{.reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
+      " fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mul.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
+// two floats in shared memory, without a branch
+__device__ __forceinline__ void add_if(unsigned at, bool in, float x, float y) {
+  asm volatile(
+      "{.reg .pred p;\n .reg .f32 a, b;\n mov.f32 a, 0f00000000;\n mov.f32 b, a;\n setp.ne.b32 p, %1, 0;\n"
+      " @p ld.shared.v2.f32 {a, b}, [%0];\n add.f32 a, a, %2;\n add.f32 b, b, %3;\n @p st.shared.v2.f32 [%0], {a, b};}" ::"r"(at),
+      "r"((int)in), "f"(x), "f"(y)
+      : "memory");
+}
+
+template <class T>
+__global__ void __launch_bounds__(32) k_tile_splat(Tiles s, PartView p, float* vel, float* old, float* wout) {
+  __shared__ TileAcc<T> sm;
+  typedef TileAcc<T> A;
+  const Dims& d = s.d;
+  const int lane = threadIdx.x;
+  const int x0 = blockIdx.x * T::x, y0 = blockIdx.y * T::y, z0 = blockIdx.z * T::z;
+  const int t = blockIdx.x + s.tx * (blockIdx.y + s.ty * blockIdx.z);
+  const unsigned lo = s.starts[t], n = s.starts[t + 1] - lo;
+  const unsigned* const list = s.list + lo;
+  for (int q = lane; q < A::kAll * A::kRow; q += 32) (&sm.acc[0][0])[q] = make_float2(0.f, 0.f);
+  // This lane's component and parity.  Its weight along an axis is that of the
+  // odd face, or 1 minus it.  (Exact: with an odd first sample the odd face has
+  // the lower weight, 1 minus the upper one, which is a multiple of 2^-23.)
+  const int c = min(lane >> 3, 2), ox = lane & 1, oy = lane >> 1 & 1, oz = lane >> 2 & 1;
+  auto both = [](float v) { return make_float2(v, v); };
+  const float2 ax = both(ox ? 0.f : 1.f), bx = both(ox ? 1.f : -1.f);
+  const float2 ay = both(oy ? 0.f : 1.f), by = both(oy ? 1.f : -1.f);
+  const float2 az = both(oz ? 0.f : 1.f), bz = both(oz ? 1.f : -1.f);
+  // The face's row is (first sample + 1 - parity) / 2 per axis, in the tile if
+  // the fields' upper bits are 8; bit 15 keeps the last lanes out.
+  const unsigned up = (unsigned)((1 - ox) | (1 - oy) << 5 | (1 - oz) << 10) | (lane < 24 ? 0u : 0x8000u);
+  constexpr unsigned kMask = (0x1fu & ~(T::x - 1u)) | (0x1fu & ~(T::y - 1u)) << 5 | (0x3fu & ~(T::z - 1u)) << 10;
+  constexpr unsigned kIn = 8u | 8u << 5 | 8u << 10;
+  constexpr int kStep = 8 * A::kRow;
+  static_assert((kStep & kStep * A::kY) == 0 && (kStep * A::kY & kStep * A::kZ) == 0 && (kStep & kStep * A::kZ) == 0, "steps share bits");
+  const unsigned steps = (ox ? 0 : kStep) | (oy ? 0 : kStep * A::kY) | (oz ? 0 : kStep * A::kZ);
+  const unsigned own = (unsigned)__cvta_generic_to_shared(&sm.acc[0][min(lane, A::kRow - 1)]);
+  // a particle's index is fetched two batches ahead, the particle one
+  unsigned next = 0;
+  float px = 0.f, py = 0.f, pz = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f;
+  auto fetch = [&](unsigned e) {
+    if (e >= n) return;
+    px = __ldg(p.x + next);
+    py = __ldg(p.y + next);
+    pz = __ldg(p.z + next);
+    v0 = __ldg(s.v[0] + next);
+    v1 = __ldg(s.v[1] + next);
+    v2 = __ldg(s.v[2] + next);
+    if (e + 32 < n) next = list[e + 32];
+  };
+  if (lane < n) next = list[lane];
+  fetch(lane);
+  for (unsigned b = 0; b < n; b += 32) {
+    {
+      float sx, sy, sz, cx, cy, cz;
+      const int isx = axis_sample(px, d.nx, sx) - x0, icx = axis_sample(px - 0.5f, d.nx, cx) - x0;
+      const int isy = axis_sample(py, d.ny, sy) - y0, icy = axis_sample(py - 0.5f, d.ny, cy) - y0;
+      const int isz = axis_sample(pz, d.nz, sz) - z0, icz = axis_sample(pz - 0.5f, d.nz, cz) - z0;
+      auto odd = [](int i, float w) { return i & 1 ? 1.f - w : w; };
+      auto pack = [&](int comp, int x, int y, int z, float wx, float wy, float wz, float v) {
+        float* const w = (float*)&sm.w[lane >> 1][2 * comp] + (lane & 1);
+        w[0] = wx;
+        w[2] = wy;
+        w[4] = wz;
+        w[6] = v;
+        const unsigned in = (unsigned)(x + 8) | (unsigned)(y + 8) << 5 | (unsigned)(z + 8) << 10;
+        ((unsigned*)sm.in[comp])[lane] = b + lane < n ? in : 0u;
+        ((unsigned*)sm.at[comp])[lane] = (unsigned)(kStep * ((x >> 1) + A::kY * (y >> 1) + A::kZ * (z >> 1))) << 16 |
+                                         kStep * ((x & 1) + A::kY * (y & 1) + A::kZ * (z & 1));
+      };
+      sx = odd(isx, sx);
+      sy = odd(isy, sy);
+      sz = odd(isz, sz);
+      cx = odd(icx, cx);
+      cy = odd(icy, cy);
+      cz = odd(icz, cz);
+      pack(0, isx, icy, icz, sx, cy, cz, v0);
+      pack(1, icx, isy, icz, cx, sy, cz, v1);
+      pack(2, icx, icy, isz, cx, cy, sz, v2);
+    }
+    __syncwarp();
+    fetch(b + 32 + lane);
+    const int m = (int)min(32u, n - b);
+    for (int k0 = 0; k0 < m; k0 += 4) {
+      const uint4 i4 = sm.in[c][k0 >> 2], a4 = sm.at[c][k0 >> 2];
+      const unsigned in[4] = {i4.x, i4.y, i4.z, i4.w}, at[4] = {a4.x, a4.y, a4.z, a4.w};
+      float2 wk[2], wv[2];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const float4 xy = sm.w[(k0 >> 1) + k][2 * c], zv = sm.w[(k0 >> 1) + k][2 * c + 1];
+        // fma with factors 1 and -1: the odd face's weight itself, or 1 minus it
+        const float2 S = fma2(bx, make_float2(xy.x, xy.y), ax), Ty = fma2(by, make_float2(xy.z, xy.w), ay);
+        const float2 F = fma2(bz, make_float2(zv.x, zv.y), az);
+        wk[k] = mul2(Ty, mul2(S, F));
+        wv[k] = mul2(wk[k], make_float2(zv.z, zv.w));
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        add_if(own + ((int)at[k] >> 16) + (at[k] & steps), ((in[k] + up) & kMask) == kIn, k & 1 ? wk[k >> 1].y : wk[k >> 1].x,
+               k & 1 ? wv[k >> 1].y : wv[k >> 1].x);
+    }
+    __syncwarp();
+  }
+  __syncwarp();
+  for (int q = lane; q < 3 * T::x * T::y * T::z; q += 32) {
+    const int comp = q / (T::x * T::y * T::z), e = q % (T::x * T::y * T::z);
+    const int x = e % T::x, y = e / T::x % T::y, z = e / (T::x * T::y);
+    const int i = x0 + x, j = y0 + y, k = z0 + z;
+    if (i >= d.nx || j >= d.ny || k >= d.nz) continue;
+    // stomp and safeDivide, as k_p2g_gather for MAC components
+    const float2 o = sm.acc[(x >> 1) + A::kY * (y >> 1) + A::kZ * (z >> 1)][8 * comp + (x & 1) + 2 * (y & 1) + 4 * (z & 1)];
+    const long long g = comp * d.n + ix(d, i, j, k);
+    const float ws = o.x < kVecEps ? 0.f : o.x;
+    const float v = ws != 0.f ? o.y / ws : o.y;
+    vel[g] = v;
+    old[g] = v;
+    if (wout) wout[g] = ws;
   }
 }
 
@@ -483,6 +891,11 @@ struct mg_particles_s {
   unsigned *hist = nullptr, *sums = nullptr, *starts = nullptr;
   float* sorted[6] = {};  // positions and up to 3 values in bucket order
   void* stage = nullptr;  // 16 bytes per particle for record transfers
+  // scratch of mapPartsToMAC's tile lists, from its first call on, and whether
+  // it could not be had
+  void* tileMem = nullptr;
+  Tiles tiles{};
+  bool tileNone = false;
 };
 
 struct mg_pdata_s {
@@ -509,7 +922,7 @@ bool valid_pdata(mg_pdata d) {
 void free_parts(mg_particles p) {
   cudaStreamSynchronize(p->st);
   void* bufs[] = {p->x, p->y, p->z, p->flag, p->keys[0], p->keys[1], p->vals[0], p->vals[1], p->hist, p->sums,
-                  p->starts, p->stage};
+                  p->starts, p->stage, p->tileMem};
   for (void* b : bufs)
     if (b) cudaFree(b);
   for (float* b : p->sorted)
@@ -579,6 +992,59 @@ SortedParts sorted_copy(mg_particles p, const unsigned* sorted, const PartView& 
   }
   SortedParts sp{p->sorted[0], p->sorted[1], p->sorted[2], {p->sorted[3], p->sorted[4], p->sorted[5]}};
   return sp;
+}
+
+// Scratch for the tile lists: room for every particle in the eight tiles that
+// it can reach.  Tiles of 8^3 from a million cells on; below, a list of 8^3
+// cells is too long a serial walk for the few tiles there are (75 x 62 x 90:
+// of 0.45 ms with the transfer back).
+bool tile_scratch(mg_particles p) {
+  if (p->tileMem || p->tileNone) return !p->tileNone;
+  Tiles& s = p->tiles;
+  s.d = p->d;
+  s.large = s.d.n >= 1000000;
+  auto across = [&](int n, int large, int small) { return s.large ? (n + large - 1) / large : (n + small - 1) / small; };
+  s.tx = across(s.d.nx, TileLarge::x, TileSmall::x);
+  s.ty = across(s.d.ny, TileLarge::y, TileSmall::y);
+  s.tz = across(s.d.nz, TileLarge::z, TileSmall::z);
+  const size_t cap = (size_t)std::max<long long>(p->cap, 1), tiles = (size_t)s.tx * s.ty * s.tz;
+  auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  p->tileNone = !s.d.is3d || s.d.nx < 3 || s.d.ny < 3 || s.d.nz < 3 || 8 * cap > 0xffffffffu || s.ty > 65535 || s.tz > 65535 ||
+                cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem(kSortShort)) != cudaSuccess ||
+                cudaFuncSetAttribute(k_tile_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem(kSortLong)) != cudaSuccess ||
+                cudaMalloc(&p->tileMem, up((tiles + 1) * 4) + tiles * kLine * 4 + 8 * cap * 4) != cudaSuccess;
+  if (p->tileNone) {
+    cudaGetLastError();
+    p->tileMem = nullptr;
+    return false;
+  }
+  s.starts = (unsigned*)p->tileMem;
+  s.cursor = (unsigned*)((char*)p->tileMem + up((tiles + 1) * 4));
+  s.list = s.cursor + tiles * kLine;
+  return true;
+}
+
+// mapPartsToMAC in 3D
+template <class T>
+void tile_mac(mg_particles p, const Tiles& s, const PartView& v, float* vel, float* old, float* w) {
+  cudaStream_t st = p->st;
+  if (s.n == 0) cudaMemsetAsync(s.starts, 0, (s.count() + 1) * sizeof(unsigned), st);
+  else {
+    cudaMemsetAsync(s.cursor, 0, (size_t)s.count() * kLine * sizeof(unsigned), st);
+    const int blocks = blocks_of(s.n);
+    count_launch();
+    k_tile_lists<T, false><<<blocks, 256, 0, st>>>(s, v);
+    count_launch();
+    k_tile_starts<<<1, 1024, 0, st>>>(s);
+    count_launch();
+    k_tile_lists<T, true><<<blocks, 256, 0, st>>>(s, v);
+    count_launch();
+    k_tile_sort<<<s.count(), kSortThreads, sort_smem(kSortShort), st>>>(s);
+    count_launch();
+    k_tile_sort_long<<<std::min(152, (s.count() + kSortThreads - 1) / kSortThreads), kSortThreads, sort_smem(kSortLong), st>>>(s);
+  }
+  count_launch();
+  k_tile_splat<T><<<dim3(s.tx, s.ty, s.tz), 32, 0, st>>>(s, v, vel, old, w);
 }
 
 PartView view_of(mg_particles p, mg_pdata ptype, int exclude) {
@@ -797,6 +1263,14 @@ extern "C" int mg_map_parts_to_mac(mg_grid flags, mg_grid vel, mg_grid velOld, m
   if (ptype && pdata_of(parts, ptype, MG_INT, what)) return MG_ERR_ARG;
   const Dims& d = parts->d;
   const PartView pv = view_of(parts, ptype, exclude);
+  if (tile_scratch(parts)) {
+    Tiles s = parts->tiles;
+    s.n = parts->n;
+    for (int c = 0; c < 3; c++) s.v[c] = partVel->c[c];
+    if (s.large) tile_mac<TileLarge>(parts, s, pv, v, vo, w);
+    else tile_mac<TileSmall>(parts, s, pv, v, vo, w);
+    return launch_status(what);
+  }
   const dim3 b(32, 8, 1);
   for (int c = 0; c < 3; c++) {
     const unsigned* sorted = sort_stencil(parts, c, pv);
