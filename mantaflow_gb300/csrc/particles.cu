@@ -437,15 +437,19 @@ __global__ void __launch_bounds__(256) k_p2g_gather(Dims d, int comp, SortedPart
 // particles that reach the tile, in particle order.  So: list those (a
 // particle near a tile's border is in up to eight lists: 1.9 on average with
 // 8 x 8 x 4 cells, 2.6 with 4^3), put every list into particle order, and let
-// one warp per tile walk its list.  Lane 8 c + k of it holds corner k of
-// component c: it reads the particle's three weights and value of that
-// component, forms its corner's weight as the reference does, and adds to its
-// face in shared memory, about 20 instructions for a particle's 24 faces.  The
-// weights come from a batch of 32 particles whose lanes prepared one each.
+// one warp per tile walk its list.  Lane 8 c + k of it owns the faces of
+// component c and parity k: it reads the particle's three weights and value of
+// that component, forms its face's weight as the reference does, and adds in
+// shared memory, about 20 instructions for a particle's 24 faces.  The weights
+// come from a batch of 32 particles whose lanes prepared one each.
 //
 // At 128^3 with 16.8 M particles mapPartsToMAC took 5.5 ms with a radix sort
 // and eight-way merges per component (3.2 ms of it in the merges, about 100
-// instructions per contribution); FIGURES
+// instructions per contribution); now 1.5 ms: lists 0.11 + 0.16, sort 0.38,
+// splat 0.9.  The splat is bound by shared memory, ten wavefronts per particle
+// of a tile (95 % of the rate), the sort by its instructions.  With particles
+// in random order the lists' atomics and the loads by index weigh more: 10.8 M
+// in 108 x 125 x 100 take 3.3 ms (before: 5.8), in seeding order 0.95 (3.8).
 template <int X, int Y, int Z>
 struct TileShape {
   static constexpr int x = X, y = Y, z = Z;
@@ -493,7 +497,8 @@ __device__ __forceinline__ int axis_sample(float q, int n) {
 // of all three components lie in at most 2 x 2 x 2 tiles.  The lanes of a warp
 // with the same tile take it with one atomic; particles in flight are mostly
 // neighbours, so each tile's counter has a line of its own (side by side, the
-// atomics queue at a few L2 slices: 295 and 361 us at 128^3, now FIGURES2).
+// atomics queue at a few L2 slices: 295 and 361 us at 128^3, now 110
+// and 156).
 template <class T, bool kFill>
 __global__ void __launch_bounds__(256) k_tile_lists(Tiles s, PartView p) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -995,9 +1000,10 @@ SortedParts sorted_copy(mg_particles p, const unsigned* sorted, const PartView& 
 }
 
 // Scratch for the tile lists: room for every particle in the eight tiles that
-// it can reach.  Tiles of 8^3 from a million cells on; below, a list of 8^3
-// cells is too long a serial walk for the few tiles there are (75 x 62 x 90:
-// of 0.45 ms with the transfer back).
+// it can reach.  The larger tiles from a million cells on: with the small ones
+// 128^3 takes 2.31 instead of 1.58 ms.  Below, a large tile's list is too long
+// a serial walk for the few tiles there are (75 x 62 x 90: 0.52 instead of
+// 0.45 ms with the transfer back).
 bool tile_scratch(mg_particles p) {
   if (p->tileMem || p->tileNone) return !p->tileNone;
   Tiles& s = p->tiles;
