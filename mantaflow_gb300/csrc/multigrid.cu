@@ -337,15 +337,7 @@ __global__ void k_mg_coarse_op(Lev C, Lev F, int S) {
 // their terms subtract zero and need no type test.  The loads of one z-plane
 // of the stencil (9 matrix entries, 9 values) are issued together before
 // its subtractions; the chain of float operations is the reference's.
-// vectors that other CTAs of the same launch write (the cluster V-cycle
-// below) are read at L2, past the SM's non-coherent L1
-template <bool CG>
-__device__ __forceinline__ float ldv(const float* p) {
-  if (CG) return __ldcg(p);
-  return *p;
-}
-
-template <bool IS3D, bool SKIP_CENTER, bool CG = false>
+template <bool IS3D, bool SKIP_CENTER>
 __device__ __forceinline__ float stencil_sub(const Lev& L, int vx, int vy, int vz, long long v, float sum) {
   constexpr int ZL = IS3D ? -1 : 0, ZH = IS3D ? 1 : 0;
   constexpr int S = IS3D ? 14 : 5;
@@ -364,40 +356,12 @@ __device__ __forceinline__ float stencil_sub(const Lev& L, int vx, int vy, int v
         in[q] = o.ix[dx + 1] && o.iy[dy + 1] && o.iz[dz + 1] && !(SKIP_CENTER && s == S - 1);
         const int nn = in[q] ? vi + o.ox[dx + 1] + o.oy[dy + 1] + o.oz[dz + 1] : vi;
         a[q] = s < S ? L.A[(long long)(S - 1 - s) * L.n + nn] : L.A[(long long)(s - S + 1) * L.n + vi];
-        xv[q] = ldv<CG>(&L.x[nn]);
+        xv[q] = L.x[nn];
       }
 #pragma unroll
     for (int q = 0; q < 9; q++)
       if (in[q]) sum = sum - a[q] * xv[q];
   }
-  return sum;
-}
-
-// The same sum with every load of the stencil (and of the centre's type,
-// right-hand side and diagonal) issued before any arithmetic: one memory
-// round trip per vertex, for the cluster tail, whose passes have about one
-// vertex per thread and nothing else to overlap the latency with.
-// Levels in the tail have few slots (kTailSlots): offsets are 32-bit.
-template <bool IS3D, bool SKIP_CENTER>
-__device__ __forceinline__ float stencil_sub_flat(const Lev& L, int vx, int vy, int vz, int v, float sum) {
-  constexpr int NZ = IS3D ? 3 : 1, ZL = IS3D ? -1 : 0;
-  constexpr int S = IS3D ? 14 : 5;
-  const int n = (int)L.n;
-  const Nb3 o = nb3(L, vx, vy, vz);  // L is colour-blocked
-  float a[NZ * 9], xv[NZ * 9];
-  unsigned inm = 0;
-#pragma unroll
-  for (int s = 0; s < NZ * 9; s++) {
-    const int dx = s % 3, dy = (s / 3) % 3, dz = s / 9 + ZL + 1;
-    const bool in = o.ix[dx] && o.iy[dy] && o.iz[dz] && !(SKIP_CENTER && s == S - 1);
-    inm |= in ? 1u << s : 0u;
-    const int nn = in ? v + o.ox[dx] + o.oy[dy] + o.oz[dz] : v;
-    a[s] = s < S ? L.A[(S - 1 - s) * n + nn] : L.A[(s - S + 1) * n + v];
-    xv[s] = __ldcg(&L.x[nn]);
-  }
-#pragma unroll
-  for (int s = 0; s < NZ * 9; s++)
-    if (inm & (1u << s)) sum = sum - a[s] * xv[s];
   return sum;
 }
 
@@ -530,7 +494,7 @@ __global__ void __launch_bounds__(256) k_dict_verify(Lev L, const uint16_t* sid,
 
 // stencil_sub with the coefficients from the dictionary tuple t (CG: x is
 // written by other CTAs of the same launch and read at L2)
-template <bool IS3D, bool SKIP_CENTER, bool CG = false>
+template <bool IS3D, bool SKIP_CENTER>
 __device__ __forceinline__ float stencil_sub_dict(const Lev& L, const float* __restrict__ t, int vx, int vy, int vz,
                                                   float sum) {
   constexpr int ZL = IS3D ? -1 : 0, ZH = IS3D ? 1 : 0;
@@ -549,7 +513,7 @@ __device__ __forceinline__ float stencil_sub_dict(const Lev& L, const float* __r
         const int s = (dz - ZL) * 9 + q;
         in[q] = o.ix[dx + 1] && o.iy[dy + 1] && o.iz[dz + 1] && !(SKIP_CENTER && s == S - 1);
         a[q] = t[s];
-        xv[q] = in[q] ? ldv<CG>(&L.x[vi + o.ox[dx + 1] + o.oy[dy + 1] + o.oz[dz + 1]]) : 0.f;
+        xv[q] = in[q] ? L.x[vi + o.ox[dx + 1] + o.oy[dy + 1] + o.oz[dz + 1]] : 0.f;
       }
 #pragma unroll
     for (int q = 0; q < 9; q++)
@@ -560,7 +524,7 @@ __device__ __forceinline__ float stencil_sub_dict(const Lev& L, const float* __r
 
 // knSmoothColor on a coarse level, one vertex: block bi of colour offset
 // (ox, oy, oz) in 2x2x2 blocks, bx x by blocks per z-plane
-template <bool IS3D, bool CG>
+template <bool IS3D>
 __device__ __forceinline__ void smooth_vertex(const Lev& L, long long bi, int ox, int oy, int oz, int bx, int by) {
   int vx, vy, vz;
   block_xyz(bi, bx, by, vx, vy, vz);
@@ -570,76 +534,22 @@ __device__ __forceinline__ void smooth_vertex(const Lev& L, long long bi, int ox
   if (!inside(L, vx, vy, vz)) return;
   const long long v = L.colored ? (long long)(ox | (oy << 1) | (oz << 2)) * L.nb + bi : lin(L, vx, vy, vz);
   if (L.type[v] == kVtInactive) return;
-  const float sum = stencil_sub<IS3D, true, CG>(L, vx, vy, vz, v, ldv<CG>(&L.b[v]));
+  const float sum = stencil_sub<IS3D, true>(L, vx, vy, vz, v, L.b[v]);
   L.x[v] = sum / L.A[v];
 }
 
-// smooth_vertex for the cluster tail: the vertex type is tested after all
-// loads were issued (inactive vertices only cost loads)
-template <bool IS3D>
-__device__ __forceinline__ void smooth_vertex_flat(const Lev& L, long long bi, int ox, int oy, int oz, int bx, int by) {
-  int vx, vy, vz;
-  block_xyz(bi, bx, by, vx, vy, vz);
-  vx = 2 * vx + ox;
-  vy = 2 * vy + oy;
-  vz = 2 * vz + oz;
-  if (!inside(L, vx, vy, vz)) return;
-  const long long v = L.colored ? (long long)(ox | (oy << 1) | (oz << 2)) * L.nb + bi : lin(L, vx, vy, vz);
-  const int8_t ty = L.type[v];
-  const float diag = L.A[v];
-  const float sum = stencil_sub_flat<IS3D, true>(L, vx, vy, vz, (int)v, __ldcg(&L.b[v]));
-  if (ty != kVtInactive) L.x[v] = sum / diag;
-}
-
-template <bool IS3D>
-__device__ __forceinline__ void residual_vertex_flat(const Lev& L, long long v) {
-  int vx, vy, vz;
-  coords(L, v, vx, vy, vz);
-  const int8_t ty = L.type[v];
-  const float r = stencil_sub_flat<IS3D, false>(L, vx, vy, vz, (int)v, __ldcg(&L.b[v]));
-  if (ty != kVtInactive) L.r[v] = r;
-}
-
-// the same two passes for the cluster tail on a level with a stencil
-// dictionary: the vertex's id, then its tuple and every x at once
-template <bool IS3D>
-__device__ __forceinline__ void smooth_vertex_dict_flat(const Lev& L, long long bi, int ox, int oy, int oz, int bx, int by) {
-  constexpr int S = IS3D ? 14 : 5;
-  int vx, vy, vz;
-  block_xyz(bi, bx, by, vx, vy, vz);
-  vx = 2 * vx + ox;
-  vy = 2 * vy + oy;
-  vz = 2 * vz + oz;
-  if (!inside(L, vx, vy, vz)) return;
-  const long long v = (long long)(ox | (oy << 1) | (oz << 2)) * L.nb + bi;
-  const int8_t ty = L.type[v];
-  const float* t = L.T + (int)L.sid[v] * kDictStride;
-  const float sum = stencil_sub_dict<IS3D, true, true>(L, t, vx, vy, vz, __ldcg(&L.b[v]));
-  if (ty != kVtInactive) L.x[v] = sum / t[S - 1];
-}
-template <bool IS3D>
-__device__ __forceinline__ void residual_vertex_dict_flat(const Lev& L, long long v) {
-  int vx, vy, vz;
-  coords(L, v, vx, vy, vz);
-  if (!inside(L, vx, vy, vz)) return;  // padding slot
-  const int8_t ty = L.type[v];
-  const float* t = L.T + (int)L.sid[v] * kDictStride;
-  const float r = stencil_sub_dict<IS3D, false, true>(L, t, vx, vy, vz, __ldcg(&L.b[v]));
-  if (ty != kVtInactive) L.r[v] = r;
-}
-
 // knCalcResidual on a coarse level, one storage slot
-template <bool IS3D, bool CG>
+template <bool IS3D>
 __device__ __forceinline__ void residual_vertex(const Lev& L, long long v) {
   if (L.type[v] == kVtInactive) return;
   int vx, vy, vz;
   coords(L, v, vx, vy, vz);
-  L.r[v] = stencil_sub<IS3D, false, CG>(L, vx, vy, vz, v, ldv<CG>(&L.b[v]));
+  L.r[v] = stencil_sub<IS3D, false>(L, vx, vy, vz, v, L.b[v]);
 }
 
 // knRestrict into slot v of level D from the level below (level 0 when
 // FROM0), plus knSet(x[D], 0) of the next smoothing's initial guess
-template <bool FROM0, bool CG>
+template <bool FROM0>
 __device__ __forceinline__ void restrict_vertex_at(const Lev& D, const Lev& S, const Lev0& F, long long v, int vx, int vy,
                                                    int vz) {
   const int sx = FROM0 ? F.d.nx : S.sx, sy = FROM0 ? F.d.ny : S.sy, sz = FROM0 ? F.d.nz : S.sz;
@@ -655,7 +565,7 @@ __device__ __forceinline__ void restrict_vertex_at(const Lev& D, const Lev& S, c
     const int rx = 2 * vx - 1 + q % 3, ry = 2 * vy - 1 + (q / 3) % 3, rz = 2 * vz - 1 + q / 9;
     in[q] = rx >= 0 && ry >= 0 && rz >= 0 && rx < sx && ry < sy && rz < sz;
     // inactive fine vertices hold r = 0: adding their term adds zero
-    rv[q] = in[q] ? (FROM0 ? F.r[rx + py * ry + pz * rz] : ldv<CG>(&S.r[lin(S, rx, ry, rz)])) : 0.f;
+    rv[q] = in[q] ? (FROM0 ? F.r[rx + py * ry + pz * rz] : S.r[lin(S, rx, ry, rz)]) : 0.f;
   }
   float sum = 0.f;
 #pragma unroll
@@ -665,15 +575,15 @@ __device__ __forceinline__ void restrict_vertex_at(const Lev& D, const Lev& S, c
   }
   if (ty != kVtInactive) D.b[v] = sum;
 }
-template <bool FROM0, bool CG>
+template <bool FROM0>
 __device__ __forceinline__ void restrict_vertex(const Lev& D, const Lev& S, const Lev0& F, long long v) {
   int vx, vy, vz;
   coords(D, v, vx, vy, vz);
-  restrict_vertex_at<FROM0, CG>(D, S, F, v, vx, vy, vz);
+  restrict_vertex_at<FROM0>(D, S, F, v, vx, vy, vz);
 }
 
 // knInterpolate from level S = D+1 and knAddAssign: x[D] += I * x[S]
-template <bool IS3D, bool CG>
+template <bool IS3D>
 __device__ __forceinline__ void interp_vertex(const Lev& D, const Lev& S, long long v) {
   const int8_t ty = D.type[v];
   int vx, vy, vz;
@@ -687,15 +597,16 @@ __device__ __forceinline__ void interp_vertex(const Lev& D, const Lev& S, long l
   for (int q = 0; q < 8; q++) {
     const int ox = q & 1, oy = (q >> 1) & 1, oz = q >> 2;
     const bool use = (ox <= hx) && (oy <= hy) && (oz <= hz);
-    cv[q] = use ? ldv<CG>(&S.x[lin(S, vx / 2 + ox, vy / 2 + oy, vz / 2 + oz)]) : 0.f;
+    cv[q] = S.x[use ? lin(S, vx / 2 + ox, vy / 2 + oy, vz / 2 + oz) : 0];
   }
+  const float dx = D.x[v];
   float sum = 0.f;
 #pragma unroll
   for (int q = 0; q < 8; q++) {
     const int ox = q & 1, oy = (q >> 1) & 1, oz = q >> 2;
     if ((ox <= hx) && (oy <= hy) && (oz <= hz)) sum = sum + cv[q];
   }
-  const float xv = ldv<CG>(&D.x[v]) + inv_pow2(parity3(vx, vy, vz)) * sum;
+  const float xv = dx + inv_pow2(parity3(vx, vy, vz)) * sum;
   if (ty != kVtInactive) D.x[v] = xv;
 }
 
@@ -704,13 +615,13 @@ __global__ void __launch_bounds__(256, 3) k_mg_smooth(Lev L, int S, int ox, int 
   if (sc->done) return;
   const int bx = (L.sx + 1) / 2, by = (L.sy + 1) / 2, bz = (L.sz + 1) / 2;
   const long long nb = (long long)bx * by * bz;
-  GRID_STRIDE(bi, nb) smooth_vertex<IS3D, false>(L, bi, ox, oy, oz, bx, by);
+  GRID_STRIDE(bi, nb) smooth_vertex<IS3D>(L, bi, ox, oy, oz, bx, by);
 }
 
 template <bool IS3D>
 __global__ void __launch_bounds__(256, 3) k_mg_residual(Lev L, int S, const CgScalars* sc) {
   if (sc->done) return;
-  GRID_STRIDE(v, L.n) residual_vertex<IS3D, false>(L, v);
+  GRID_STRIDE(v, L.n) residual_vertex<IS3D>(L, v);
 }
 
 // the same passes on a level with a stencil dictionary
@@ -754,7 +665,7 @@ __global__ void __launch_bounds__(256, 4) k_mg_residual_dict(Lev L, const CgScal
 template <bool FROM0>
 __global__ void __launch_bounds__(256) k_mg_restrict(Lev D, Lev S, Lev0 F, const CgScalars* sc) {
   if (sc->done) return;
-  GRID_STRIDE(v, D.n) restrict_vertex<FROM0, false>(D, S, F, v);
+  GRID_STRIDE(v, D.n) restrict_vertex<FROM0>(D, S, F, v);
 }
 
 // restriction from level 0 with threads in x-fastest coarse order over a
@@ -765,13 +676,13 @@ __global__ void __launch_bounds__(256) k_mg_restrict0(Lev D, Lev0 F, const CgSca
   const unsigned e = blockIdx.x * 256u + threadIdx.x;  // a coarse plane holds < 2^31 vertices
   if (e >= (unsigned)D.sx * (unsigned)D.sy) return;
   const int vy = (int)(e / (unsigned)D.sx), vx = (int)(e - (unsigned)vy * (unsigned)D.sx), vz = blockIdx.y;
-  restrict_vertex_at<true, false>(D, D, F, lin(D, vx, vy, vz), vx, vy, vz);
+  restrict_vertex_at<true>(D, D, F, lin(D, vx, vy, vz), vx, vy, vz);
 }
 
 template <bool IS3D>
 __global__ void __launch_bounds__(256) k_mg_interp_add(Lev D, Lev S, const CgScalars* sc) {
   if (sc->done) return;
-  GRID_STRIDE(v, D.n) interp_vertex<IS3D, false>(D, S, v);
+  GRID_STRIDE(v, D.n) interp_vertex<IS3D>(D, S, v);
 }
 
 // ---- fused level-0 passes, streamed along z.  A CTA of 512 threads owns
@@ -1229,21 +1140,38 @@ constexpr size_t kCgDynSmem = (size_t)kCgNb * kCgThreads * (sizeof(float) + size
 // here a hardware cluster barrier.  Every pass does the per-vertex float
 // operations of the separate kernels above (the same device functions), so
 // the levels' results are bit-identical to them; vectors written inside
-// the launch are read at L2 (ldv<true>).
-constexpr int kTailThreads = 384;
-constexpr int kTailMaxCta = 16;
-constexpr int kTailVpc = 128;  // coarsest-level vertices per CTA (<= 1024 over >= 8 CTAs)
-constexpr long long kTailSlots = 100000;  // largest level run inside the cluster (33^3 and below)
+// the launch are read at L2 (tail_ld).
+constexpr int kTailThreads = 512;
+// Largest level run inside the cluster, in storage slots.  With 57^3 (195 000)
+// in it a solve at 112^3 takes 2.26 ms instead of 1.89, with 41 x 50 x 36
+// (74 000) one at 161 x 199 x 143 as long as without (3.38 and 3.40 ms), with
+// the levels of 33^3 outside one at 256^3 0.25 ms longer.
+constexpr long long kTailSlots = 100000;
+constexpr int kCoarseMax = 2 * kTailThreads;  // coarsest-level vertices
 
-struct TailSmem {
-  float coef[kCgNb][kTailVpc];  // own vertices' stencils (applyAStencil order)
-  short nbr[kCgNb][kTailVpc];
-  unsigned char nn[kTailVpc];
-  float ph[kCgThreads], pl[kCgThreads];  // the whole search vector p
-  float zh[kCgThreads], zl[kCgThreads];  // the whole z: every CTA stores its share into every CTA
-  ff wpart[kTailThreads / 32][2];        // per-warp partial dot products
-  ff cpart[kTailMaxCta][3];              // per-CTA partials (rr, rz | pq), stored by each CTA into every CTA
-};
+// A value that other CTAs of the launch write, and one that nobody writes.
+// Volatile: the compiler would move the loads of a pass behind the barrier that
+// hides them and to their uses, one by one (a pass then takes twice as long).
+__device__ __forceinline__ float tail_ld(const float* p) {
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float tail_ld_const(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 tail_ld_const(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int tail_ld_const(const uint16_t* p) {
+  unsigned short v;
+  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
 
 // f1 < f2 for normalised pairs
 __device__ __forceinline__ bool ff_lt(ff a, ff b) { return a.h < b.h || (a.h == b.h && a.l < b.l); }
@@ -1255,233 +1183,402 @@ __device__ __forceinline__ ff ff_div(ff a, ff b) {
   return quick_two_sum(q1, q2);
 }
 
-// The CTA's sums of NV pairs held by the lanes with sub == 0 (zero
-// elsewhere), stored into cpart[rank][slot..] of every CTA of the cluster;
-// the caller's cluster barrier publishes them.  The pq slot is apart from
-// the rr / rz slots: a CTA may store the next phase's sums while another
-// still reads this phase's.
+struct CoarseSmem {
+  float2 p[kCoarseMax + 256];     // search vector, and zeros as far as the stencils reach
+  ff part[3][kTailThreads / 32];  // per-warp partial dot products
+};
+constexpr int kCoarseCoefBytes = sizeof(float) * kCgNb * kCoarseMax;  // stencils, entry by entry
+
+// the barrier of the first `warps` warps
+__device__ __forceinline__ void coarse_sync(int warps) { asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory"); }
+
+// Sums over those warps of each thread's NV values, one or two.  The sums carry
+// their rounding errors in l and are normalised at the end (a butterfly step is
+// then a shuffle and one dependent addition).  Of two values, the lower lanes
+// add up the first and the upper ones the second.  Every warp adds up the same
+// partials in the same order, so all threads get the same bits.  A slot is
+// written again only two barriers after its last reading.
 template <int NV>
-__device__ __forceinline__ void tail_push_sums(cooperative_groups::cluster_group& cl, TailSmem& sm, ff* v, int tpv,
-                                               int slot) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int o = 16; o >= tpv; o >>= 1)
+__device__ __forceinline__ void coarse_dots(CoarseSmem& sm, int warps, int slot, ff* v) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool second = NV == 2 && lane >= 16;
+  auto add = [](ff a, ff b) {
+    const ff s = two_sum(a.h, b.h);
+    return ff{s.h, (a.l + b.l) + s.l};
+  };
+  auto across = [](ff a, int o) { return ff{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)}; };
+  auto from = [](ff a, int l) { return ff{__shfl_sync(0xffffffffu, a.h, l), __shfl_sync(0xffffffffu, a.l, l)}; };
+  ff s = add(second ? v[NV - 1] : v[0], across(NV == 2 && !second ? v[NV - 1] : v[0], 16));
 #pragma unroll
-    for (int q = 0; q < NV; q++) {
-      const ff w{__shfl_xor_sync(0xffffffffu, v[q].h, o), __shfl_xor_sync(0xffffffffu, v[q].l, o)};
-      v[q] = ff_add(v[q], w);
+  for (int o = 8; o > 0; o >>= 1) s = add(s, across(s, o));
+  if ((lane & 15) == 0 && (NV == 2 || lane == 0)) sm.part[slot + second][w] = s;
+  coarse_sync(warps);
+  s = (lane & 15) < warps ? sm.part[slot + second][lane & 15] : ff{0.f, 0.f};
+  if (warps > 8) s = add(s, across(s, 8));
+  if (warps > 4) s = add(s, across(s, 4));
+  if (warps > 2) s = add(s, across(s, 2));
+  s = add(s, across(s, 1));
+  s = two_sum(s.h, s.l);
+  v[0] = from(s, 0);
+  if (NV == 2) v[NV - 1] = from(s, 16);
+}
+
+// GridMg::solveCG (multigrid.cpp:793-902) on the coarsest level in one CTA.
+// Each iteration is a chain of two dot products and three barriers, so what
+// counts is latency: spread over the cluster, with two cluster barriers, it
+// took 4.6 us for 288 vertices and 50 iterations to a solve (240 of the 345 us
+// of a launch); here 2 us (3 us for 729 vertices).  A thread has K vertices, t and t + threads, in an
+// order with the longest axis last, so that a neighbour is a fixed, short step
+// away in the search vector.  Absent neighbours have coefficient zero.
+// Vectors, dot products and scalars are double-float pairs on the FP32 pipe
+// (the stencil product is a compensated sum of exact float products); the
+// iterates follow an IEEE-double CG to ~1e-14 relative.
+template <bool IS3D, int K>
+__device__ void coarse_cg(const Lev& L, int S, float accuracy, CoarseSmem& sm, float* coef) {
+  constexpr int NZ = IS3D ? 3 : 1, E = 9 * NZ;
+  constexpr int NA = IS3D ? 3 : 2;
+  const int n = L.sx * L.sy * L.sz, t = threadIdx.x;
+  const int len[3] = {L.sx, L.sy, IS3D ? L.sz : 1};
+  // strides of vertices and of stencil entries, axes by length: 1, a, a * b; 1, 3, 9
+  int st[3] = {1, 1, IS3D ? 1 : n}, es[3] = {1, 1, IS3D ? 1 : 0}, s1 = 0, s2 = 0;
+#pragma unroll
+  for (int q = 0; q < NA; q++) {
+    for (int o = 0; o < NA; o++)
+      if (o != q && (len[o] < len[q] || (len[o] == len[q] && o < q))) {
+        st[q] *= len[o];
+        es[q] *= 3;
+      }
+    if (es[q] == 3) s1 = st[q];
+    if (es[q] == 9) s2 = st[q];
+  }
+  const int reach = 1 + s1 + s2;
+  auto place = [&](int u, int& x, int& y, int& z) {
+    x = u / st[0] % len[0];
+    y = u / st[1] % len[1];
+    z = u / st[2] % len[2];
+  };
+  // the stencils, nine entries' loads at a time
+  for (int u0 = t; u0 < ((n + 31) & ~31); u0 += blockDim.x) {
+    const int u = min(u0, n - 1);
+    int x, y, z;
+    place(u, x, y, z);
+    const int v = (int)lin(L, x, y, z), ln = (int)L.n;
+    const bool act = L.type[v] != kVtInactive;
+    for (int dz = 0; dz < NZ; dz++) {
+      float a[9];
+      int8_t type[9];
+#pragma unroll
+      for (int e = 0; e < 9; e++) {
+        const int nx = x + e % 3 - 1, ny = y + e / 3 - 1, nz = z + (IS3D ? dz - 1 : 0), s = 9 * dz + e;
+        const bool in = inside(L, nx, ny, nz);
+        const int q = in ? (int)lin(L, nx, ny, nz) : v;
+        type[e] = in ? L.type[q] : (int8_t)kVtInactive;
+        a[e] = tail_ld_const(s < S ? L.A + (S - 1 - s) * ln + q : L.A + (s - S + 1) * ln + v);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int e = 0; e < 9; e++)
+        coef[(e % 3 * es[0] + e / 3 * es[1] + dz * es[2]) * kCoarseMax + u] = act && type[e] != kVtInactive ? a[e] : 0.f;
     }
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < NV; q++) sm.wpart[wid][q] = v[q];
+  }
+  for (int q = t; q < n + 2 * reach; q += blockDim.x) sm.p[q] = make_float2(0.f, 0.f);
   __syncthreads();
-  if (wid == 0) {
-    const int ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int threads = (n + K - 1) / K, warps = (threads + 31) / 32;
+  if (t >= 32 * warps) return;
+  long long slot[K];
+  float dg[K], bv[K];
+  ff inv[K], x[K], r[K], z[K], p[K];
 #pragma unroll
-    for (int q = 0; q < NV; q++) {
-      ff t = lane < nw ? sm.wpart[lane][q] : ff{0.f, 0.f};
-      for (int o = 16; o > 0; o >>= 1) {
-        const ff w{__shfl_xor_sync(0xffffffffu, t.h, o), __shfl_xor_sync(0xffffffffu, t.l, o)};
-        t = ff_add(t, w);
-      }
-      if (lane < ncta) *cl.map_shared_rank(&sm.cpart[rank][slot + q], lane) = t;
+  for (int k = 0; k < K; k++) {
+    const int u = t + k * threads;
+    const bool ok = t < threads && u < n;
+    int vx, vy, vz;
+    place(ok ? u : 0, vx, vy, vz);
+    const long long v = lin(L, vx, vy, vz);
+    const bool act = ok && L.type[v] != kVtInactive;
+    dg[k] = L.A[v];
+    bv[k] = __ldcg(&L.b[v]);
+    slot[k] = ok ? v : -1;
+    if (!act) {
+      dg[k] = 1.f;
+      bv[k] = 0.f;
     }
+    inv[k].h = 1.f / dg[k];
+    inv[k].l = fmaf(-dg[k], inv[k].h, 1.f) / dg[k];
+    // x = 0, so r = b - A*0 = b
+    x[k] = ff{0.f, 0.f};
+    r[k] = ff{bv[k], 0.f};
+    p[k] = z[k] = ff_mul(r[k], inv[k]);
   }
-}
-
-// after the cluster barrier: the cluster's sum of cpart[.][q], summed in
-// the same order in every warp of every CTA (identical bits everywhere)
-__device__ __forceinline__ ff tail_total(const TailSmem& sm, int q, int ncta) {
-  const int lane = threadIdx.x & 31;
-  ff t = lane < ncta ? sm.cpart[lane][q] : ff{0.f, 0.f};
-  for (int o = 16; o > 0; o >>= 1) {
-    const ff w{__shfl_xor_sync(0xffffffffu, t.h, o), __shfl_xor_sync(0xffffffffu, t.l, o)};
-    t = ff_add(t, w);
-  }
-  return t;
-}
-
-// this CTA's z values into zh/zl of every CTA (the tpv lanes of a vertex
-// hold the same z and share its stores)
-__device__ __forceinline__ void tail_push_z(cooperative_groups::cluster_group& cl, TailSmem& sm, bool own, int v, int sub,
-                                            int tpv, ff z) {
-  if (!own) return;
-  const int ncta = (int)cl.num_blocks();
-  for (int rk = sub; rk < ncta; rk += tpv) {
-    *cl.map_shared_rank(&sm.zh[v], rk) = z.h;
-    *cl.map_shared_rank(&sm.zl[v], rk) = z.l;
-  }
-}
-
-// GridMg::solveCG (multigrid.cpp:793-902) on the coarsest level across the
-// cluster: CTA c owns vertices [c*vpc, (c+1)*vpc), tpv threads per vertex
-// split its stencil.  Each CTA stores its partial dot products and its z
-// values into the shared memory of every CTA before a cluster barrier, so
-// every CTA then holds the whole z (and rebuilds the whole p) and all
-// partials; an iteration has two barriers and no remote loads.  Vectors,
-// dot products and scalars are double-float pairs on the FP32 pipe (the
-// stencil product is a compensated sum of exact float products); the
-// iterates follow an IEEE-double CG to ~1e-14 relative.  Every warp forms
-// the scalars from the same rank-ordered sums, so all CTAs take the same
-// branches.
-template <bool IS3D>
-__device__ void tail_coarse_cg(cooperative_groups::cluster_group& cl, const Lev& L, int S, float accuracy, TailSmem& sm) {
-  const int ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  const int n = (int)L.n;
-  const int vpc = (n + ncta - 1) / ncta;
-  int tpv = 8;
-  while (tpv > 1 && tpv * vpc > (int)blockDim.x) tpv >>= 1;
-  const int lv = threadIdx.x / tpv, sub = threadIdx.x % tpv;
-  const int v = rank * vpc + lv;
-  const bool own = lv < vpc && v < n;
-  bool act = false;
-  float diag = 1.f, bv = 0.f;
-  if (own) {
-    act = L.type[v] != kVtInactive;
-    if (act) {
-      diag = L.A[v];
-      bv = __ldcg(&L.b[v]);
-    }
-    if (sub == 0) {
-      int nn = 0;
-      if (act) {
-        constexpr int ZL = IS3D ? -1 : 0, ZH = IS3D ? 1 : 0;
-        int vx, vy, vz;
-        coords(L, v, vx, vy, vz);
-        int s = 0;
-        for (int dz = ZL; dz <= ZH; dz++)
-          for (int dy = -1; dy <= 1; dy++)
-            for (int dx = -1; dx <= 1; dx++, s++) {
-              const int nx = vx + dx, ny = vy + dy, nz = vz + dz;
-              if (!inside(L, nx, ny, nz)) continue;
-              const int q = (int)lin(L, nx, ny, nz);
-              if (L.type[q] == kVtInactive) continue;
-              sm.coef[nn][lv] = s < S ? L.A[(long long)(S - 1 - s) * L.n + q] : L.A[(long long)(s - S + 1) * L.n + v];
-              sm.nbr[nn][lv] = (short)q;
-              nn++;
-            }
-      }
-      sm.nn[lv] = (unsigned char)nn;
-    }
-  }
-  const bool lead = act && sub == 0;
-  // x = 0, so r = b - A*0 = b
-  ff x{0.f, 0.f}, r{0.f, 0.f}, z{0.f, 0.f};
-  if (act) {
-    r = ff{bv, 0.f};
-    z = ff_div_f(r, diag);
-  }
-  tail_push_z(cl, sm, own, v, sub, tpv, z);
-  {
-    ff t[2] = {lead ? ff_mul(r, r) : ff{0.f, 0.f}, lead ? ff_mul(r, z) : ff{0.f, 0.f}};
-    tail_push_sums<2>(cl, sm, t, tpv, 0);
-  }
-  cl.sync();
-  const ff rr0 = tail_total(sm, 0, ncta);
-  ff alphaTop = tail_total(sm, 1, ncta);
+  auto publish = [&]() {
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (slot[k] >= 0) sm.p[reach + t + k * threads] = make_float2(p[k].h, p[k].l);
+  };
+  auto dot = [&](const ff* a, const ff* b) {
+    ff s = ff_mul(a[0], b[0]);
+    if (K == 2) s = ff_add(s, ff_mul(a[K - 1], b[K - 1]));
+    return s;
+  };
+  ff d[2] = {dot(r, r), dot(r, z)};
+  coarse_dots<2>(sm, warps, 1, d);
+  const ff rr0 = d[0];
+  ff alphaTop = d[1];
   // residual / initialResidual < accuracy  <=>  rr < rr0 * accuracy^2
   const ff stopAt = ff_mul(rr0, two_prod(accuracy, accuracy));
-  for (int u = threadIdx.x; u < n; u += blockDim.x) {  // p = z
-    sm.ph[u] = sm.zh[u];
-    sm.pl[u] = sm.zl[u];
-  }
-  __syncthreads();
-  const int nn = own ? sm.nn[lv] : 0;
+  publish();
+  coarse_sync(warps);
   // initialResidual > 1e-12
   for (int iter = 0; iter < 10000 && rr0.h > 1e-24f; iter++) {
-    // q = A p: this lane's share of the stencil as a compensated sum, then
-    // the vertex's lanes
-    float qs = 0.f, qe = 0.f;
-    for (int e = sub; e < nn; e += tpv) {
-      const int k = sm.nbr[e][lv];
-      const float c = sm.coef[e][lv];
-      const ff pr = two_prod(c, sm.ph[k]);
-      const ff t = two_sum(qs, pr.h);
-      qs = t.h;
-      qe = qe + (t.l + (pr.l + c * sm.pl[k]));
-    }
-    ff q = two_sum(qs, qe);
-    for (int o = tpv >> 1; o > 0; o >>= 1) {
-      const ff w{__shfl_xor_sync(0xffffffffu, q.h, o), __shfl_xor_sync(0xffffffffu, q.l, o)};
-      q = ff_add(q, w);
-    }
-    const ff p = own ? ff{sm.ph[v], sm.pl[v]} : ff{0.f, 0.f};
-    {
-      ff t[1] = {lead ? ff_mul(p, q) : ff{0.f, 0.f}};
-      tail_push_sums<1>(cl, sm, t, tpv, 2);
-    }
-    cl.sync();
-    const ff alpha = ff_div(alphaTop, tail_total(sm, 2, ncta));
-    ff t[2] = {ff{0.f, 0.f}, ff{0.f, 0.f}};
-    if (act) {
-      x = ff_add(x, ff_mul(alpha, p));
-      r = ff_add(r, ff_neg(ff_mul(alpha, q)));
-      z = ff_div_f(r, diag);
-      if (sub == 0) {
-        t[0] = ff_mul(r, r);
-        t[1] = ff_mul(r, z);
+    // q = A p: three compensated sums at a time
+    ff q[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const int u = slot[k] >= 0 ? t + k * threads : 0;
+      const float2* const own = sm.p + reach + u;
+      const float* const cf = coef + u;
+      ff acc[3] = {};
+#pragma unroll
+      for (int row = 0; row < E / 3; row++) {
+        const float2* const f = own + (row % 3 - 1) * s1 + (IS3D ? (row / 3 - 1) * s2 : 0);
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+          const float c = cf[(3 * row + e) * kCoarseMax];
+          const ff pr = two_prod(c, f[e - 1].x), s = two_sum(acc[e].h, pr.h);
+          acc[e] = ff{s.h, acc[e].l + (s.l + fmaf(c, f[e - 1].y, pr.l))};
+        }
       }
+      const ff t1 = two_sum(acc[0].h, acc[1].h), t2 = two_sum(t1.h, acc[2].h);
+      q[k] = two_sum(t2.h, ((acc[0].l + acc[1].l) + (acc[2].l + t1.l)) + t2.l);
+      if (slot[k] < 0) q[k] = ff{0.f, 0.f};
     }
-    tail_push_z(cl, sm, own, v, sub, tpv, z);
-    tail_push_sums<2>(cl, sm, t, tpv, 0);
-    cl.sync();
-    const ff rr = tail_total(sm, 0, ncta);
-    const ff atn = tail_total(sm, 1, ncta);
-    if (ff_lt(rr, stopAt)) break;
-    const ff beta = ff_div(atn, alphaTop);
-    alphaTop = atn;
-    for (int u = threadIdx.x; u < n; u += blockDim.x) {
-      const ff pu = ff_add(ff{sm.zh[u], sm.zl[u]}, ff_mul(beta, ff{sm.ph[u], sm.pl[u]}));
-      sm.ph[u] = pu.h;
-      sm.pl[u] = pu.l;
+    ff pq = dot(p, q);
+    coarse_dots<1>(sm, warps, 0, &pq);
+    const ff alpha = ff_div(alphaTop, pq);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      x[k] = ff_add(x[k], ff_mul(alpha, p[k]));
+      r[k] = ff_add(r[k], ff_neg(ff_mul(alpha, q[k])));
+      z[k] = ff_mul(r[k], inv[k]);
     }
-    __syncthreads();
+    d[0] = dot(r, r);
+    d[1] = dot(r, z);
+    coarse_dots<2>(sm, warps, 1, d);
+    if (ff_lt(d[0], stopAt)) break;
+    const ff beta = ff_div(d[1], alphaTop);
+    alphaTop = d[1];
+#pragma unroll
+    for (int k = 0; k < K; k++) p[k] = ff_add(z[k], ff_mul(beta, p[k]));
+    publish();
+    coarse_sync(warps);
   }
-  if (own && sub == 0) L.x[v] = x.h + x.l;
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (slot[k] >= 0) L.x[slot[k]] = x[k].h + x[k].l;
 }
 
+// restrict_vertex from a colour-blocked level
+template <bool IS3D>
+__device__ __forceinline__ void tail_restrict(const Lev& D, const Lev& L, int v) {
+  constexpr int E = IS3D ? 27 : 9;
+  const bool ok = v < (int)D.n;
+  v = ok ? v : 0;
+  int vx, vy, vz;
+  coords(D, v, vx, vy, vz);
+  const int8_t type = D.type[v];
+  // the fine vertices 2V-1 .. 2V+1 inside the level, in the reference's order
+  const Nb3 o = nb3(L, 2 * vx, 2 * vy, 2 * vz);
+  const int u = (int)lin(L, 2 * vx, 2 * vy, 2 * vz);
+  float rv[E];
+  auto in = [&](int q) { return o.ix[q % 3] && o.iy[q / 3 % 3] && o.iz[IS3D ? q / 9 : 1]; };
+#pragma unroll
+  for (int q = 0; q < E; q++) rv[q] = tail_ld(&L.r[in(q) ? u + o.ox[q % 3] + o.oy[q / 3 % 3] + o.oz[IS3D ? q / 9 : 1] : 0]);
+  __syncwarp();
+  float sum = 0.f;
+#pragma unroll
+  for (int q = 0; q < E; q++) {
+    // 1/2 per odd coordinate; inactive fine vertices hold r = 0
+    const int odd = (q % 3 != 1) + (q / 3 % 3 != 1) + (IS3D && q / 9 != 1);
+    const float t = sum + (odd == 0 ? 1.f : odd == 1 ? 0.5f : odd == 2 ? 0.25f : 0.125f) * rv[q];
+    sum = in(q) ? t : sum;
+  }
+  if (!ok) return;
+  D.x[v] = 0.f;
+  if (type != kVtInactive) D.b[v] = sum;
+}
+
+// interp_vertex within the tail
+template <bool IS3D>
+__device__ __forceinline__ void tail_interp(const Lev& D, const Lev& C, int v) {
+  int vx, vy, vz;
+  coords(D, min(v, (int)D.n - 1), vx, vy, vz);
+  const bool ok = v < (int)D.n && inside(D, vx, vy, vz);
+  v = ok ? v : 0;
+  if (!ok) vx = vy = vz = 0;
+  const int8_t type = D.type[v];
+  // coarse parents V/2 .. (V+1)/2 per axis, in the reference's order; inactive
+  // ones hold x = 0
+  auto use = [&](int q) { return (q & 1) <= (vx & 1) && (q >> 1 & 1) <= (vy & 1) && (q >> 2) <= (vz & 1); };
+  float cv[IS3D ? 8 : 4];
+#pragma unroll
+  for (int q = 0; q < (IS3D ? 8 : 4); q++)
+    cv[q] = tail_ld(&C.x[use(q) ? lin(C, vx / 2 + (q & 1), vy / 2 + (q >> 1 & 1), vz / 2 + (q >> 2)) : 0]);
+  const float x = tail_ld(&D.x[v]);
+  __syncwarp();
+  float sum = 0.f;
+#pragma unroll
+  for (int q = 0; q < (IS3D ? 8 : 4); q++) {
+    const float t = sum + cv[q];
+    sum = use(q) ? t : sum;
+  }
+  const float xv = x + inv_pow2(parity3(vx, vy, vz)) * sum;
+  if (ok && type != kVtInactive) D.x[v] = xv;
+}
+
+// One vertex of a tail level with everything of it that no pass writes: its
+// stencil (in applyAStencil's order), right-hand side and whether it is active.
+template <bool IS3D>
+struct TailVertex {
+  static constexpr int E = IS3D ? 27 : 9, S = IS3D ? 14 : 5;
+  float a[(E + 3) / 4 * 4];
+  float b;
+  int v, x, y, z;
+  bool act;
+
+  // id: the slot's stencil in the level's dictionary, if it has one
+  __device__ __forceinline__ void load(const Lev& L, bool ok, int slot, int vx, int vy, int vz, int id) {
+    ok = ok && inside(L, vx, vy, vz);
+    v = ok ? slot : 0;  // slot 0 is vertex (0, 0, 0)
+    x = ok ? vx : 0;
+    y = ok ? vy : 0;
+    z = ok ? vz : 0;
+    const int8_t type = L.type[v];
+    if (L.sid) {
+      const float4* const t = (const float4*)(L.T + id * kDictStride);
+#pragma unroll
+      for (int q = 0; q < (E + 3) / 4; q++) {
+        const float4 f = tail_ld_const(t + q);
+        a[4 * q] = f.x;
+        a[4 * q + 1] = f.y;
+        a[4 * q + 2] = f.z;
+        a[4 * q + 3] = f.w;
+      }
+    } else {
+      const Nb3 o = nb3(L, x, y, z);
+      const int n = (int)L.n;
+#pragma unroll
+      for (int s = 0; s < E; s++) {
+        const int dx = s % 3, dy = s / 3 % 3, dz = IS3D ? s / 9 : 1;
+        const int nn = o.ix[dx] && o.iy[dy] && o.iz[dz] ? v + o.ox[dx] + o.oy[dy] + o.oz[dz] : v;
+        a[s] = tail_ld_const(s < S ? L.A + (S - 1 - s) * n + nn : L.A + (s - S + 1) * n + v);
+      }
+    }
+    b = tail_ld(&L.b[v]);
+    __syncwarp();
+    act = ok && type != kVtInactive;
+  }
+  // b minus the stencil's terms, every x loaded before the first use
+  template <bool SKIP_CENTER>
+  __device__ __forceinline__ float sub(const Lev& L) const {
+    const Nb3 o = nb3(L, x, y, z);  // L is colour-blocked
+    float xv[E];
+    auto in = [&](int s) { return o.ix[s % 3] && o.iy[s / 3 % 3] && o.iz[IS3D ? s / 9 : 1] && !(SKIP_CENTER && s == S - 1); };
+#pragma unroll
+    for (int s = 0; s < E; s++) xv[s] = tail_ld(&L.x[in(s) ? v + o.ox[s % 3] + o.oy[s / 3 % 3] + o.oz[IS3D ? s / 9 : 1] : v]);
+    __syncwarp();  // keeps the loads ahead of the sum
+    float sum = b;
+#pragma unroll
+    for (int s = 0; s < E; s++) {
+      const float t = sum - a[s] * xv[s];
+      sum = in(s) ? t : sum;
+    }
+    return sum;
+  }
+};
+
+// The passes' latencies decide the time, so no pass waits for a load that it
+// could have had before: while a colour's results travel to the other CTAs
+// (a barrier of the cluster takes 1100 cycles by itself), the next colour's
+// stencils are fetched, and every pass issues all its loads before the first
+// use: 2.1 us a pass, before 3.5.  With the coarsest level's solver this took a
+// launch from 400 to 205 us, a solve at 161 x 199 x 143 from 4.51 to 3.38 ms.
 template <bool IS3D>
 __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const Lev* __restrict__ levs, int first, int last, int S,
                                                              float accuracy, const CgScalars* sc) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   if (sc->done) return;  // the same for every CTA of the cluster
-  __shared__ TailSmem sm;
-  const long long T = (long long)cl.num_blocks() * blockDim.x;
-  const long long t0 = (long long)cl.block_rank() * blockDim.x + threadIdx.x;
+  __shared__ CoarseSmem sm;
+  extern __shared__ float coef[];
+  // A pass' vertices are spread over all CTAs: a CTA's loads pass its one
+  // SM's port to L2.  Threads without a vertex load nothing.
+  auto share = [&](int count) { return ((count + cl.num_blocks() - 1) / cl.num_blocks() + 31) & ~31; };
+  const int rank = cl.block_rank(), t = threadIdx.x;
   constexpr int ncol = IS3D ? 8 : 4;
-  for (int l = first; l < last; l++) {
-    const Lev L = levs[l];
-    const int bx = (L.sx + 1) / 2, by = (L.sy + 1) / 2;
-    const long long nb = (long long)bx * by * ((L.sz + 1) / 2);
-    for (int c = 0; c < ncol; c++) {
-      if (L.sid)
-        for (long long bi = t0; bi < nb; bi += T) smooth_vertex_dict_flat<IS3D>(L, bi, c & 1, (c >> 1) & 1, c >> 2, bx, by);
-      else
-        for (long long bi = t0; bi < nb; bi += T) smooth_vertex_flat<IS3D>(L, bi, c & 1, (c >> 1) & 1, c >> 2, bx, by);
+  // levels down, the coarsest level, levels up
+  for (int step = 0;; step++) {
+    const bool up = step >= last - first;
+    if (step == last - first) {
+      if (cl.block_rank() == 0) {
+        const Lev C = levs[last];
+        if (C.sx * C.sy * C.sz <= kTailThreads) coarse_cg<IS3D, 1>(C, S, accuracy, sm, coef);
+        else coarse_cg<IS3D, 2>(C, S, accuracy, sm, coef);
+      }
       cl.sync();
     }
-    if (L.sid)
-      for (long long v = t0; v < L.n; v += T) residual_vertex_dict_flat<IS3D>(L, v);
-    else
-      for (long long v = t0; v < L.n; v += T) residual_vertex_flat<IS3D>(L, v);
-    cl.sync();
-    const Lev D = levs[l + 1];
-    for (long long v = t0; v < D.n; v += T) restrict_vertex<false, true>(D, L, Lev0{}, v);
-    cl.sync();
-  }
-  tail_coarse_cg<IS3D>(cl, levs[last], S, accuracy, sm);
-  cl.sync();  // x of the coarsest level written; no CTA reads another's shared memory any more
-  for (int l = last - 1; l >= first; l--) {
-    const Lev D = levs[l], Sv = levs[l + 1];
-    for (long long v = t0; v < D.n; v += T) interp_vertex<IS3D, true>(D, Sv, v);
-    cl.sync();
-    const int bx = (D.sx + 1) / 2, by = (D.sy + 1) / 2;
-    const long long nb = (long long)bx * by * ((D.sz + 1) / 2);
-    for (int c = ncol - 1; c >= 0; c--) {
-      if (D.sid)
-        for (long long bi = t0; bi < nb; bi += T) smooth_vertex_dict_flat<IS3D>(D, bi, c & 1, (c >> 1) & 1, c >> 2, bx, by);
-      else
-        for (long long bi = t0; bi < nb; bi += T) smooth_vertex_flat<IS3D>(D, bi, c & 1, (c >> 1) & 1, c >> 2, bx, by);
+    if (step == 2 * (last - first)) break;
+    const int l = up ? 2 * last - first - 1 - step : first + step;
+    const Lev L = levs[l], D = levs[l + 1];
+    if (up) {
+      const int own = share((int)L.n);
+      for (int i = t; i < own; i += blockDim.x) tail_interp<IS3D>(L, D, rank * own + i);
+      cl.sync();
+    }
+    const int nb = (int)L.nb, own = share(nb);
+    TailVertex<IS3D> V;
+    auto color = [&](int k) { return up ? ncol - 1 - k : k; };
+    auto slot_of = [&](int k, int i) { return rank * own + i < nb ? color(k) * nb + rank * own + i : 0; };
+    auto id_of = [&](int k, int i) { return L.sid && k < ncol ? tail_ld_const(L.sid + slot_of(k, i)) : 0; };
+    auto load = [&](int k, int i, int id) {
+      const int c = color(k), bi = rank * own + i;
+      int x, y, z;
+      block_xyz(bi < nb ? bi : 0, L.bx, L.by, x, y, z);
+      V.load(L, bi < nb, c * nb + bi, 2 * x + (c & 1), 2 * y + (c >> 1 & 1), 2 * z + (c >> 2), id);
+    };
+    auto smooth = [&]() {
+      const float x = V.template sub<true>(L) / V.a[V.S - 1];
+      if (V.act) L.x[V.v] = x;
+    };
+    int id = 0;  // of the next colour
+    if (t < own) {
+      id = id_of(1, t);
+      load(0, t, id_of(0, t));
+    }
+    for (int k = 0; k < ncol; k++) {
+      if (t < own) smooth();
+      for (int i = t + blockDim.x; i < own; i += blockDim.x) {
+        load(k, i, id_of(k, i));
+        smooth();
+      }
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      if (k + 1 < ncol && t < own) {
+        load(k + 1, t, id);
+        id = id_of(k + 2, t);
+      }
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+    if (!up) {
+      const int ownAll = share((int)L.n), ownNext = share((int)D.n);
+      for (int i = t; i < ownAll; i += blockDim.x) {
+        const int v = rank * ownAll + i;
+        int x, y, z;
+        coords(L, min(v, (int)L.n - 1), x, y, z);
+        V.load(L, v < (int)L.n, v, x, y, z, L.sid && v < (int)L.n ? tail_ld_const(L.sid + v) : 0);
+        const float r = V.template sub<false>(L);
+        if (V.act) L.r[v] = r;
+      }
+      cl.sync();
+      for (int i = t; i < ownNext; i += blockDim.x) tail_restrict<IS3D>(D, L, rank * ownNext + i);
       cl.sync();
     }
   }
@@ -1594,7 +1691,9 @@ int ensure_paths() {
   // the cluster V-cycle tail: 16 CTAs where the GPU can co-schedule them
   g_tailCta = 0;
   if (cudaFuncSetAttribute(k_mg_tail<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-      cudaFuncSetAttribute(k_mg_tail<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+      cudaFuncSetAttribute(k_mg_tail<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+      cudaFuncSetAttribute(k_mg_tail<true>, ring, kCoarseCoefBytes) == cudaSuccess &&
+      cudaFuncSetAttribute(k_mg_tail<false>, ring, kCoarseCoefBytes) == cudaSuccess) {
     for (int c = 16; c >= 8 && !g_tailCta; c /= 2) {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1];
@@ -1604,6 +1703,7 @@ int ensure_paths() {
       at[0].val.clusterDim.z = 1;
       cfg.gridDim = dim3(c);
       cfg.blockDim = dim3(kTailThreads);
+      cfg.dynamicSmemBytes = kCoarseCoefBytes;
       cfg.attrs = at;
       cfg.numAttrs = 1;
       int nc = 0;
@@ -1833,7 +1933,7 @@ MgHierarchy* mg_hierarchy_create(const Dims& d) {
   if (const char* e = std::getenv("MANTAGPU_MG0_PLANES")) h->zc = std::max(2, std::atoi(e) & ~1);
   // the levels of at most kTailSlots storage slots (and the coarsest) run in
   // one cluster launch
-  if (h->ok && L > 1 && g_tailCta && nc <= (long long)g_tailCta * kTailVpc) {
+  if (h->ok && L > 1 && g_tailCta && (long long)h->size[L - 1][0] * h->size[L - 1][1] * h->size[L - 1][2] <= kCoarseMax) {
     long long lim = kTailSlots;
     if (const char* e = std::getenv("MANTAGPU_MG_TAIL_SLOTS")) lim = std::atoll(e);
     int f = L - 1;
@@ -2129,6 +2229,7 @@ int mg_apply(MgHierarchy* h, const PcgBuffers& b, bool init, cudaStream_t s) {
       at[0].val.clusterDim.z = 1;
       cfg.gridDim = dim3(g_tailCta);
       cfg.blockDim = dim3(kTailThreads);
+      cfg.dynamicSmemBytes = kCoarseCoefBytes;
       cfg.stream = s;
       cfg.attrs = at;
       cfg.numAttrs = 1;

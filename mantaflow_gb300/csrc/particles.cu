@@ -33,6 +33,7 @@
 #include "../../include/mantagpu.h"
 #include "mg_batch.h"
 #include "mg_common.cuh"
+#include "mg_f32x2.cuh"
 #include "mg_kernels.h"
 
 using namespace mgpu;
@@ -705,21 +706,6 @@ struct TileAcc {
   uint4 at[3][8];  // from bit 16: byte offset of the first sample's row of acc; below, the rows' steps along axes with an odd sample
 };
 
-// two floats at once, each rounded as by itself
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{.reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
-      " fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;}"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("{.reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mul.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;}"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-
 // two floats in shared memory, without a branch
 __device__ __forceinline__ void add_if(unsigned at, bool in, float x, float y) {
   asm volatile(
@@ -744,7 +730,6 @@ __global__ void __launch_bounds__(32) k_tile_splat(Tiles s, PartView p, float* v
   // odd face, or 1 minus it.  (Exact: with an odd first sample the odd face has
   // the lower weight, 1 minus the upper one, which is a multiple of 2^-23.)
   const int c = min(lane >> 3, 2), ox = lane & 1, oy = lane >> 1 & 1, oz = lane >> 2 & 1;
-  auto both = [](float v) { return make_float2(v, v); };
   const float2 ax = both(ox ? 0.f : 1.f), bx = both(ox ? 1.f : -1.f);
   const float2 ay = both(oy ? 0.f : 1.f), by = both(oy ? 1.f : -1.f);
   const float2 az = both(oz ? 0.f : 1.f), bz = both(oz ? 1.f : -1.f);
