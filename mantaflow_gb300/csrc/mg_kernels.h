@@ -46,11 +46,11 @@ void launch_add_buoyancy(const Dims& d, const int* flags, const float* rho, Mac 
                          cudaStream_t s);
 void launch_add_force(const Dims& d, const int* flags, Mac vel, float fx, float fy, float fz, const float* exclude,
                       cudaStream_t s);
-void launch_extrapolate_mac_simple(const Dims& d, const int* flags, Mac vel, int* tmp, Mac snap, int distance, int intoObs,
+// tmp: extrapolate_marks() bytes of scratch
+size_t extrapolate_marks(const Dims& d);
+void launch_extrapolate_mac_simple(const Dims& d, const int* flags, Mac vel, void* tmp, Mac snap, int distance, int intoObs,
                                    const float* phiObs, cudaStream_t s);
-// extrapolateLsSimple; tmp, mark: int scratch grids
-void launch_extrapolate_ls_simple(const Dims& d, float* phi, int* tmp, int* mark, int distance, int inside,
-                                  cudaStream_t s);
+void launch_extrapolate_ls_simple(const Dims& d, float* phi, void* tmp, int distance, int inside, cudaStream_t s);
 void launch_init_domain(const Dims& d, int* flags, int bw, const int* types, cudaStream_t s);
 void launch_fill_grid(const Dims& d, int* flags, int type, cudaStream_t s);
 void launch_set_open_bound(const Dims& d, int* flags, int bw, const int* lo, const int* up, int type, cudaStream_t s);

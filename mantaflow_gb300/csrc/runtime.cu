@@ -1068,11 +1068,11 @@ extern "C" int mg_extrapolate_mac_simple(mg_grid flags, mg_grid vel, int distanc
     NEED_GRID(phiObs, "extrapolateMACSimple");
     if (!is_real(phiObs) || phiObs->s != s) return fail(MG_ERR_ARG, "extrapolateMACSimple: phiObs must be a levelset of the same solver");
   }
-  Tmp tmp(s, sizeof(int) * (size_t)s->d.n);
+  Tmp tmp(s, extrapolate_marks(s->d));
   Tmp snap(s, vel->bytes());
   if (!tmp.p || !snap.p) return fail(MG_ERR_NOMEM, "extrapolateMACSimple: out of device memory");
   ProfScope ps(s, "extrapolate_mac_simple");
-  launch_extrapolate_mac_simple(s->d, flags->i(), vel->mac(), tmp.i(), snap.mac(), distance, intoObs,
+  launch_extrapolate_mac_simple(s->d, flags->i(), vel->mac(), tmp.p, snap.mac(), distance, intoObs,
                                 phiObs ? phiObs->f() : nullptr, s->stream);
   CKL();
   return MG_OK;
@@ -1082,10 +1082,10 @@ extern "C" int mg_extrapolate_ls_simple(mg_grid phi, int distance, int inside) {
   NEED_GRID(phi, "extrapolateLsSimple");
   if (!is_real(phi)) return fail(MG_ERR_ARG, "extrapolateLsSimple: phi must be a Real or Levelset grid");
   mg_solver s = phi->s;
-  Tmp tmp(s, sizeof(int) * (size_t)s->d.n), mark(s, sizeof(int) * (size_t)s->d.n);
-  if (!tmp.p || !mark.p) return fail(MG_ERR_NOMEM, "extrapolateLsSimple: out of device memory");
+  Tmp tmp(s, extrapolate_marks(s->d));
+  if (!tmp.p) return fail(MG_ERR_NOMEM, "extrapolateLsSimple: out of device memory");
   ProfScope ps(s, "extrapolate_ls_simple");
-  launch_extrapolate_ls_simple(s->d, phi->f(), tmp.i(), mark.i(), distance, inside, s->stream);
+  launch_extrapolate_ls_simple(s->d, phi->f(), tmp.p, distance, inside, s->stream);
   CKL();
   return MG_OK;
 }
