@@ -235,4 +235,26 @@ inline dim3 grid3(const Dims& d, dim3 b) {
   return dim3((unsigned)((d.nx + b.x - 1) / b.x), (unsigned)((d.ny + b.y - 1) / b.y), (unsigned)d.nz);
 }
 
+// Programmatic launches, for chains of short kernels on one stream: a kernel's
+// CTAs start while the kernel before it finishes, fetch what that one does not
+// write, and wait for its results.  A kernel that calls pass_started() lets the
+// next one's CTAs in; one launched so calls pass_wait() before it touches what
+// others write.  (Both are no-ops in other launches.)
+__device__ __forceinline__ void pass_started() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+cudaError_t launch_pass(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool early, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 }  // namespace mgpu

@@ -324,6 +324,8 @@ __global__ void __launch_bounds__(kMcThreads, 1) k_mic_cluster(McArgs a) {
     mbar_init(&s_done[0][0] + tid, 32);
     mbar_fence_init();
   }
+  pass_started();
+  pass_wait();
   if (rank == 0 && tid == 0) {
     const int first = a.scenes ? 0 : *((volatile const int*)&a.one.sc->done);  // (beside the ticket's round trip)
     const int t = (int)atomicInc(a.counter, (unsigned)a.njobs - 1u);           // wraps to 0 with the last ticket
@@ -612,72 +614,75 @@ __global__ void __launch_bounds__(64 * kMcWarps) k_mic_order(McArgs a) {
 constexpr size_t kOrderSmem = 64 * kMcWarps * (34 * sizeof(unsigned short) + 33 * sizeof(float));
 
 // Between grid and level order, with the element-wise work of the iteration
-// on the way: a CTA takes a block's four bundles over 32 levels, rows of 32
-// cells on the grid side, turned in shared memory.  All of it is memory
-// traffic; the skewed rows cost a fifth more sectors than aligned ones.
+// on the way: a CTA takes one bundle over 32 levels, rows of 32 cells on the
+// grid side, turned in shared memory.  All of it is memory traffic; the skewed
+// rows cost a fifth more sectors than aligned ones.  A CTA per block (48 at
+// 64^3) with its rows in four batches took 11.3 us for axpy and 6.4 for the
+// update there, a CTA per bundle with one batch 8.3 and 6.4 (cold caches); with
+// the chain's launches overlapped (pass_started) an iteration of the solver
+// takes 73 instead of 82 us at 64^3, 142 instead of 154 on the dam at 128^3.
 enum { kLvlInit = 0, kLvlAxpy = 1, kLvlUpdate = 2, kLvlSearch = 3 };
-constexpr int kLvlThreads = 512;
+constexpr int kLvlThreads = 256;
 template <int OP, bool L2 = false>
-__global__ void __launch_bounds__(kLvlThreads, 2) k_lvl(McArgs a) {
-  __shared__ float tile[64 * kMcWarps][33];
+__global__ void __launch_bounds__(kLvlThreads, 3) k_lvl(McArgs a) {
+  __shared__ float tile[64][33];
+  pass_started();
+  pass_wait();
   const MicClusterScene& S = a.scenes ? a.scenes[blockIdx.y] : a.one;
   CgScalars* const sc = S.sc;
   const int nx = S.d.nx, ny = S.d.ny, nz = S.d.nz, nlp = S.nlp;
-  const int tiles = (nlp + 31) / 32, total = S.nby * S.nbz * tiles;
-  if ((int)blockIdx.x >= total) return;
+  // part has a slot for every block's 32 levels, in a single solve for more
+  const int tiles = (nlp + 31) / 32, total = S.nby * S.nbz * tiles * kMcWarps;
+  const int ctas = min((int)gridDim.x, a.scenes ? total / kMcWarps : total);
+  if ((int)blockIdx.x >= ctas) return;
   if ((OP == kLvlAxpy || OP == kLvlUpdate) && sc->done) return;
   const float alpha = OP == kLvlAxpy ? sc->alpha : 0.f, na = -alpha;
   const float beta = OP == kLvlUpdate ? sc->beta : 0.f;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, u = w >> 2, k = w & 3;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float mn = FLT_MAX, mx = -FLT_MAX;
   double ss = 0.;
-  for (int t = blockIdx.x; t < total; t += gridDim.x) {
-    const int b = t / tiles, L0 = (t - b * tiles) * 32;
+  for (int t = blockIdx.x; t < total; t += ctas) {
+    const int ub = t / tiles, L0 = (t - ub * tiles) * 32, u = ub & (kMcWarps - 1), b = ub / kMcWarps;
     const int y0 = (b % S.nby) * kBlk + (u & 1) * kUY, z0 = (b / S.nby) * kBlk + (u >> 1) * kUZ;
-    // grid side: this warp's lines z = 2k and 2k + 1 of the bundle, y = q mod
-    // 8.  Four rows' loads are all issued before the first of their stores.
-    const long long g0 = ((long long)(z0 + 2 * k) * ny + y0) * nx + L0 + lane - 2 * k;
-    auto row = [&](int q) -> float& { return tile[u * 64 + (q >> 3) * 32 + k * 8 + (q & (kUY - 1))][lane]; };
-    auto cell = [&](int q) { return g0 + (long long)(q >> 3) * ((long long)nx * ny - 1) + (long long)(q & (kUY - 1)) * (nx - 1); };
+    // grid side: this warp's line z = w of the bundle, eight rows y.  All loads
+    // are issued before the first store.
+    const long long g0 = ((long long)(z0 + w) * ny + y0) * nx + L0 + lane - w;
+    const int line = (w & 1) * 32 + (w >> 1) * 8;
+    auto cell = [&](int q) { return g0 + (long long)q * (nx - 1); };
     unsigned in = 0u;
 #pragma unroll
-    for (int q = 0; q < 16; q++) {
-      const int yl = q & (kUY - 1), zl = 2 * k + (q >> 3);
-      in |= ((unsigned)(L0 + lane - yl - zl) < (unsigned)nx && y0 + yl < ny && z0 + zl < nz) ? 1u << q : 0u;
-    }
-    // level side: levels 8k .. 8k + 7; a lane's even line in tile row lane, its odd one in row 32 + lane
-    const long long base = (((long long)b * kMcWarps + u) * nlp + L0 + 8 * k) * 32 + lane;
-    const float *ta = &tile[u * 64 + lane][8 * k], *tb = &tile[u * 64 + 32 + lane][8 * k];
-    const int levels = min(8, nlp - L0 - 8 * k);
-    const int y = y0 + (lane & 7), z = z0 + 2 * (lane >> 3), xs = L0 + 8 * k - (lane & 7) - 2 * (lane >> 3);
+    for (int q = 0; q < kUY; q++)
+      in |= ((unsigned)(L0 + lane - q - w) < (unsigned)nx && y0 + q < ny && z0 + w < nz) ? 1u << q : 0u;
+    // level side: levels 4w .. 4w + 3; a lane's even line in tile row lane, its odd one in row 32 + lane
+    const long long base = (((long long)b * kMcWarps + u) * nlp + L0 + 4 * w) * 32 + lane;
+    const float *ta = &tile[lane][4 * w], *tb = &tile[32 + lane][4 * w];
+    const int levels = min(4, nlp - L0 - 4 * w);
+    const int y = y0 + (lane & 7), z = z0 + 2 * (lane >> 3), xs = L0 + 4 * w - (lane & 7) - 2 * (lane >> 3);
     float2* const r2 = reinterpret_cast<float2*>(S.r) + base;
     if (OP == kLvlInit || OP == kLvlAxpy) {
+      float t8[kUY], s8[kUY], p8[kUY];
 #pragma unroll
-      for (int h = 0; h < 16; h += 4) {
-        float t4[4], s4[4], p4[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const bool ok = in >> (h + q) & 1u;
-          const long long g = cell(h + q);
-          t4[q] = ok ? (OP == kLvlInit ? S.rhs[g] : S.t[g]) : 0.f;
-          if (OP == kLvlAxpy) {
-            s4[q] = ok ? S.s[g] : 0.f;
-            p4[q] = ok ? S.p[g] : 0.f;
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          row(h + q) = t4[q];
-          if (in >> (h + q) & 1u) S.p[cell(h + q)] = OP == kLvlInit ? 0.f : p4[q] + alpha * s4[q];
+      for (int q = 0; q < kUY; q++) {
+        const bool ok = in >> q & 1u;
+        const long long g = cell(q);
+        t8[q] = ok ? (OP == kLvlInit ? S.rhs[g] : S.t[g]) : 0.f;
+        if (OP == kLvlAxpy) {
+          s8[q] = ok ? S.s[g] : 0.f;
+          p8[q] = ok ? S.p[g] : 0.f;
         }
       }
-      float2 o[8];
+      float2 o[4];
       if (OP == kLvlAxpy)
 #pragma unroll
-        for (int i = 0; i < 8; i++) o[i] = i < levels ? r2[32 * i] : make_float2(0.f, 0.f);
+        for (int i = 0; i < 4; i++) o[i] = i < levels ? r2[32 * i] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int q = 0; q < kUY; q++) {
+        tile[line + q][lane] = t8[q];
+        if (in >> q & 1u) S.p[cell(q)] = OP == kLvlInit ? 0.f : p8[q] + alpha * s8[q];
+      }
       __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
+      for (int i = 0; i < 4; i++) {
         float2 r = make_float2(ta[i], tb[i]);
         if (OP == kLvlAxpy) {
           const bool oka = y < ny && z < nz && (unsigned)(xs + i) < (unsigned)nx;
@@ -698,20 +703,20 @@ __global__ void __launch_bounds__(kLvlThreads, 2) k_lvl(McArgs a) {
       }
     } else {
       const float2* const z2 = reinterpret_cast<const float2*>(S.z) + base;
-      float s16[16];
+      float s8[kUY];
       if (OP == kLvlUpdate)
 #pragma unroll
-        for (int q = 0; q < 16; q++) s16[q] = (in >> q & 1u) ? S.s[cell(q)] : 0.f;
+        for (int q = 0; q < kUY; q++) s8[q] = (in >> q & 1u) ? S.s[cell(q)] : 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
+      for (int i = 0; i < 4; i++) {
         const float2 v = i < levels ? z2[32 * i] : make_float2(0.f, 0.f);
-        tile[u * 64 + lane][8 * k + i] = v.x;
-        tile[u * 64 + 32 + lane][8 * k + i] = v.y;
+        tile[lane][4 * w + i] = v.x;
+        tile[32 + lane][4 * w + i] = v.y;
       }
       __syncthreads();
 #pragma unroll
-      for (int q = 0; q < 16; q++)
-        if (in >> q & 1u) S.s[cell(q)] = OP == kLvlSearch ? row(q) : row(q) + beta * s16[q];
+      for (int q = 0; q < kUY; q++)
+        if (in >> q & 1u) S.s[cell(q)] = OP == kLvlSearch ? tile[line + q][lane] : tile[line + q][lane] + beta * s8[q];
     }
     __syncthreads();
   }
@@ -719,7 +724,6 @@ __global__ void __launch_bounds__(kLvlThreads, 2) k_lvl(McArgs a) {
   // residual norm and convergence test (conjugategrad.cpp:262-276)
   block_minmax(mn, mx);
   const double bs = L2 ? block_sum(ss) : 0.;
-  const unsigned ctas = min((int)gridDim.x, total);
   float* const pf = reinterpret_cast<float*>(S.part);
   if (threadIdx.x == 0) {
     if (L2) {
@@ -845,23 +849,25 @@ cudaError_t launch_mic_cluster_order(const MicClusterLaunch& m, cudaStream_t s) 
 
 cudaError_t launch_mic_level(const MicClusterLaunch& m, int op, cudaStream_t s) {
   const McArgs a = mc_args(m);
-  const int tiles = m.maxBlocks * ((m.nlpMax + 31) / 32);
+  const int tiles = m.maxBlocks * ((m.nlpMax + 31) / 32) * (m.scenes ? 1 : kMcWarps);
   const dim3 g((unsigned)std::min(tiles, m.maxParts), (unsigned)m.nscenes);
+  const auto k = op == kMicInit ? k_lvl<kLvlInit> : op == kMicAxpy ? (m.l2 ? k_lvl<kLvlAxpy, true> : k_lvl<kLvlAxpy>)
+                 : op == kMicUpdate ? k_lvl<kLvlUpdate> : k_lvl<kLvlSearch>;
   count_launch();
-  if (op == kMicInit) k_lvl<kLvlInit><<<g, kLvlThreads, 0, s>>>(a);
-  else if (op == kMicAxpy && m.l2) k_lvl<kLvlAxpy, true><<<g, kLvlThreads, 0, s>>>(a);
-  else if (op == kMicAxpy) k_lvl<kLvlAxpy><<<g, kLvlThreads, 0, s>>>(a);
-  else if (op == kMicUpdate) k_lvl<kLvlUpdate><<<g, kLvlThreads, 0, s>>>(a);
-  else k_lvl<kLvlSearch><<<g, kLvlThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_pass(k, g, dim3(kLvlThreads), 0, s, !m.scenes, a);
 }
 
 // mode: 0 factor, 1 forward, 2 backward (beta), 3 backward for doInit (sigma)
 cudaError_t launch_mic_cluster(const MicClusterLaunch& m, int mode, cudaStream_t s) {
   McArgs a = mc_args(m);
   a.init = mode == 3 ? 1 : 0;
-  cudaLaunchAttribute at[1];
-  const cudaLaunchConfig_t cfg = mc_config(m.njobs, mc_smem(m.nlpMax), at, s);
+  cudaLaunchAttribute at[2];
+  cudaLaunchConfig_t cfg = mc_config(m.njobs, mc_smem(m.nlpMax), at, s);
+  if (!m.scenes) {
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
   count_launch();
   return cudaLaunchKernelEx(&cfg, mc_kernel(mode), a);
 }

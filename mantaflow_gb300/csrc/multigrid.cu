@@ -621,11 +621,6 @@ __global__ void __launch_bounds__(256, 3) k_mg_residual(Lev L, int S, const CgSc
   GRID_STRIDE(v, L.n) residual_vertex<IS3D>(L, v);
 }
 
-// Programmatic launches: a pass' CTAs start while those of the pass before
-// finish, fetch what no pass writes, and wait for its results.
-__device__ __forceinline__ void pass_started() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // The same passes on a level with a stencil dictionary.  A level of 590 000
 // slots or fewer is bound by latency: a launch, an id, its tuple, the values.
 // With the ids fetched while the pass before ends and all values loaded at
@@ -1808,22 +1803,6 @@ void gen_coarse_grid(const int fs[3], const std::vector<int8_t>& tf, const int c
   }
 }
 
-// a launch whose CTAs may start before the kernel ahead of it has finished: for
-// kernels that call pass_wait() before they touch what others write
-template <class... P, class... A>
-void launch_pass(void (*kernel)(P...), int blocks, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(256);
-  cfg.stream = s;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-
 int blocks_for(long long n) {
   // one vertex per thread: each thread's loads are then independent of the
   // others' (a grid-stride loop would serialise their memory latency)
@@ -2192,8 +2171,8 @@ int mg_apply(MgHierarchy* h, const PcgBuffers& b, bool init, cudaStream_t s) {
       const int c = reversed ? ncol - 1 - q : q;
       count_launch();
       if (v.sid) {
-        if (h->is3d) launch_pass(k_mg_smooth_dict<true>, nb, s, v, off[c][0], off[c][1], off[c][2], sc);
-        else launch_pass(k_mg_smooth_dict<false>, nb, s, v, off[c][0], off[c][1], off[c][2], sc);
+        if (h->is3d) launch_pass(k_mg_smooth_dict<true>, dim3(nb), dim3(kThreads1), 0, s, true, v, off[c][0], off[c][1], off[c][2], sc);
+        else launch_pass(k_mg_smooth_dict<false>, dim3(nb), dim3(kThreads1), 0, s, true, v, off[c][0], off[c][1], off[c][2], sc);
       } else {
         if (h->is3d) k_mg_smooth<true><<<nb, kThreads1, 0, s>>>(v, S, off[c][0], off[c][1], off[c][2], sc);
         else k_mg_smooth<false><<<nb, kThreads1, 0, s>>>(v, S, off[c][0], off[c][1], off[c][2], sc);
@@ -2236,8 +2215,8 @@ int mg_apply(MgHierarchy* h, const PcgBuffers& b, bool init, cudaStream_t s) {
       count_launch();
       const Lev& v = h->lev[l];
       if (v.sid) {
-        if (h->is3d) launch_pass(k_mg_residual_dict<true>, blocks_for(v.n), s, v, sc);
-        else launch_pass(k_mg_residual_dict<false>, blocks_for(v.n), s, v, sc);
+        if (h->is3d) launch_pass(k_mg_residual_dict<true>, dim3(blocks_for(v.n)), dim3(kThreads1), 0, s, true, v, sc);
+        else launch_pass(k_mg_residual_dict<false>, dim3(blocks_for(v.n)), dim3(kThreads1), 0, s, true, v, sc);
       } else {
         if (h->is3d) k_mg_residual<true><<<blocks_for(v.n), kThreads1, 0, s>>>(v, S, sc);
         else k_mg_residual<false><<<blocks_for(v.n), kThreads1, 0, s>>>(v, S, sc);

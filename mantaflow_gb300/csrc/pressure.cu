@@ -605,6 +605,8 @@ __device__ __forceinline__ float4 spmv_apply_sel(const SpmvQuad& Q, FSum& acc) {
 __global__ void __launch_bounds__(256, 4) k_pcg_spmv_zm(Dims d, ZmGeom g, const code_t* __restrict__ code,
                                                       const float* __restrict__ A0f, const float* __restrict__ x,
                                                       float* y, double* part, CgScalars* sc) {
+  pass_started();
+  pass_wait();
   if (sc->done) return;
   FSum acc;
   const int r = threadIdx.x / g.nq, xq = threadIdx.x - r * g.nq;
@@ -1546,7 +1548,7 @@ void launch_pcg_spmv(const PcgBuffers& b, cudaStream_t s) {
   dim3 grid;
   const int mode = spmv_mode();
   if (mode == kSpmvZm && zm_geom(b.d, 2 * b.nblocks, g_zmSlots, &zg, &grid)) {
-    k_pcg_spmv_zm<<<grid, 256, 0, s>>>(b.d, zg, b.code, b.A0f, b.search, b.tmp, b.part, b.sc);
+    launch_pass(k_pcg_spmv_zm, grid, dim3(256), 0, s, true, b.d, zg, b.code, b.A0f, b.search, b.tmp, b.part, b.sc);
     return;
   }
   if (mode != kSpmvQuad && stream_geom(b.d, 2 * b.nblocks, g_sms, &g, &grid)) {
