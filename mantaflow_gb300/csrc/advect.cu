@@ -97,8 +97,8 @@ __device__ __forceinline__ void clamp_component(const Dims& d, const int* __rest
 #pragma unroll
         for (int c = 0; c < CH; c++) {
           const float v = ov[q][c];
-          if (v < mn[c]) mn[c] = v;
-          if (v > mx[c]) mx[c] = v;
+          mn[c] = fminf(mn[c], v);  // a NaN is passed over, as by the reference's comparisons
+          mx[c] = fmaxf(mx[c], v);
         }
         haveFl = true;
       }
@@ -274,7 +274,7 @@ __device__ __forceinline__ float clamp_component_mac(const Dims& d, int fo, int 
   const float posx = (float)i, posy = (float)j, posz = (float)k;
   if (clampMode == 2 && !((fo & (kFluid | kEmpty)) && (fnb & (kFluid | kEmpty)))) return fwd;
   const int np = clampMode == 1 ? 2 : 1;
-  const int Y = (int)d.sy, Z = (int)d.sz;  // grids hold < 2^31 cells
+  const int Y = (int)d.sy, Z = d.is3d ? (int)d.sz : 0;  // grids hold < 2^31 cells; in 2D the plane twice
   for (int l = 0; l < np; l++) {
     const int qx = (int)(l == 0 ? posx - vel.x : posx + vel.x);
     const int qy = (int)(l == 0 ? posy - vel.y : posy + vel.y);
@@ -283,14 +283,12 @@ __device__ __forceinline__ float clamp_component_mac(const Dims& d, int fo, int 
     const int j0 = min(max(qy, 0), d.ny - 2);
     const int k0 = min(max(qz, 0), d.is3d ? d.nz - 2 : 0);
     const float* p = orig + (i0 + Y * j0 + Z * k0);
-    const int nk = d.is3d ? 2 : 1;
-    for (int kk = 0; kk < nk; kk++) {
+    // a NaN is passed over, as by the reference's comparisons
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const float v = __ldg(p + (q & 1) + Y * (q >> 1) + Z * kk);
-        if (v < mn) mn = v;
-        if (v > mx) mx = v;
-      }
+    for (int q = 0; q < 8; q++) {
+      const float v = __ldg(p + (q & 1) + Y * (q >> 1 & 1) + Z * (q >> 2));
+      mn = fminf(mn, v);
+      mx = fmaxf(mx, v);
     }
   }
   if (clampMode == 1) {
@@ -353,14 +351,14 @@ __device__ __forceinline__ void maccormack_mac_cell(const Dims& d, const int* __
   dst.w[idx] = val[2];
 }
 
-template <int kTrace, int kOS>
+template <int kTrace, int kOS, int kClamp>
 __global__ void __launch_bounds__(256, 5) k_maccormack_mac(Dims d, const int* __restrict__ flags, CMac vel, CMac orig,
-                                                        CMac fwd, Mac dst, float dt, float strength, int clampMode) {
+                                                        CMac fwd, Mac dst, float dt, float strength) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
   if (i >= d.nx || j >= d.ny) return;
-  maccormack_mac_cell<kTrace, kOS>(d, flags, vel, orig, fwd, dst, dt, strength, clampMode, i, j, k);
+  maccormack_mac_cell<kTrace, kOS>(d, flags, vel, orig, fwd, dst, dt, strength, kClamp, i, j, k);
 }
 
 // extrapolateVelConvectiveBC (advection.cpp:346-381): velDst for outflow
@@ -628,17 +626,19 @@ void launch_advect_sl_mac(const Dims& d, CMac vel, CMac src, Mac dst, float dt, 
   }
 }
 
+// the modes that the clamp tells apart: 1, 2 and neither
+template <int kTrace, int kOS>
+static auto mc_mac(int clampMode) {
+  return clampMode == 1 ? k_maccormack_mac<kTrace, kOS, 1> : clampMode == 2 ? k_maccormack_mac<kTrace, kOS, 2> : k_maccormack_mac<kTrace, kOS, 0>;
+}
+
 void launch_advect_maccormack_mac(const Dims& d, const int* flags, CMac vel, CMac orig, CMac fwd, Mac dst, float dt,
                                   float strength, int clampMode, int orderSpace, int orderTrace, cudaStream_t s) {
   count_launch();
   const dim3 g = grid3(d, kBlk);
-  if (orderSpace == 1) {
-    if (orderTrace == 1) k_maccormack_mac<1, 1><<<g, kBlk, 0, s>>>(d, flags, vel, orig, fwd, dst, dt, strength, clampMode);
-    else k_maccormack_mac<2, 1><<<g, kBlk, 0, s>>>(d, flags, vel, orig, fwd, dst, dt, strength, clampMode);
-  } else {
-    if (orderTrace == 1) k_maccormack_mac<1, 2><<<g, kBlk, 0, s>>>(d, flags, vel, orig, fwd, dst, dt, strength, clampMode);
-    else k_maccormack_mac<2, 2><<<g, kBlk, 0, s>>>(d, flags, vel, orig, fwd, dst, dt, strength, clampMode);
-  }
+  const auto k = orderSpace == 1 ? orderTrace == 1 ? mc_mac<1, 1>(clampMode) : mc_mac<2, 1>(clampMode)
+                                 : orderTrace == 1 ? mc_mac<1, 2>(clampMode) : mc_mac<2, 2>(clampMode);
+  k<<<g, kBlk, 0, s>>>(d, flags, vel, orig, fwd, dst, dt, strength);
 }
 
 void launch_outflow_bc(const Dims& d, const int* flags, CMac vel, CMac velPrev, Mac velDst, Mac velOut, float timeStep,
