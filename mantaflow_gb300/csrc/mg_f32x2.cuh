@@ -19,15 +19,6 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("{.reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 neg2(float2 a) { return mul2(a, both(-1.f)); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, both(-1.f), a); }  // a - b
 
 }  // namespace mgpu
