@@ -399,7 +399,7 @@ def batched_form(m, steps, seed, plain_steps, acc_steps, sim_steps=100):
     batched = {"sims_per_hour": len(sizes) * 3600.0 / (per_step * sim_steps), "step_ms_mean": 1e3 * per_step,
                "step_ms_p50": 1e3 * float(np.percentile(lat, 50)), "step_ms_p99": 1e3 * float(np.percentile(lat, 99)),
                "cells_per_s": info["cells"] / per_step, "cg_sweeps_per_step": sweeps, "steps_timed": steps,
-               "preconditioner": "MIC(0) in 3D scenes (one dataflow launch over all 3D scenes), none in 2D",
+               "preconditioner": "MIC(0) in 3D scenes (one launch per sweep over all 3D scenes), none in 2D",
                "autotuned_sweep_tile": {"rows": tune[0], "ms_per_8_sweeps_for_8_16_32_64_rows": tune[1]}}
     # plain: every scene, one after another
     per_scene, plain_lat = [], []
