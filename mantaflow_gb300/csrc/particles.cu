@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(256) k_p2g_gather(Dims d, int comp, SortedPart
 // shared memory, about 20 instructions for a particle's 24 faces.  The weights
 // come from a batch of 32 particles whose lanes prepared one each.
 //
-// At 128^3 with 16.8 M particles mapPartsToMAC took 5.5 ms with a radix sort
+// At 128^3 with 16.0 M particles mapPartsToMAC took 5.5 ms with a radix sort
 // and eight-way merges per component (3.2 ms of it in the merges, about 100
 // instructions per contribution); now 1.5 ms: lists 0.11 + 0.16, sort 0.38,
 // splat 0.9.  The splat is bound by shared memory, ten wavefronts per particle
