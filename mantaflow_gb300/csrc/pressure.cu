@@ -602,8 +602,11 @@ __device__ __forceinline__ float4 spmv_apply_sel(const SpmvQuad& Q, FSum& acc) {
   return make_float4(out[0], out[1], out[2], out[3]);
 }
 
+// x is written by the kernel that this one may start beside (a programmatic
+// launch), so it is read with ordinary loads behind pass_wait(): the read-only
+// path (__ldg, const __restrict__) is for what nobody writes meanwhile.
 __global__ void __launch_bounds__(256, 4) k_pcg_spmv_zm(Dims d, ZmGeom g, const code_t* __restrict__ code,
-                                                      const float* __restrict__ A0f, const float* __restrict__ x,
+                                                      const float* __restrict__ A0f, const float* x,
                                                       float* y, double* part, CgScalars* sc) {
   pass_started();
   pass_wait();
@@ -624,12 +627,12 @@ __global__ void __launch_bounds__(256, 4) k_pcg_spmv_zm(Dims d, ZmGeom g, const 
     int q = zs * pq + row * g.nq + xq;
     // x below, at and above plane z (and x of plane z+2 in flight), the
     // codes and the neighbour rows / end cells of plane z
-    float4 cm = zs > 0 ? __ldg(x4 + q - pq) : z4;
-    float4 cc = __ldg(x4 + q);
-    float4 cp = zs + 1 < d.nz ? __ldg(x4 + q + pq) : z4;
+    float4 cm = zs > 0 ? x4[q - pq] : z4;
+    float4 cc = x4[q];
+    float4 cp = zs + 1 < d.nz ? x4[q + pq] : z4;
     uint2 cw = __ldg(c2 + q);
-    float4 ylo = __ldg(x4 + q - dn), yhi = __ldg(x4 + q + up);
-    float xl = __ldg(x + max(4 * q - 1, 0)), xr = __ldg(x + min(4 * q + 4, nlast));
+    float4 ylo = x4[q - dn], yhi = x4[q + up];
+    float xl = x[max(4 * q - 1, 0)], xr = x[min(4 * q + 4, nlast)];
 #pragma unroll 2
     for (int z = zs; z < ze; z++) {
       const bool more = z + 1 < ze;
@@ -639,11 +642,11 @@ __global__ void __launch_bounds__(256, 4) k_pcg_spmv_zm(Dims d, ZmGeom g, const 
       float nxl = xl, nxr = xr;
       if (more) {
         ncw = __ldg(c2 + qn);
-        nylo = __ldg(x4 + qn - dn);
-        nyhi = __ldg(x4 + qn + up);
-        nxl = __ldg(x + (4 * qn - 1));  // qn >= pq > 0
-        nxr = __ldg(x + min(4 * qn + 4, nlast));
-        if (z + 2 < d.nz) cn = __ldg(x4 + qn + pq);
+        nylo = x4[qn - dn];
+        nyhi = x4[qn + up];
+        nxl = x[4 * qn - 1];  // qn >= pq > 0
+        nxr = x[min(4 * qn + 4, nlast)];
+        if (z + 2 < d.nz) cn = x4[qn + pq];
       }
       SpmvQuad Q;
       Q.cw = cw;
