@@ -7,9 +7,6 @@
 //   k_maccormack_*  bwd = SL(fwd, -dt) evaluated on the fly, then the
 //                   correction and the clamp; bwd is never stored.
 // Per cell the arithmetic is the reference's, so the result is the same.
-// The second sweep's CTAs start while the first one's last wave drains (256^3:
-// velocity 612 -> 604 us, a whole smoke step 7.22 -> 7.17 ms; no difference on
-// grids of one wave).
 #include "mg_common.cuh"
 #include "mg_kernels.h"
 #include "mg_batch.h"
@@ -54,7 +51,6 @@ __device__ __forceinline__ void sl_real_cell(const Dims& d, CMac vel, const floa
 template <int CH, int kOrderSpace, int kTrace>
 __global__ void __launch_bounds__(256) k_sl_cell(Dims d, CMac vel, const float* __restrict__ src, float* __restrict__ dst,
                                                  float dt) {
-  pass_started();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -202,7 +198,6 @@ template <int CH, int kOrderSpace, int kTrace>
 __global__ void __launch_bounds__(256, 6) k_maccormack_cell(Dims d, const int* __restrict__ flags, CMac vel,
                                                          const float* __restrict__ orig, const float* __restrict__ fwd,
                                                          float* __restrict__ dst, float dt, float strength, int clampMode) {
-  pass_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -264,7 +259,6 @@ __device__ __forceinline__ void sl_mac_grid_cell(const Dims& d, CMac vel, CMac s
 
 template <int kTrace, int kOS>
 __global__ void __launch_bounds__(256) k_sl_mac(Dims d, CMac vel, CMac src, Mac dst, float dt) {
-  pass_started();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -360,7 +354,6 @@ __device__ __forceinline__ void maccormack_mac_cell(const Dims& d, const int* __
 template <int kTrace, int kOS, int kClamp>
 __global__ void __launch_bounds__(256, 5) k_maccormack_mac(Dims d, const int* __restrict__ flags, CMac vel, CMac orig,
                                                         CMac fwd, Mac dst, float dt, float strength) {
-  pass_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -588,7 +581,7 @@ template <int CH, int OS, int TR>
 static void launch_mc(const Dims& d, const int* flags, CMac vel, const float* orig, const float* fwd, float* dst, float dt,
                       float strength, int clampMode, cudaStream_t s) {
   count_launch();
-  launch_pass(k_maccormack_cell<CH, OS, TR>, grid3(d, kBlk), kBlk, 0, s, true, d, flags, vel, orig, fwd, dst, dt, strength, clampMode);
+  k_maccormack_cell<CH, OS, TR><<<grid3(d, kBlk), kBlk, 0, s>>>(d, flags, vel, orig, fwd, dst, dt, strength, clampMode);
 }
 
 template <int CH>
@@ -645,7 +638,7 @@ void launch_advect_maccormack_mac(const Dims& d, const int* flags, CMac vel, CMa
   const dim3 g = grid3(d, kBlk);
   const auto k = orderSpace == 1 ? orderTrace == 1 ? mc_mac<1, 1>(clampMode) : mc_mac<2, 1>(clampMode)
                                  : orderTrace == 1 ? mc_mac<1, 2>(clampMode) : mc_mac<2, 2>(clampMode);
-  launch_pass(k, g, kBlk, 0, s, true, d, flags, vel, orig, fwd, dst, dt, strength);
+  k<<<g, kBlk, 0, s>>>(d, flags, vel, orig, fwd, dst, dt, strength);
 }
 
 void launch_outflow_bc(const Dims& d, const int* flags, CMac vel, CMac velPrev, Mac velDst, Mac velOut, float timeStep,
