@@ -30,6 +30,7 @@ void noise_release();
 void particles_release(mg_solver s);
 // runtime.cu: a solver's dimensions and stream (MG_ERR_ARG for a bad handle)
 int solver_info(mg_solver s, Dims* d, cudaStream_t* st);
+int sm_count();  // of the device
 
 struct BTile {
   int scene;

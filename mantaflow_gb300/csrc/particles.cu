@@ -458,20 +458,26 @@ struct TileShape {
 using TileLarge = TileShape<8, 8, 4>;
 using TileSmall = TileShape<4, 4, 4>;
 constexpr int kLine = 32;  // words of 128 bytes
-constexpr int kSortThreads = 256, kSortWarps = kSortThreads / 32;
-constexpr int kSortShort = 4608, kSortLong = 24576;  // list entries sorted in shared memory, by two kernels
-constexpr int kDigit = 10;                           // most bits of a sort pass
+// the two sorts in shared memory: most list entries, warps, most bits of a pass
+constexpr int kSortShort = 4608, kShortWarps = 8, kShortBits = 10;
+constexpr int kSortLong = 24576, kLongWarps = 32, kLongBits = 9;
+constexpr int kPieceBits = 14;  // longer lists are sorted in pieces
 struct Tiles {
   Dims d;
   long long n;
   int tx, ty, tz;
   bool large;         // TileLarge, not TileSmall
   unsigned* starts;   // [tiles + 1]: the lists' first entries
-  unsigned* cursor;   // [tiles][kLine]: counts, then next entries
+  unsigned* cursor;   // [tiles][kLine], word 0: counts, then next entries
   unsigned* list;     // particles by tile
   const float* v[3];  // velocity components
   __host__ __device__ int count() const { return tx * ty * tz; }
   __device__ unsigned* counter(int t) const { return cursor + (size_t)t * kLine; }
+  // the lists too long for the first sort, in any order, in word 1; how many,
+  // and how many of them are taken
+  __device__ unsigned* job(unsigned q) const { return cursor + (size_t)q * kLine + 1; }
+  __device__ unsigned* jobs() const { return cursor + 2; }
+  __device__ unsigned* ticket() const { return cursor + 3; }
 };
 
 // one axis of BUILD_INDEX / BUILD_INDEX_SHIFT: first sample and upper weight
@@ -536,7 +542,8 @@ __global__ void __launch_bounds__(256) k_tile_lists(Tiles s, PartView p) {
   }
 }
 
-// counts to first entries; one CTA, eight tiles per thread at a time
+// counts to first entries, and the list of the long lists; one CTA, eight tiles
+// per thread at a time
 __global__ void __launch_bounds__(1024) k_tile_starts(Tiles s) {
   __shared__ unsigned sh[32];
   const int tiles = s.count();
@@ -553,6 +560,7 @@ __global__ void __launch_bounds__(1024) k_tile_starts(Tiles s) {
 #pragma unroll
     for (int q = 0; q < 8; q++) {
       if (t0 + q < tiles) s.starts[t0 + q] = *s.counter(t0 + q) = at;
+      if (c[q] > kSortShort) *s.job(atomicAdd(s.jobs(), 1u)) = t0 + q;
       at += c[q];
     }
   }
@@ -560,33 +568,18 @@ __global__ void __launch_bounds__(1024) k_tile_starts(Tiles s) {
 }
 
 // A tile's list into particle order.  Up to kCap entries: an LSD radix sort in
-// shared memory over the bits in which the list's entries can differ, eight
+// shared memory over the bits in which the list's entries can differ, kWarps
 // warps on consecutive pieces of the list (digit counts per warp, scanned
-// digit by digit, keep it stable).  A first kernel takes a CTA for every list
-// and sorts the short ones with four CTAs per SM; in a second one few CTAs
-// walk over all lists for those that were too long, and sort what does not
-// fit into shared memory either (crowded tiles) by a bitonic network in place.
-__device__ void sort_in_place(unsigned* list, unsigned n) {
-  unsigned long long top = 1;
-  while (top < n) top <<= 1;
-  for (unsigned long long g = 2; g <= top; g <<= 1)
-    for (unsigned long long h = g >> 1; h > 0; h >>= 1) {
-      for (unsigned long long e = threadIdx.x; e < top / 2; e += blockDim.x) {
-        // every comparison upward: the first step of a merge pairs an
-        // entry with its mirror image; places past the end count as larger
-        const unsigned long long b = e / h * 2 * h, x = b + e % h, y = h == g >> 1 ? b + 2 * h - 1 - e % h : x + h;
-        if (y < n && list[y] < list[x]) {
-          const unsigned v = list[x];
-          list[x] = list[y];
-          list[y] = v;
-        }
-      }
-      __syncthreads();
-    }
-}
-
-template <int kCap>
+// digit by digit, keep it stable), at most kBits bits to a pass.  A first
+// kernel takes a CTA for every list and sorts the short ones, four CTAs of 8
+// warps per SM; the longer ones, which k_tile_starts has listed, go to a second
+// one, a CTA of 32 warps per SM that takes them one after another.  At 128^3
+// lists are short up to nine particles per cell, and fit the shared memory up
+// to 49; mapPartsToMAC with 8, 16, 27, 48 and 64 per cell in seeding order takes
+// 1.6, 3.6, 5.9, 9.9 and 18 ms (sorted by cell and merged: 5.6, 11, 22, 48 and 79).
+template <int kCap, int kWarps, int kBits>
 __device__ __forceinline__ void sort_list(unsigned* list, unsigned n, unsigned* sm) {
+  constexpr int kThreads = 32 * kWarps;
   __shared__ unsigned sh[32], range[2];
   unsigned *in = sm, *out = sm + kCap;
   unsigned short* const cnt = (unsigned short*)(sm + 2 * kCap);  // [warps][1 << width]
@@ -596,7 +589,7 @@ __device__ __forceinline__ void sort_list(unsigned* list, unsigned n, unsigned* 
     range[1] = 0u;
   }
   unsigned least = 0xffffffffu, most = 0u;
-  for (unsigned e = t; e < n; e += kSortThreads) {
+  for (unsigned e = t; e < n; e += kThreads) {
     const unsigned v = list[e];
     in[e] = v;
     least = min(least, v);
@@ -611,10 +604,11 @@ __device__ __forceinline__ void sort_list(unsigned* list, unsigned n, unsigned* 
   }
   __syncthreads();
   least = range[0];
-  const int bits = 32 - __clz(range[1] - least), passes = (bits + kDigit - 1) / kDigit;
-  const int width = max(8, (bits + passes - 1) / max(passes, 1)), digits = 1 << width, each = digits / kSortThreads;
+  const int bits = 32 - __clz(range[1] - least), passes = (bits + kBits - 1) / kBits;
+  const int width = max(8, (bits + passes - 1) / max(passes, 1)), digits = 1 << width;
+  const int each = max(1, digits / kThreads);
   const unsigned mask = digits - 1;
-  const unsigned per = ((n + kSortWarps - 1) / kSortWarps + 31) & ~31u;
+  const unsigned per = ((n + kWarps - 1) / kWarps + 31) & ~31u;
   const unsigned from = min(n, w * per), to = min(n, from + per);
   unsigned short* const mine = cnt + w * digits;
   for (int pass = 0, shift = 0; pass < passes; pass++, shift += width) {
@@ -626,13 +620,13 @@ __device__ __forceinline__ void sort_list(unsigned* list, unsigned n, unsigned* 
     }
     __syncthreads();
     unsigned sum = 0, total;
-    for (int g = t * each; g < (t + 1) * each; g++)
+    for (int g = t * each; g < min((t + 1) * each, digits); g++)
 #pragma unroll
-      for (int q = 0; q < kSortWarps; q++) sum += cnt[q * digits + g];
+      for (int q = 0; q < kWarps; q++) sum += cnt[q * digits + g];
     unsigned at = block_excl_scan(sum, sh, &total);
-    for (int g = t * each; g < (t + 1) * each; g++)
+    for (int g = t * each; g < min((t + 1) * each, digits); g++)
 #pragma unroll
-      for (int q = 0; q < kSortWarps; q++) {
+      for (int q = 0; q < kWarps; q++) {
         const unsigned c = cnt[q * digits + g];
         cnt[q * digits + g] = (unsigned short)at;
         at += c;
@@ -645,7 +639,7 @@ __device__ __forceinline__ void sort_list(unsigned* list, unsigned n, unsigned* 
       // far longer when all digits differ
       unsigned peers = __ballot_sync(0xffffffffu, ok);
 #pragma unroll
-      for (int q = 0; q < kDigit; q++)
+      for (int q = 0; q < kBits; q++)
         if (q < width) {
           const unsigned ones = __ballot_sync(0xffffffffu, dig >> q & 1u);
           peers &= dig >> q & 1u ? ones : ~ones;
@@ -663,31 +657,62 @@ __device__ __forceinline__ void sort_list(unsigned* list, unsigned n, unsigned* 
     in = out;
     out = x;
   }
-  for (unsigned e = t; e < n; e += kSortThreads) list[e] = in[e];
+  for (unsigned e = t; e < n; e += kThreads) list[e] = in[e];
   __syncthreads();
 }
-constexpr size_t sort_smem(int cap) { return 2 * (size_t)cap * 4 + (kSortWarps << kDigit) * 2; }
+constexpr size_t sort_smem(int cap, int warps, int bits) { return 2 * (size_t)cap * 4 + ((size_t)warps << bits) * 2; }
+constexpr size_t kShortSmem = sort_smem(kSortShort, kShortWarps, kShortBits);
+constexpr size_t kLongSmem = sort_smem(kSortLong, kLongWarps, kLongBits);
 
-__global__ void __launch_bounds__(kSortThreads) k_tile_sort(Tiles s) {
+__global__ void __launch_bounds__(32 * kShortWarps) k_tile_sort(Tiles s) {
   extern __shared__ __align__(16) unsigned sm[];
   const unsigned lo = s.starts[blockIdx.x], n = s.starts[blockIdx.x + 1] - lo;
-  if (n > 1 && n <= kSortShort) sort_list<kSortShort>(s.list + lo, n, sm);
+  if (n > 1 && n <= kSortShort) sort_list<kSortShort, kShortWarps, kShortBits>(s.list + lo, n, sm);
 }
-__global__ void __launch_bounds__(kSortThreads) k_tile_sort_long(Tiles s) {
-  extern __shared__ __align__(16) unsigned sm[];
-  __shared__ unsigned many[kSortThreads], found;
-  for (int t0 = blockIdx.x * kSortThreads; t0 < s.count(); t0 += gridDim.x * kSortThreads) {
-    if (threadIdx.x == 0) found = 0;
-    __syncthreads();
-    const int t = t0 + threadIdx.x;
-    if (t < s.count() && s.starts[t + 1] - s.starts[t] > kSortShort) many[atomicAdd(&found, 1u)] = t;
-    __syncthreads();
-    for (unsigned q = 0; q < found; q++) {
-      const unsigned lo = s.starts[many[q]], n = s.starts[many[q] + 1] - lo;
-      if (n <= kSortLong) sort_list<kSortLong>(s.list + lo, n, sm);
-      else sort_in_place(s.list + lo, n);
+
+// Lists longer than the shared memory: pieces of kPiece entries are sorted,
+// then merged two, four, ... at a time by a bitonic network, whose steps
+// across pieces run in place in the list; what is left of a merge inside a
+// piece is the piece's sort.  Every comparison is upward (the first step of a
+// merge pairs an entry with its mirror image), so that places past the end
+// count as larger and never move.
+constexpr unsigned kPiece = 1u << kPieceBits;
+static_assert(kPiece <= kSortLong, "a piece is sorted in shared memory");
+__device__ void sort_list_pieces(unsigned* list, unsigned n, unsigned* sm) {
+  auto pieces = [&]() {
+    for (unsigned b = 0; b < n; b += kPiece) sort_list<kSortLong, kLongWarps, kLongBits>(list + b, min(kPiece, n - b), sm);
+  };
+  pieces();
+  for (int top = kPieceBits; top < 31 && 1u << top < n; top++) {
+    for (int lg = top; lg >= kPieceBits; lg--) {
+      const unsigned h = 1u << lg, pairs = (((n - 1) >> (lg + 1)) + 1) << lg;
+      for (unsigned e = threadIdx.x; e < pairs; e += 32 * kLongWarps) {
+        const unsigned r = e & (h - 1), x = ((e >> lg) << (lg + 1)) + r, y = lg == top ? x + 2 * h - 1 - 2 * r : x + h;
+        if (y >= n) continue;
+        const unsigned vx = list[x], vy = list[y];
+        if (vy < vx) {
+          list[x] = vy;
+          list[y] = vx;
+        }
+      }
+      __syncthreads();
     }
+    pieces();
+  }
+}
+__global__ void __launch_bounds__(32 * kLongWarps) k_tile_sort_long(Tiles s) {
+  extern __shared__ __align__(16) unsigned sm[];
+  __shared__ unsigned taken;
+  const unsigned jobs = *s.jobs();
+  while (jobs > 0) {
+    if (threadIdx.x == 0) taken = atomicAdd(s.ticket(), 1u);
     __syncthreads();
+    const unsigned q = taken;
+    __syncthreads();
+    if (q >= jobs) break;
+    const unsigned t = *s.job(q), lo = s.starts[t], n = s.starts[t + 1] - lo;
+    if (n <= kSortLong) sort_list<kSortLong, kLongWarps, kLongBits>(s.list + lo, n, sm);
+    else sort_list_pieces(s.list + lo, n, sm);
   }
 }
 
@@ -1001,8 +1026,8 @@ bool tile_scratch(mg_particles p) {
   const size_t cap = (size_t)std::max<long long>(p->cap, 1), tiles = (size_t)s.tx * s.ty * s.tz;
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
   p->tileNone = !s.d.is3d || s.d.nx < 3 || s.d.ny < 3 || s.d.nz < 3 || 8 * cap > 0xffffffffu || s.ty > 65535 || s.tz > 65535 ||
-                cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem(kSortShort)) != cudaSuccess ||
-                cudaFuncSetAttribute(k_tile_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem(kSortLong)) != cudaSuccess ||
+                cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShortSmem) != cudaSuccess ||
+                cudaFuncSetAttribute(k_tile_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongSmem) != cudaSuccess ||
                 cudaMalloc(&p->tileMem, up((tiles + 1) * 4) + tiles * kLine * 4 + 8 * cap * 4) != cudaSuccess;
   if (p->tileNone) {
     cudaGetLastError();
@@ -1030,9 +1055,9 @@ void tile_mac(mg_particles p, const Tiles& s, const PartView& v, float* vel, flo
     count_launch();
     k_tile_lists<T, true><<<blocks, 256, 0, st>>>(s, v);
     count_launch();
-    k_tile_sort<<<s.count(), kSortThreads, sort_smem(kSortShort), st>>>(s);
+    k_tile_sort<<<s.count(), 32 * kShortWarps, kShortSmem, st>>>(s);
     count_launch();
-    k_tile_sort_long<<<std::min(152, (s.count() + kSortThreads - 1) / kSortThreads), kSortThreads, sort_smem(kSortLong), st>>>(s);
+    k_tile_sort_long<<<std::min(sm_count(), s.count()), 32 * kLongWarps, kLongSmem, st>>>(s);
   }
   count_launch();
   k_tile_splat<T><<<dim3(s.tx, s.ty, s.tz), 32, 0, st>>>(s, v, vel, old, w);

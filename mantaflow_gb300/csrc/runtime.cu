@@ -516,6 +516,7 @@ extern "C" int mg_solver_size(mg_solver s, int* nx, int* ny, int* nz) {
   return MG_OK;
 }
 
+int mgpu::sm_count() { return g_ctx.sms; }
 int mgpu::solver_info(mg_solver s, Dims* d, cudaStream_t* st) {
   if (!valid_solver(s)) return fail(MG_ERR_ARG, "invalid solver");
   *d = s->d;
