@@ -900,17 +900,17 @@ struct mg_particles_s {
   long long cap = 0, n = 0;
   float *x = nullptr, *y = nullptr, *z = nullptr;
   int* flag = nullptr;
-  // sorting scratch: keys and particle indices (ping-pong), per-tile digit
-  // counts and their scan's block totals, bucket starts (ncells + 1)
+  // Scratch of the transfers, ten words per particle: the tile lists of
+  // mapPartsToMAC, or the sort's keys and particle indices (ping-pong) and the
+  // particles in bucket order.  Beside it the sort's per-tile digit counts,
+  // their scan's block totals and the bucket starts (ncells + 1).
+  unsigned* scratch = nullptr;
   unsigned *keys[2] = {nullptr, nullptr}, *vals[2] = {nullptr, nullptr};
   unsigned *hist = nullptr, *sums = nullptr, *starts = nullptr;
   float* sorted[6] = {};  // positions and up to 3 values in bucket order
   void* stage = nullptr;  // 16 bytes per particle for record transfers
-  // scratch of mapPartsToMAC's tile lists, from its first call on, and whether
-  // it could not be had
-  void* tileMem = nullptr;
+  void* tileMem = nullptr;  // the tile lists' starts and counters, from the first mapPartsToMAC on
   Tiles tiles{};
-  bool tileNone = false;
 };
 
 struct mg_pdata_s {
@@ -936,15 +936,14 @@ bool valid_pdata(mg_pdata d) {
 
 void free_parts(mg_particles p) {
   cudaStreamSynchronize(p->st);
-  void* bufs[] = {p->x, p->y, p->z, p->flag, p->keys[0], p->keys[1], p->vals[0], p->vals[1], p->hist, p->sums,
-                  p->starts, p->stage, p->tileMem};
+  void* bufs[] = {p->x, p->y, p->z, p->flag, p->scratch, p->hist, p->sums, p->starts, p->stage, p->tileMem};
   for (void* b : bufs)
-    if (b) cudaFree(b);
-  for (float* b : p->sorted)
     if (b) cudaFree(b);
 }
 
 int tiles_of(long long n) { return (int)((n + kRsTile - 1) / kRsTile); }
+
+size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 int blocks_of(long long n, int b = 256) { return (int)std::max<long long>(1, (n + b - 1) / b); }
 
@@ -1009,13 +1008,14 @@ SortedParts sorted_copy(mg_particles p, const unsigned* sorted, const PartView& 
   return sp;
 }
 
-// Scratch for the tile lists: room for every particle in the eight tiles that
-// it can reach.  The larger tiles from a million cells on: with the small ones
-// 128^3 takes 2.31 instead of 1.58 ms.  Below, a large tile's list is too long
-// a serial walk for the few tiles there are (75 x 62 x 90: 0.52 instead of
-// 0.45 ms with the transfer back).
-bool tile_scratch(mg_particles p) {
-  if (p->tileMem || p->tileNone) return !p->tileNone;
+// Whether mapPartsToMAC takes the tile lists: in 3D, with room for every
+// particle in the eight tiles that it can reach (eight of the scratch's ten
+// words), and memory for the tiles' tables.  The larger tiles from a million
+// cells on: with the small ones 128^3 takes 2.31 instead of 1.58 ms.  Below, a
+// large tile's list is too long a serial walk for the few tiles there are
+// (75 x 62 x 90: 0.52 instead of 0.45 ms with the transfer back).
+bool tile_lists(mg_particles p) {
+  if (p->tileMem) return true;
   Tiles& s = p->tiles;
   s.d = p->d;
   s.large = s.d.n >= 1000000;
@@ -1024,19 +1024,18 @@ bool tile_scratch(mg_particles p) {
   s.ty = across(s.d.ny, TileLarge::y, TileSmall::y);
   s.tz = across(s.d.nz, TileLarge::z, TileSmall::z);
   const size_t cap = (size_t)std::max<long long>(p->cap, 1), tiles = (size_t)s.tx * s.ty * s.tz;
-  auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  p->tileNone = !s.d.is3d || s.d.nx < 3 || s.d.ny < 3 || s.d.nz < 3 || 8 * cap > 0xffffffffu || s.ty > 65535 || s.tz > 65535 ||
-                cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShortSmem) != cudaSuccess ||
-                cudaFuncSetAttribute(k_tile_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongSmem) != cudaSuccess ||
-                cudaMalloc(&p->tileMem, up((tiles + 1) * 4) + tiles * kLine * 4 + 8 * cap * 4) != cudaSuccess;
-  if (p->tileNone) {
+  if (!s.d.is3d || s.d.nx < 3 || s.d.ny < 3 || s.d.nz < 3 || 8 * cap > 0xffffffffu || s.ty > 65535 || s.tz > 65535) return false;
+  const size_t starts = align256((tiles + 1) * 4);
+  if (cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShortSmem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_tile_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongSmem) != cudaSuccess ||
+      cudaMalloc(&p->tileMem, starts + tiles * kLine * 4) != cudaSuccess) {
     cudaGetLastError();
     p->tileMem = nullptr;
     return false;
   }
   s.starts = (unsigned*)p->tileMem;
-  s.cursor = (unsigned*)((char*)p->tileMem + up((tiles + 1) * 4));
-  s.list = s.cursor + tiles * kLine;
+  s.cursor = (unsigned*)((char*)p->tileMem + starts);
+  s.list = p->scratch;
   return true;
 }
 
@@ -1111,18 +1110,21 @@ extern "C" int mg_particles_create(mg_solver s, long long capacity, mg_particles
   const long long histN = 256 * tiles;
   bool ok = cudaMalloc(&p->x, c * 4) == cudaSuccess && cudaMalloc(&p->y, c * 4) == cudaSuccess &&
             cudaMalloc(&p->z, c * 4) == cudaSuccess && cudaMalloc(&p->flag, c * 4) == cudaSuccess &&
-            cudaMalloc(&p->keys[0], c * 4) == cudaSuccess && cudaMalloc(&p->keys[1], c * 4) == cudaSuccess &&
-            cudaMalloc(&p->vals[0], c * 4) == cudaSuccess && cudaMalloc(&p->vals[1], c * 4) == cudaSuccess &&
-            cudaMalloc(&p->hist, histN * 4) == cudaSuccess &&
+            cudaMalloc(&p->scratch, 10 * align256(c * 4)) == cudaSuccess && cudaMalloc(&p->hist, histN * 4) == cudaSuccess &&
             cudaMalloc(&p->sums, ((histN + kRsTile - 1) / kRsTile) * 4) == cudaSuccess &&
             cudaMalloc(&p->starts, (p->d.n + 1) * 4) == cudaSuccess && cudaMalloc(&p->stage, c * 16) == cudaSuccess;
-  for (int q = 0; q < 6 && ok; q++) ok = cudaMalloc(&p->sorted[q], c * 4) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     free_parts(p);
     delete p;
     return set_error(MG_ERR_NOMEM, "BasicParticleSystem: out of device memory");
   }
+  auto part = [&](int q) { return p->scratch + q * (align256(c * 4) / 4); };
+  for (int q = 0; q < 2; q++) {
+    p->keys[q] = part(q);
+    p->vals[q] = part(2 + q);
+  }
+  for (int q = 0; q < 6; q++) p->sorted[q] = (float*)part(4 + q);
   {
     std::lock_guard<std::mutex> lk(g_partMu);
     g_parts.insert(p);
@@ -1279,7 +1281,7 @@ extern "C" int mg_map_parts_to_mac(mg_grid flags, mg_grid vel, mg_grid velOld, m
   if (ptype && pdata_of(parts, ptype, MG_INT, what)) return MG_ERR_ARG;
   const Dims& d = parts->d;
   const PartView pv = view_of(parts, ptype, exclude);
-  if (tile_scratch(parts)) {
+  if (tile_lists(parts)) {
     Tiles s = parts->tiles;
     s.n = parts->n;
     for (int c = 0; c < 3; c++) s.v[c] = partVel->c[c];
