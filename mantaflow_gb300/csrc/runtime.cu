@@ -103,6 +103,7 @@ struct mg_solver_s {
   size_t poolBytes = 0;  // free buffers in the pool
   size_t tmpBytes = 0;   // pool buffers handed out to temporaries
   // CG state (allocated on first solve)
+  size_t cgBytes = 0;  // device bytes of it, A0f and Aoff apart
   code_t* code = nullptr;
   float* A0f = nullptr;
   float* residual = nullptr;
@@ -223,7 +224,7 @@ static size_t held_bytes(mg_solver s) {
   size_t b = s->poolBytes + s->tmpBytes;
   for (auto g : s->grids) b += g->bytes() * (g->stage ? 2 : 1);
   const size_t n = (size_t)s->d.n;
-  if (s->code) b += n * (sizeof(code_t) + 4 * sizeof(float));
+  b += s->cgBytes;
   if (s->A0f) b += n * sizeof(float);
   if (s->Aoff) b += 3 * n * sizeof(float);
   if (s->mg) b += mg_hierarchy_bytes(s->mg);
@@ -379,6 +380,31 @@ extern "C" int mg_solver_create(int nx, int ny, int nz, int dim, mg_solver* out)
   return MG_OK;
 }
 
+// device memory of the CG state, counted
+template <class T>
+static cudaError_t cg_alloc(mg_solver s, T** p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) {
+    s->cgBytes += bytes;
+  } else {
+    *p = nullptr;
+    cudaGetLastError();
+  }
+  return e;
+}
+// the cluster sweeps' buffers: their bytes, and every pointer that owns one
+static size_t mic_cluster_bytes(const MicClusterScene& m) {
+  return mic_cluster_floats(m) * (3 * sizeof(float) + sizeof(unsigned) / 2) + mic_cluster_flag_bytes(m) +
+         mic_cluster_face_words(m) * sizeof(unsigned) + sizeof(unsigned);
+}
+static void free_mic_cluster(mg_solver s) {
+  MicClusterLaunch& m = s->micCluster;
+  cudaFree(m.one.cw); cudaFree(m.one.P); cudaFree(m.one.r); cudaFree(m.one.z); cudaFree(m.one.regular);
+  cudaFree(m.one.gface); cudaFree(m.counter);
+  m.one.cw = nullptr; m.one.P = m.one.r = m.one.z = nullptr; m.one.regular = nullptr; m.one.gface = nullptr;
+  m.counter = nullptr;
+}
+
 static void free_cg_state(mg_solver s) {
   cudaFree(s->code); cudaFree(s->A0f); cudaFree(s->residual); cudaFree(s->search); cudaFree(s->tmp); cudaFree(s->P);
   cudaFree(s->part); cudaFree(s->partf); cudaFree(s->sc); cudaFreeHost(s->scHost); cudaFree(s->intScratch);
@@ -392,14 +418,11 @@ static void free_cg_state(mg_solver s) {
   cudaFree(s->micWave.order); cudaFree(s->micWave.counter); cudaFree(s->micWave.exchange);
   cudaFree(s->micFace);
   s->micFace = nullptr;
-  // micCluster.error aliases mic.error
-  cudaFree(s->micCluster.one.cw); cudaFree(s->micCluster.one.P); cudaFree(s->micCluster.one.r);
-  cudaFree(s->micCluster.one.z); cudaFree(s->micCluster.one.gface);
-  cudaFree(s->micCluster.one.regular);
-  cudaFree(s->micCluster.counter);
+  free_mic_cluster(s);  // its error aliases mic.error
   s->micCluster = MicClusterLaunch{};
   cudaFree(s->Aoff);
   s->Aoff = nullptr;
+  s->cgBytes = 0;
   cudaGetLastError();  // a failed free must not surface as a later launch error
   s->micCol = MicColPlan{};
   s->micWave = MicWavePlan{};
@@ -1108,34 +1131,34 @@ extern "C" void mg_pressure_params_default(mg_pressure_params* p) {
 static int ensure_cg_state(mg_solver s) {
   if (s->code) return MG_OK;
   const size_t n = (size_t)s->d.n;
-  CK(cudaMalloc(&s->code, n * sizeof(code_t)));
-  CK(cudaMalloc(&s->residual, n * sizeof(float)));
-  CK(cudaMalloc(&s->search, n * sizeof(float)));
-  CK(cudaMalloc(&s->tmp, n * sizeof(float)));
+  CK(cg_alloc(s, &s->code, n * sizeof(code_t)));
+  CK(cg_alloc(s, &s->residual, n * sizeof(float)));
+  CK(cg_alloc(s, &s->search, n * sizeof(float)));
+  CK(cg_alloc(s, &s->tmp, n * sizeof(float)));
   s->nblocks = std::max(1, std::min(g_ctx.sms * 4, (int)((n + 255) / 256)));
   const dim3 g = grid3(s->d, dim3(32, 8, 1));
   const size_t nb3 = (size_t)g.x * g.y * g.z;
   int tx = (s->d.nx + 15) / 16, ty = (s->d.ny + 15) / 16, tz = (s->d.nz + 15) / 16;
   const size_t ntiles = (size_t)tx * ty * tz;
   s->partCount = std::max(std::max(2 * nb3, ntiles), (size_t)(2 * s->nblocks));
-  CK(cudaMalloc(&s->part, s->partCount * sizeof(double)));
-  CK(cudaMalloc(&s->partf, 2 * (size_t)s->nblocks * sizeof(float)));
-  CK(cudaMalloc(&s->sc, sizeof(CgScalars)));
+  CK(cg_alloc(s, &s->part, s->partCount * sizeof(double)));
+  CK(cg_alloc(s, &s->partf, 2 * (size_t)s->nblocks * sizeof(float)));
+  CK(cg_alloc(s, &s->sc, sizeof(CgScalars)));
   CK(cudaMemset(s->sc, 0, sizeof(CgScalars)));
   CK(cudaMallocHost(&s->scHost, sizeof(CgScalars)));
-  CK(cudaMalloc(&s->intScratch, 16 * sizeof(int)));
+  CK(cg_alloc(s, &s->intScratch, 16 * sizeof(int)));
   if (s->d.is3d) {
     MicPlan& m = s->mic;
     m.tx = tx; m.ty = ty; m.tz = tz;
     m.ntiles = (int)ntiles;
     std::vector<int> order(ntiles);
     mic_plan_order(tx, ty, tz, order.data());
-    CK(cudaMalloc(&m.order, ntiles * sizeof(int)));
+    CK(cg_alloc(s, &m.order, ntiles * sizeof(int)));
     CK(cudaMemcpy(m.order, order.data(), ntiles * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&m.tileDone, ntiles * sizeof(unsigned int)));
+    CK(cg_alloc(s, &m.tileDone, ntiles * sizeof(unsigned int)));
     CK(cudaMemset(m.tileDone, 0, ntiles * sizeof(unsigned int)));
-    CK(cudaMalloc(&m.counter, sizeof(int)));
-    CK(cudaMalloc(&m.error, sizeof(int)));
+    CK(cg_alloc(s, &m.counter, sizeof(int)));
+    CK(cg_alloc(s, &m.error, sizeof(int)));
     CK(cudaMemset(m.error, 0, sizeof(int)));
     m.ctas = g_ctx.sms * g_ctx.micCtasPerSm;
     // cluster sweeps (miccluster.cu) where the grid fits them, else
@@ -1149,30 +1172,9 @@ static int ensure_cg_state(mg_solver s) {
     MicClusterLaunch& mc = s->micCluster;
     s->useMicCluster = !s->useMicCol && !s->useMicWave && mk != "tile" && mk != "flow" && mic_cluster_plan(s->d, &mc.one);
     s->useMicFlow = !s->useMicCol && !s->useMicWave && !s->useMicCluster && mk != "tile";
-    if (s->useMicCluster) {
-      const size_t words = mic_cluster_face_words(mc.one);
-      const size_t nl = mic_cluster_floats(mc.one);
-      CK(cudaMalloc(&mc.one.cw, nl / 2 * sizeof(unsigned)));
-      CK(cudaMalloc(&mc.one.P, nl * sizeof(float)));
-      CK(cudaMalloc(&mc.one.r, nl * sizeof(float)));
-      CK(cudaMalloc(&mc.one.z, nl * sizeof(float)));
-      CK(cudaMalloc(&mc.one.regular, mic_cluster_flag_bytes(mc.one)));
-      CK(cudaMalloc(&mc.one.gface, words * sizeof(unsigned)));
-      CK(cudaMemset(mc.one.gface, 0xff, words * sizeof(unsigned)));
-      CK(cudaMalloc(&mc.counter, sizeof(unsigned)));
-      CK(cudaMemset(mc.counter, 0, sizeof(unsigned)));
-      mc.njobs = mic_cluster_jobs(mc.one);
-      mc.nscenes = 1;
-      mc.maxBlocks = mc.one.nby * mc.one.nbz;
-      mc.nlpMax = mc.one.nlp;
-      mc.maxParts = s->nblocks;
-      mc.one.nanNorm = FLT_MAX;
-      mc.error = m.error;
-      if ((size_t)mc.maxBlocks > s->partCount) return fail(MG_ERR_STATE, "MIC: partial buffer too small");
-    }
     if (s->useMicFlow) {
       const size_t words = mic_flow_face_words(m.ntiles);
-      CK(cudaMalloc(&s->micFace, words * sizeof(unsigned long long)));
+      CK(cg_alloc(s, &s->micFace, words * sizeof(unsigned long long)));
       CK(cudaMemset(s->micFace, 0, words * sizeof(unsigned long long)));
     }
     if (s->useMicWave) {
@@ -1183,11 +1185,11 @@ static int ensure_cg_state(mg_solver s) {
       w.nunits = w.nyb * w.nzb;
       std::vector<int> ord((size_t)w.nunits);
       mic_wave_order(w.nyb, w.nzb, ord.data());
-      CK(cudaMalloc(&w.order, ord.size() * sizeof(int)));
+      CK(cg_alloc(s, &w.order, ord.size() * sizeof(int)));
       CK(cudaMemcpy(w.order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice));
-      CK(cudaMalloc(&w.counter, sizeof(int)));
+      CK(cg_alloc(s, &w.counter, sizeof(int)));
       const size_t words = mic_wave_exchange_words(s->d, w.zw);
-      CK(cudaMalloc(&w.exchange, words * sizeof(unsigned long long)));
+      CK(cg_alloc(s, &w.exchange, words * sizeof(unsigned long long)));
       CK(cudaMemset(w.exchange, 0, words * sizeof(unsigned long long)));
       w.error = m.error;
       if ((size_t)w.nunits > s->partCount) return fail(MG_ERR_STATE, "MIC: partial buffer too small");
@@ -1198,17 +1200,53 @@ static int ensure_cg_state(mg_solver s) {
       c.nblocks = c.nby * c.nbz;
       std::vector<int> ord((size_t)c.nblocks);
       mic_col_order(c.nby, c.nbz, ord.data());
-      CK(cudaMalloc(&c.order, ord.size() * sizeof(int)));
+      CK(cg_alloc(s, &c.order, ord.size() * sizeof(int)));
       CK(cudaMemcpy(c.order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice));
-      CK(cudaMalloc(&c.prog, ord.size() * sizeof(unsigned long long)));
+      CK(cg_alloc(s, &c.prog, ord.size() * sizeof(unsigned long long)));
       CK(cudaMemset(c.prog, 0, ord.size() * sizeof(unsigned long long)));
-      CK(cudaMalloc(&c.counter, sizeof(int)));
+      CK(cg_alloc(s, &c.counter, sizeof(int)));
       c.error = m.error;
       c.pubMask = 7;  // progress published every 8 steps
       if ((size_t)c.nblocks > s->partCount) return fail(MG_ERR_STATE, "MIC: partial buffer too small");
     }
   }
   return MG_OK;
+}
+
+// the buffers of the cluster sweeps, which only MIC(0) solves need
+static int alloc_mic_cluster(mg_solver s) {
+  MicClusterLaunch& mc = s->micCluster;
+  const size_t words = mic_cluster_face_words(mc.one);
+  const size_t nl = mic_cluster_floats(mc.one);
+  CK(cudaMalloc(&mc.one.cw, nl / 2 * sizeof(unsigned)));
+  CK(cudaMalloc(&mc.one.P, nl * sizeof(float)));
+  CK(cudaMalloc(&mc.one.r, nl * sizeof(float)));
+  CK(cudaMalloc(&mc.one.z, nl * sizeof(float)));
+  CK(cudaMalloc(&mc.one.regular, mic_cluster_flag_bytes(mc.one)));
+  CK(cudaMalloc(&mc.one.gface, words * sizeof(unsigned)));
+  CK(cudaMemsetAsync(mc.one.gface, 0xff, words * sizeof(unsigned), s->stream));
+  CK(cudaMalloc(&mc.counter, sizeof(unsigned)));
+  CK(cudaMemsetAsync(mc.counter, 0, sizeof(unsigned), s->stream));
+  mc.njobs = mic_cluster_jobs(mc.one);
+  mc.nscenes = 1;
+  mc.maxBlocks = mc.one.nby * mc.one.nbz;
+  mc.nlpMax = mc.one.nlp;
+  mc.maxParts = s->nblocks;
+  mc.one.nanNorm = FLT_MAX;
+  mc.error = s->mic.error;
+  if ((size_t)mc.maxBlocks > s->partCount) return fail(MG_ERR_STATE, "MIC: partial buffer too small");
+  return MG_OK;
+}
+static int ensure_mic_cluster(mg_solver s) {
+  if (s->micCluster.counter) return MG_OK;
+  const int st = alloc_mic_cluster(s);
+  if (st) {
+    free_mic_cluster(s);
+    cudaGetLastError();  // the failed allocation's, already reported
+  } else {
+    s->cgBytes += mic_cluster_bytes(s->micCluster.one);
+  }
+  return st;
 }
 
 static MicPlan flow_plan(mg_solver s) {
@@ -1223,7 +1261,7 @@ static int wave_ctas(mg_solver s) {
 
 // the diagonal P in grid layout, which every MIC(0) but the cluster sweeps uses
 static int ensure_grid_p(mg_solver s) {
-  if (!s->P) CK(cudaMalloc(&s->P, (size_t)s->d.n * sizeof(float)));
+  if (!s->P) CK(cg_alloc(s, &s->P, (size_t)s->d.n * sizeof(float)));
   return MG_OK;
 }
 
@@ -1499,8 +1537,8 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
     const int e = mg_setup(s->mg, b, (float)((double)p->cgAccuracy * 1E-4), s->stream);
     if (e) return fail(MG_ERR_CUDA, std::string("multigrid setup failed: ") + cudaGetErrorString(cudaGetLastError()));
   }
-  if (pc == kPcMic && (b.Aif || !s->useMicCluster)) {
-    st = ensure_grid_p(s);
+  if (pc == kPcMic) {
+    st = mic_cluster_on(s, b) ? ensure_mic_cluster(s) : ensure_grid_p(s);
     if (st) return st;
     b.P = s->P;
   }
