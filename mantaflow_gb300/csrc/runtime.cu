@@ -1128,8 +1128,7 @@ extern "C" void mg_pressure_params_default(mg_pressure_params* p) {
   p->surfTens = 0.f;
 }
 
-static int ensure_cg_state(mg_solver s) {
-  if (s->code) return MG_OK;
+static int alloc_cg_state(mg_solver s) {
   const size_t n = (size_t)s->d.n;
   CK(cg_alloc(s, &s->code, n * sizeof(code_t)));
   CK(cg_alloc(s, &s->residual, n * sizeof(float)));
@@ -1211,6 +1210,14 @@ static int ensure_cg_state(mg_solver s) {
     }
   }
   return MG_OK;
+}
+
+// all of it or nothing: after a failed allocation the next call starts anew
+static int ensure_cg_state(mg_solver s) {
+  if (s->code) return MG_OK;
+  const int st = alloc_cg_state(s);
+  if (st) free_cg_state(s);
+  return st;
 }
 
 // the buffers of the cluster sweeps, which only MIC(0) solves need

@@ -1,0 +1,107 @@
+"""An allocation of the pressure solver's state that fails: the call reports it
+and the next call on the same solver starts anew and is right.
+
+The failure is made on the host: the library's objects are linked once more,
+with cudaMalloc wrapped by a function that answers cudaErrorMemoryAllocation
+for one call of the test's choice.  Runs in a child process, which loads that
+library instead of the usual one.
+"""
+import glob
+import os
+import subprocess
+import sys
+
+import pytest
+
+from tests.conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+SHIM = r"""
+#include <stddef.h>
+int __real_cudaMalloc(void** p, size_t bytes);
+static long left = -1;
+void fail_after(long calls) { left = calls; }
+int __wrap_cudaMalloc(void** p, size_t bytes) {
+  if (left == 0) {
+    left = -1;
+    return 2; /* cudaErrorMemoryAllocation */
+  }
+  if (left > 0) left--;
+  return __real_cudaMalloc(p, bytes);
+}
+"""
+
+CHILD = r"""
+import ctypes, sys
+import numpy as np
+from mantaflow_gb300 import _lib
+L = _lib.load(sys.argv[1])
+L.fail_after.argtypes = [ctypes.c_long]
+import mantaflow_gb300 as m
+from oracle import oracle as og
+
+shape = tuple(int(v) for v in sys.argv[2].split("x"))
+f = np.full(shape[::-1], og.FLUID, np.int32)
+og.init_domain(f, 0)
+og.fill_grid(f)
+og.set_open_bound(f, 0, "Y")
+v = (np.random.default_rng(1).random(f.shape + (3,), dtype=np.float32) - 0.5).astype(np.float32)
+if shape[2] == 1:
+    v[..., 2] = 0
+
+
+def solver():
+    s = m.Solver(name="alloc", gridSize=m.vec3(*shape), dim=3 if shape[2] > 1 else 2)
+    s.timestep = 1.0
+    flags, vel, p = s.create(m.FlagGrid), s.create(m.MACGrid), s.create(m.RealGrid)
+    m.copyArrayToGridReal(f, flags)
+    return s, flags, vel, p
+
+
+def solve(g):
+    s, flags, vel, p = g
+    m.copyArrayToGridReal(v, vel)
+    p.setConst(0.0)
+    m.solvePressure(flags=flags, vel=vel, pressure=p, preconditioner=m.PcMIC)
+    return p.numpy().copy()
+
+
+want = solve(solver())
+failed = 0
+for k in range(100):
+    g = solver()
+    L.fail_after(k)
+    try:
+        solve(g)
+    except m.MantaError as e:
+        assert "memory" in str(e), str(e)
+    else:
+        break
+    finally:
+        L.fail_after(-1)
+    failed += 1
+    assert np.array_equal(solve(g), want), "after allocation %d failed" % k
+print("failed", failed)
+"""
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    d = tmp_path_factory.mktemp("alloc")
+    (d / "shim.c").write_text(SHIM)
+    objs = sorted(glob.glob(os.path.join(ROOT, "mantaflow_gb300", "_build", "*.o")))
+    assert objs
+    subprocess.run(["gcc", "-fPIC", "-O1", "-c", str(d / "shim.c"), "-o", str(d / "shim.o")], check=True)
+    from mantaflow_gb300 import build
+    subprocess.run([build.nvcc()] + build.ARCH + ["-shared", "-o", str(d / "lib.so")] + objs + [str(d / "shim.o")] +
+                   ["-Xlinker", "--wrap=cudaMalloc", "-lcudart_static", "-lrt", "-lpthread", "-ldl"], check=True)
+    return str(d / "lib.so")
+
+
+@pytest.mark.parametrize("shape,mic,least", [("20x18x22", "cluster", 18), ("20x18x22", "flow", 13), ("24x30x1", "cluster", 8)])
+def test_next_call_starts_anew(library, shape, mic, least):
+    r = subprocess.run([sys.executable, "-c", CHILD, library, shape], cwd=ROOT, capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "MANTA_GB300_MIC": mic, "PYTHONPATH": ROOT})
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert int(r.stdout.split()[-1]) >= least  # the state's allocations, each failed once
