@@ -253,7 +253,7 @@ int engine_init(Engine& e, float dt) {
   }
   CKB(cudaMalloc(&e.dDone, sizeof(int)));
   CKB(cudaMalloc(&e.dMicCounter, 4 * sizeof(int)));
-  CKB(cudaMemset(e.dMicCounter, 0, 4 * sizeof(int)));
+  CKB(cudaMemsetAsync(e.dMicCounter, 0, 4 * sizeof(int), e.stream));
   return MG_OK;
 }
 

@@ -9,7 +9,7 @@ namespace mgpu {
 
 struct MgHierarchy;
 
-MgHierarchy* mg_hierarchy_create(const Dims& d);
+MgHierarchy* mg_hierarchy_create(const Dims& d, cudaStream_t stream);
 void mg_hierarchy_destroy(MgHierarchy* h);
 // forget the matrix: the next mg_setup builds the hierarchy again (the
 // reference deletes the GridMg of a PcMGDynamic solve, pressure.cpp:418-451).

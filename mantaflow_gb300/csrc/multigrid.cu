@@ -1670,7 +1670,8 @@ int ensure_paths() {
     if ((int)p.size() > kMaxPaths) return 1;
     g_npaths[dim - 2] = (int)p.size();
     if (cudaMemcpyToSymbol(c_paths, p.data(), p.size() * sizeof(Path), (size_t)(dim - 2) * kMaxPaths * sizeof(Path)) !=
-        cudaSuccess)
+            cudaSuccess ||
+        cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)  // every solver's stream reads them
       return 1;
   }
   const int dyn = (int)kCgDynSmem;
@@ -1843,6 +1844,7 @@ struct MgHierarchy {
   int ndict[kMaxLevels] = {};  // distinct stencils of the level (0: planes)
   size_t bytes = 0;
   std::vector<void*> allocs;
+  cudaStream_t stream = nullptr;  // the solver's: buffers are filled on it
   bool ok = true;
 
   template <typename T>
@@ -1853,7 +1855,7 @@ struct MgHierarchy {
       ok = false;
       return nullptr;
     }
-    cudaMemset(p, 0, nb);
+    if (cudaMemsetAsync(p, 0, nb, stream) != cudaSuccess) ok = false;
     allocs.push_back(p);
     bytes += nb;
     return (T*)p;
@@ -1887,10 +1889,11 @@ static int level0_planes(const Dims& d) {
   return best;
 }
 
-MgHierarchy* mg_hierarchy_create(const Dims& d) {
+MgHierarchy* mg_hierarchy_create(const Dims& d, cudaStream_t stream) {
   if (ensure_paths()) return nullptr;
   MgHierarchy* h = new MgHierarchy();
   h->d = d;
+  h->stream = stream;
   h->is3d = d.is3d;
   h->S = d.is3d ? 14 : 5;
   // level sizes (GridMg ctor, multigrid.cpp:240-265)
@@ -1946,7 +1949,7 @@ MgHierarchy* mg_hierarchy_create(const Dims& d) {
     while (f > 1 && h->lev[f - 1].n <= lim) f--;
     h->tailFirst = f;
     h->dlev = h->alloc<Lev>(L);
-    if (h->ok && cudaMemcpy(h->dlev, h->lev, sizeof(Lev) * (size_t)L, cudaMemcpyHostToDevice) != cudaSuccess) h->ok = false;
+    if (h->ok && cudaMemcpyAsync(h->dlev, h->lev, sizeof(Lev) * (size_t)L, cudaMemcpyHostToDevice, stream) != cudaSuccess) h->ok = false;
   }
   // dictionary buffers for the colour-blocked levels (the cluster tail's too
   // unless MANTAGPU_MG_NO_TAIL_DICT is set)

@@ -266,7 +266,9 @@ int tile_acquire(float** out) {
       cudaGetLastError();
       return set_error(MG_ERR_NOMEM, "WaveletNoiseField: out of device memory for the noise tile");
     }
-    if (cudaMemcpy(p, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
+    // every solver's stream reads the tile: it is there when this returns
+    if (cudaMemcpy(p, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
       cudaFree(p);
       return set_error(MG_ERR_CUDA, "WaveletNoiseField: uploading the noise tile failed");
     }

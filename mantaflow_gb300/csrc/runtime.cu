@@ -1128,6 +1128,9 @@ extern "C" void mg_pressure_params_default(mg_pressure_params* p) {
   p->surfTens = 0.f;
 }
 
+// The buffers are filled on the solver's stream, which the legacy stream (of
+// cudaMemset and cudaMemcpy) is not ordered with.  Copies from pageable host
+// memory have taken the data when they return.
 static int alloc_cg_state(mg_solver s) {
   const size_t n = (size_t)s->d.n;
   CK(cg_alloc(s, &s->code, n * sizeof(code_t)));
@@ -1143,7 +1146,7 @@ static int alloc_cg_state(mg_solver s) {
   CK(cg_alloc(s, &s->part, s->partCount * sizeof(double)));
   CK(cg_alloc(s, &s->partf, 2 * (size_t)s->nblocks * sizeof(float)));
   CK(cg_alloc(s, &s->sc, sizeof(CgScalars)));
-  CK(cudaMemset(s->sc, 0, sizeof(CgScalars)));
+  CK(cudaMemsetAsync(s->sc, 0, sizeof(CgScalars), s->stream));
   CK(cudaMallocHost(&s->scHost, sizeof(CgScalars)));
   CK(cg_alloc(s, &s->intScratch, 16 * sizeof(int)));
   if (s->d.is3d) {
@@ -1153,12 +1156,12 @@ static int alloc_cg_state(mg_solver s) {
     std::vector<int> order(ntiles);
     mic_plan_order(tx, ty, tz, order.data());
     CK(cg_alloc(s, &m.order, ntiles * sizeof(int)));
-    CK(cudaMemcpy(m.order, order.data(), ntiles * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(m.order, order.data(), ntiles * sizeof(int), cudaMemcpyHostToDevice, s->stream));
     CK(cg_alloc(s, &m.tileDone, ntiles * sizeof(unsigned int)));
-    CK(cudaMemset(m.tileDone, 0, ntiles * sizeof(unsigned int)));
+    CK(cudaMemsetAsync(m.tileDone, 0, ntiles * sizeof(unsigned int), s->stream));
     CK(cg_alloc(s, &m.counter, sizeof(int)));
     CK(cg_alloc(s, &m.error, sizeof(int)));
-    CK(cudaMemset(m.error, 0, sizeof(int)));
+    CK(cudaMemsetAsync(m.error, 0, sizeof(int), s->stream));
     m.ctas = g_ctx.sms * g_ctx.micCtasPerSm;
     // cluster sweeps (miccluster.cu) where the grid fits them, else
     // tile-dataflow sweeps (micflow.cu); MANTA_GB300_MIC selects the latter
@@ -1174,7 +1177,7 @@ static int alloc_cg_state(mg_solver s) {
     if (s->useMicFlow) {
       const size_t words = mic_flow_face_words(m.ntiles);
       CK(cg_alloc(s, &s->micFace, words * sizeof(unsigned long long)));
-      CK(cudaMemset(s->micFace, 0, words * sizeof(unsigned long long)));
+      CK(cudaMemsetAsync(s->micFace, 0, words * sizeof(unsigned long long), s->stream));
     }
     if (s->useMicWave) {
       MicWavePlan& w = s->micWave;
@@ -1185,11 +1188,11 @@ static int alloc_cg_state(mg_solver s) {
       std::vector<int> ord((size_t)w.nunits);
       mic_wave_order(w.nyb, w.nzb, ord.data());
       CK(cg_alloc(s, &w.order, ord.size() * sizeof(int)));
-      CK(cudaMemcpy(w.order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice));
+      CK(cudaMemcpyAsync(w.order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
       CK(cg_alloc(s, &w.counter, sizeof(int)));
       const size_t words = mic_wave_exchange_words(s->d, w.zw);
       CK(cg_alloc(s, &w.exchange, words * sizeof(unsigned long long)));
-      CK(cudaMemset(w.exchange, 0, words * sizeof(unsigned long long)));
+      CK(cudaMemsetAsync(w.exchange, 0, words * sizeof(unsigned long long), s->stream));
       w.error = m.error;
       if ((size_t)w.nunits > s->partCount) return fail(MG_ERR_STATE, "MIC: partial buffer too small");
     }
@@ -1200,9 +1203,9 @@ static int alloc_cg_state(mg_solver s) {
       std::vector<int> ord((size_t)c.nblocks);
       mic_col_order(c.nby, c.nbz, ord.data());
       CK(cg_alloc(s, &c.order, ord.size() * sizeof(int)));
-      CK(cudaMemcpy(c.order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice));
+      CK(cudaMemcpyAsync(c.order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
       CK(cg_alloc(s, &c.prog, ord.size() * sizeof(unsigned long long)));
-      CK(cudaMemset(c.prog, 0, ord.size() * sizeof(unsigned long long)));
+      CK(cudaMemsetAsync(c.prog, 0, ord.size() * sizeof(unsigned long long), s->stream));
       CK(cg_alloc(s, &c.counter, sizeof(int)));
       c.error = m.error;
       c.pubMask = 7;  // progress published every 8 steps
@@ -1538,7 +1541,7 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
     // afterwards; PcMGStatic keeps the first one (pressure.cpp:418-451)
     if (s->mg && preconditioner == MG_PC_MG_DYNAMIC) mg_hierarchy_reset(s->mg);
     if (!s->mg) {
-      s->mg = mg_hierarchy_create(d);
+      s->mg = mg_hierarchy_create(d, s->stream);
       if (!s->mg) return fail(MG_ERR_NOMEM, "solvePressureSystem: multigrid allocation failed");
     }
     const int e = mg_setup(s->mg, b, (float)((double)p->cgAccuracy * 1E-4), s->stream);
@@ -1850,7 +1853,7 @@ extern "C" int mg_multigrid_vcycle(mg_grid flags, mg_grid phi, mg_grid src, mg_g
     launch_ghost_fluid_diag(b, phi->f(), gfClamp, s->stream);
     CKL();
   }
-  mgpu::MgHierarchy* h = mg_hierarchy_create(s->d);
+  mgpu::MgHierarchy* h = mg_hierarchy_create(s->d, s->stream);
   if (!h) return fail(MG_ERR_NOMEM, "mg_multigrid_vcycle: multigrid allocation failed");
   CgScalars init{};
   CK(cudaMemcpyAsync(s->sc, &init, sizeof(CgScalars), cudaMemcpyHostToDevice, s->stream));
@@ -1875,7 +1878,7 @@ extern "C" int mg_multigrid_describe(mg_grid flags, mg_multigrid_layout* out) {
   PcgBuffers b = cg_buffers(s, flags, nullptr, nullptr);
   launch_make_codes(b, s->stream);
   CKL();
-  mgpu::MgHierarchy* h = mg_hierarchy_create(s->d);
+  mgpu::MgHierarchy* h = mg_hierarchy_create(s->d, s->stream);
   if (!h) return fail(MG_ERR_NOMEM, "mg_multigrid_describe: multigrid allocation failed");
   const int e = mg_setup(h, b, 1e-8f, s->stream);
   cudaStreamSynchronize(s->stream);
