@@ -174,4 +174,26 @@ struct FSum {
   __device__ __forceinline__ double value() const { return (double)h + (double)l; }
 };
 
+// The same with the error of the error kept as well, h + l + m: more than a
+// double's 53 bits, where threads' sums are added up without the FP64 pipe.
+// (A sum beyond the largest float is what a double would become in a float.)
+struct TSum {
+  float h = 0.f, l = 0.f, m = 0.f;
+  __device__ __forceinline__ void add(float p) {
+    const ff s = two_sum(h, p), t = two_sum(l, s.l);
+    h = s.h;
+    l = t.h;
+    m += t.l;
+  }
+  __device__ __forceinline__ void add(const TSum& b) {
+    const ff s = two_sum(h, b.h), t = two_sum(l, b.l), u = two_sum(t.h, s.l);
+    h = s.h;
+    l = u.h;
+    m = (m + b.m) + (t.l + u.l);
+  }
+  __device__ __forceinline__ double value() const {
+    return fabsf(h) <= FLT_MAX ? (double)h + ((double)l + (double)m) : (double)h;
+  }
+};
+
 }  // namespace mgpu

@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kMcThreads, 1) k_mic_cluster(McArgs a) {
   const int by = rank % nby, cz = rank / nby, bz = zb0 + cz;
   const int nyp = nby * kBlk;
   CgScalars* const sc = S.sc;
-  FSum acc;
+  TSum acc;
 
   constexpr int kSgn = kBack ? -1 : 1;
   const int u = w & (kMcWarps - 1), uy = u & 1, uz = u >> 1;  // the line bundle of this warp
