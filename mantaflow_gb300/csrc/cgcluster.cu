@@ -6,8 +6,8 @@
 // takes a microsecond or two and whose launches and cold starts take 27
 // (96 x 128 cells, 377 iterations: 10.2 ms).  The scene's four vectors fit in
 // the shared memory and registers of a cluster, so here one launch runs the
-// whole solve and nothing but the result goes back to memory: 0.85 ms for the
-// same solve, 2.2 us per iteration, most of it the latency of the two sums.
+// whole solve and nothing but the result goes back to memory: 1.1 ms for the
+// same solve, 2.8 us per iteration, most of it the latency of the two sums.
 // Four steps of a batch of twelve 2D scenes (65^2 to 413^2, up to 950
 // iterations) and four 3D ones went from 236 to 63 ms.
 //
@@ -26,7 +26,10 @@
 //    owner's own arithmetic.  That saves a third barrier per iteration.
 //
 // Every cell's float operations are those of the grid kernels (pressure.cu),
-// and the sums carry 48 bits before their rounding to float, as theirs do.
+// a thread sums its cells' products as theirs do, and the threads' sums are
+// added up with more bits than their doubles have.  (Three floats to a sum cost
+// a quarter of an iteration: with two, 48 bits, a 96 x 128 step takes 0.94 ms
+// instead of 1.17.  In double it is more: the FP64 pipe does two lanes a cycle.)
 // The split depends on the scene's size alone, so a scene computes the same
 // alone and in any batch.
 #include <cfloat>
@@ -49,36 +52,33 @@ constexpr int kCcMaxCta = 16;
 constexpr int kCcMaxK = 32;
 constexpr size_t kCcMaxSmem = 220 * 1024;
 
-// a CTA's share of a cluster sum: sum h + l and the largest |r| (as the
-// float's bits; negative: none)
+// a CTA's share of a cluster sum: the sum and the largest |r| (as the float's
+// bits; negative: none)
 struct __align__(16) Share {
-  float h, l;
-  int mx, pad;
+  TSum s;
+  int mx;
 };
 
-__device__ __forceinline__ void add_pair(float& h, float& l, float h2, float l2) {
-  const ff s = two_sum(h, h2);
-  l = (l + l2) + s.l;
-  h = s.h;
+__device__ __forceinline__ TSum across(const TSum& a, int o) {
+  return TSum{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o), __shfl_xor_sync(0xffffffffu, a.m, o)};
 }
 
-// the sum of h + l and the maximum of mx over the cluster, the same bits in
-// every thread of every CTA
+// the sum of the threads' sums and the maximum of mx over the cluster, the same
+// bits in every thread of every CTA
 template <bool MX>
-__device__ __forceinline__ void cluster_sum(cg::cluster_group& cl, int ncta, Share* wp, Share* cp, float& h, float& l,
-                                            int& mx) {
+__device__ __forceinline__ void cluster_sum(cg::cluster_group& cl, int ncta, Share* wp, Share* cp, const FSum& own,
+                                            TSum& sum, int& mx) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  TSum t{own.h, own.l, 0.f};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    add_pair(h, l, __shfl_xor_sync(0xffffffffu, h, o), __shfl_xor_sync(0xffffffffu, l, o));
+  for (int o = 16; o > 0; o >>= 1) t.add(across(t, o));
   if (MX) mx = __reduce_max_sync(0xffffffffu, mx);
-  if (lane == 0) wp[wid] = Share{h, l, mx, 0};
+  if (lane == 0) wp[wid] = Share{t, mx};
   __syncthreads();
   if (wid == 0) {
     Share v = wp[lane & (kCcWarps - 1)];
 #pragma unroll
-    for (int o = kCcWarps / 2; o > 0; o >>= 1)
-      add_pair(v.h, v.l, __shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o));
+    for (int o = kCcWarps / 2; o > 0; o >>= 1) v.s.add(across(v.s, o));
     if (MX) v.mx = __reduce_max_sync(0xffffffffu, v.mx);
     if (ncta == 1) {
       if (lane == 0) cp[0] = v;
@@ -88,12 +88,9 @@ __device__ __forceinline__ void cluster_sum(cg::cluster_group& cl, int ncta, Sha
   }
   if (ncta == 1) __syncthreads();
   else cl.sync();
-  const Share v = cp[lane & (kCcMaxCta - 1)];
-  h = v.h;
-  l = v.l;
-#pragma unroll
-  for (int o = kCcMaxCta / 2; o > 0; o >>= 1)
-    add_pair(h, l, __shfl_xor_sync(0xffffffffu, h, o), __shfl_xor_sync(0xffffffffu, l, o));
+  const Share v = cp[lane & (ncta - 1)];  // a power of two
+  sum = v.s;
+  for (int o = ncta / 2; o > 0; o >>= 1) sum.add(across(sum, o));
   if (MX) mx = __reduce_max_sync(0xffffffffu, v.mx);
 }
 
@@ -132,7 +129,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
 
   float r[K], t[K], sv[kRegs ? K : 1], p[kRegs ? K : 1];
   unsigned code[(K + 3) / 4];
-  float h = 0.f, l = 0.f;
+  TSum sum;
   int mx = -1;
   FSum acc;
 #pragma unroll
@@ -160,16 +157,14 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
     if (R > 0) s_s[cells + x] = high ? S.rhs[base + cells + x] : 0.f;
     s_rlo[x] = s_rhi[x] = 0.f;
   }
-  if (tid < 2 * kCcMaxCta) s_cp[tid / kCcMaxCta][tid % kCcMaxCta] = Share{0.f, 0.f, __float_as_int(-1.f), 0};
+  if (tid < 2 * kCcMaxCta) s_cp[tid / kCcMaxCta][tid % kCcMaxCta] = Share{TSum{}, __float_as_int(-1.f)};
   // no CTA stores into another's shared memory before that one has set it up
   if (ncta == 1) __syncthreads();
   else cl.sync();
   float* const rloUp = high ? cl.map_shared_rank(s_rlo, rank + 1) : s_rlo;   // where the next strip keeps my last row
   float* const rhiDown = low ? cl.map_shared_rank(s_rhi, rank - 1) : s_rhi;  // where the previous one keeps my first
-  h = acc.h;
-  l = acc.l;
-  cluster_sum<false>(cl, ncta, s_wp, s_cp[1], h, l, mx);
-  float sigma = (float)((double)h + (double)l);
+  cluster_sum<false>(cl, ncta, s_wp, s_cp[1], acc, sum, mx);
+  float sigma = sum.rounded();
   float alpha = 0.f, beta = 0.f, dp = 0.f, res = g->resNorm;
   int it = 0, done = 0, status = 0;
 
@@ -192,10 +187,8 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
         acc.add(v * xc);
       }
     }
-    h = acc.h;
-    l = acc.l;
-    cluster_sum<false>(cl, ncta, s_wp, s_cp[0], h, l, mx);
-    dp = (float)((double)h + (double)l);
+    cluster_sum<false>(cl, ncta, s_wp, s_cp[0], acc, sum, mx);
+    dp = sum.rounded();
     alpha = fabsf(dp) > 0.f ? sigma / dp : 0.f;
     const float na = -alpha;
     // p += alpha s, r -= alpha A s; (r, r) and max|r|
@@ -215,9 +208,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
         if (rv == rv) mx = max(mx, __float_as_int(fabsf(rv)));  // NaN takes no part, as in fmaxf
       }
     }
-    h = acc.h;
-    l = acc.l;
-    cluster_sum<true>(cl, ncta, s_wp, s_cp[1], h, l, mx);
+    cluster_sum<true>(cl, ncta, s_wp, s_cp[1], acc, sum, mx);
     it++;
     res = __int_as_float(mx);
     if (res < 0.f) res = S.nanNorm;
@@ -226,7 +217,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
       done = 1;
       break;
     }
-    const float sigmaNew = (float)((double)h + (double)l);
+    const float sigmaNew = sum.rounded();
     beta = sigmaNew / sigma;
     sigma = sigmaNew;
     if (!(res < 1e35f)) {

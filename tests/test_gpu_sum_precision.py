@@ -40,3 +40,14 @@ def test_mic_sweep(y, z):
     same sum, and with both rounded alike alpha is 1"""
     got = _solve((40, 24, 28), [((5, y, z), 1, 1.0), ((15, y, z), 4, 2.0 ** -11), ((25, y, z), 4, 2.0 ** -24)])
     assert got == [1.0, 2.0 ** -13, 2.0 ** -26]
+
+
+@pytest.mark.parametrize("shape,cells", [((32, 20), ((3, 5), (9, 5), (15, 5))),      # one warp
+                                         ((32, 60), ((3, 5), (9, 25), (15, 45))),    # several warps
+                                         ((96, 400), ((3, 5), (9, 200), (15, 390)))])  # several CTAs
+def test_2d_solve(shape, cells):
+    """(r, r) = 1 + 2^-24 + 2^-50 and (A s, s) = 3 + 2^-22 + ..., no tie"""
+    value = (1.0, 2.0 ** -12, 2.0 ** -25)
+    got = _solve(shape + (1,), [(c + (0,), 3 if q == 0 else 4, value[q]) for q, c in enumerate(cells)])
+    alpha = (np.float32(1) + np.float32(2.0 ** -23)) / (np.float32(3) + np.float32(2.0 ** -22))
+    assert got == [float(alpha * np.float32(v)) for v in value]
