@@ -1191,42 +1191,41 @@ __device__ __forceinline__ ff ff_div(ff a, ff b) {
 
 struct CoarseSmem {
   float2 p[kCoarseMax + 256];     // search vector, and zeros as far as the stencils reach
-  ff part[3][kTailThreads / 32];  // per-warp partial dot products
+  TSum part[3][kTailThreads / 32];  // per-warp partial dot products
 };
 constexpr int kCoarseCoefBytes = sizeof(float) * kCgNb * kCoarseMax;  // stencils, entry by entry
 
 // the barrier of the first `warps` warps
 __device__ __forceinline__ void coarse_sync(int warps) { asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory"); }
 
-// Sums over those warps of each thread's NV values, one or two.  The sums carry
-// their rounding errors in l and are normalised at the end (a butterfly step is
-// then a shuffle and one dependent addition).  Of two values, the lower lanes
-// add up the first and the upper ones the second.  Every warp adds up the same
-// partials in the same order, so all threads get the same bits.  A slot is
-// written again only two barriers after its last reading.
+// Sums over those warps of each thread's NV values, one or two, in three floats
+// (TSum: as long a chain as normalised pairs, and more bits).  Of two values, the
+// lower lanes add up the first and the upper ones the second.  Every warp adds up
+// the same partials in the same order, so all threads get the same bits.  A slot
+// is written again only two barriers after its last reading.
 template <int NV>
 __device__ __forceinline__ void coarse_dots(CoarseSmem& sm, int warps, int slot, ff* v) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool second = NV == 2 && lane >= 16;
-  auto add = [](ff a, ff b) {
-    const ff s = two_sum(a.h, b.h);
-    return ff{s.h, (a.l + b.l) + s.l};
+  auto across = [](const TSum& a, int o) {
+    return TSum{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o), __shfl_xor_sync(0xffffffffu, a.m, o)};
   };
-  auto across = [](ff a, int o) { return ff{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)}; };
   auto from = [](ff a, int l) { return ff{__shfl_sync(0xffffffffu, a.h, l), __shfl_sync(0xffffffffu, a.l, l)}; };
-  ff s = add(second ? v[NV - 1] : v[0], across(NV == 2 && !second ? v[NV - 1] : v[0], 16));
+  const ff own = second ? v[NV - 1] : v[0], other = NV == 2 && !second ? v[NV - 1] : v[0];
+  TSum s{own.h, own.l, 0.f};
+  s.add(across(TSum{other.h, other.l, 0.f}, 16));
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) s = add(s, across(s, o));
+  for (int o = 8; o > 0; o >>= 1) s.add(across(s, o));
   if ((lane & 15) == 0 && (NV == 2 || lane == 0)) sm.part[slot + second][w] = s;
   coarse_sync(warps);
-  s = (lane & 15) < warps ? sm.part[slot + second][lane & 15] : ff{0.f, 0.f};
-  if (warps > 8) s = add(s, across(s, 8));
-  if (warps > 4) s = add(s, across(s, 4));
-  if (warps > 2) s = add(s, across(s, 2));
-  s = add(s, across(s, 1));
-  s = two_sum(s.h, s.l);
-  v[0] = from(s, 0);
-  if (NV == 2) v[NV - 1] = from(s, 16);
+  s = (lane & 15) < warps ? sm.part[slot + second][lane & 15] : TSum{};
+  if (warps > 8) s.add(across(s, 8));
+  if (warps > 4) s.add(across(s, 4));
+  if (warps > 2) s.add(across(s, 2));
+  s.add(across(s, 1));
+  const ff r = two_sum(s.h, s.l + s.m);
+  v[0] = from(r, 0);
+  if (NV == 2) v[NV - 1] = from(r, 16);
 }
 
 // GridMg::solveCG (multigrid.cpp:793-902) on the coarsest level in one CTA.
@@ -1293,7 +1292,7 @@ __device__ void coarse_cg(const Lev& L, int S, float accuracy, CoarseSmem& sm, f
   if (t >= 32 * warps) return;
   long long slot[K];
   float dg[K], bv[K];
-  ff inv[K], x[K], r[K], z[K], p[K];
+  ff x[K], r[K], z[K], p[K];
 #pragma unroll
   for (int k = 0; k < K; k++) {
     const int u = t + k * threads;
@@ -1309,12 +1308,10 @@ __device__ void coarse_cg(const Lev& L, int S, float accuracy, CoarseSmem& sm, f
       dg[k] = 1.f;
       bv[k] = 0.f;
     }
-    inv[k].h = 1.f / dg[k];
-    inv[k].l = fmaf(-dg[k], inv[k].h, 1.f) / dg[k];
     // x = 0, so r = b - A*0 = b
     x[k] = ff{0.f, 0.f};
     r[k] = ff{bv[k], 0.f};
-    p[k] = z[k] = ff_mul(r[k], inv[k]);
+    p[k] = z[k] = ff_div_f(r[k], dg[k]);
   }
   auto publish = [&]() {
 #pragma unroll
@@ -1365,7 +1362,7 @@ __device__ void coarse_cg(const Lev& L, int S, float accuracy, CoarseSmem& sm, f
     for (int k = 0; k < K; k++) {
       x[k] = ff_add(x[k], ff_mul(alpha, p[k]));
       r[k] = ff_add(r[k], ff_neg(ff_mul(alpha, q[k])));
-      z[k] = ff_mul(r[k], inv[k]);
+      z[k] = ff_div_f(r[k], dg[k]);
     }
     d[0] = dot(r, r);
     d[1] = dot(r, z);
@@ -1942,9 +1939,10 @@ MgHierarchy* mg_hierarchy_create(const Dims& d, cudaStream_t stream) {
   if (const char* e = std::getenv("MANTAGPU_MG0_PLANES")) h->zc = std::max(2, std::atoi(e) & ~1);
   // the levels of at most kTailSlots storage slots (and the coarsest) run in
   // one cluster launch
-  if (h->ok && L > 1 && g_tailCta && (long long)h->size[L - 1][0] * h->size[L - 1][1] * h->size[L - 1][2] <= kCoarseMax) {
-    long long lim = kTailSlots;
-    if (const char* e = std::getenv("MANTAGPU_MG_TAIL_SLOTS")) lim = std::atoll(e);
+  long long lim = kTailSlots;
+  if (const char* e = std::getenv("MANTAGPU_MG_TAIL_SLOTS")) lim = std::atoll(e);  // negative: no cluster launch
+  if (h->ok && L > 1 && g_tailCta && lim >= 0 &&
+      (long long)h->size[L - 1][0] * h->size[L - 1][1] * h->size[L - 1][2] <= kCoarseMax) {
     int f = L - 1;
     while (f > 1 && h->lev[f - 1].n <= lim) f--;
     h->tailFirst = f;
