@@ -90,7 +90,9 @@ int mg_solver_set_memory_limit(mg_solver s, size_t bytes);
  * `limitNs` nanoseconds (default 200 ms; 0 restores it); the solve then
  * returns MG_ERR_TIMEOUT instead of hanging.  With stallNextSolve != 0 the
  * next MIC(0) solve's sweeps wait for tile words that no tile publishes, so
- * its first wait runs out: a failure-path test that leaves the GPU usable. */
+ * its first wait runs out: a failure-path test that leaves the GPU usable.
+ * (2: the copies into the cluster sweeps' shared memory do not come, whose
+ * limit is twice limitNs and a second.) */
 int mg_solver_set_wait_limit(mg_solver s, long long limitNs, int stallNextSolve);
 
 /* ---- grids (source/grid.cpp) --------------------------------------------- */

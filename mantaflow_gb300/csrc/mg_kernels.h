@@ -242,7 +242,7 @@ struct MicClusterLaunch {
   int* error;
   int* ndone;                     // finished scenes of a batch, or null
   long long waitNs;
-  bool stall;                     // the waits run out (failure-path tests)
+  int stall;                      // failure-path tests: 1 the words of a sweep never come, 2 its copies
   bool l2;                        // residual norm: sum of squares instead of max-abs
 };
 int mic_cluster_prepare();

@@ -84,7 +84,7 @@ struct McArgs {
   long long waitNs;
   int nlpMax;                      // levels the shared memory is laid out for
   int init;                        // backward for doInit: sigma instead of beta
-  int stall;                       // publish nothing (failure-path tests)
+  int stall;                       // failure-path tests: 1 publish nothing, 2 fetch nothing
 };
 
 // words of this CTA's shared memory
@@ -116,15 +116,37 @@ __device__ __forceinline__ void st_glob(unsigned* p, unsigned v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// A wait has lasted too long: the sweep is lost.  That ends the CG (done), so that
+// the solve's later launches return at once and the host reports the timeout.
+__device__ __noinline__ void give_up(int* error, CgScalars* sc) {
+  if (atomicExch(error, 7) == 0) {
+    sc->status = 3;
+    sc->done = 1;
+  }
+}
+
 // wait for a phase of an mbarrier, with pauses of `pause` ns and the timer
-// read only now and then: the warps that compute share the SM's pipes
-__device__ __forceinline__ void wait_bar(uint64_t* bar, uint32_t parity, long long limitNs, unsigned pause) {
+// read only now and then: the warps that compute share the SM's pipes.  When
+// the limit is over it is reported, and once more waited for as long (a copy
+// must not arrive in shared memory that is no longer this CTA's); after that a
+// thread's other waits are short.
+__device__ __forceinline__ void wait_bar(uint64_t* bar, uint32_t parity, long long& limitNs, unsigned pause, int* error,
+                                         CgScalars* sc) {
   unsigned long long t0 = 0ull;
+  bool told = false;
   for (unsigned n = 0; !mbar_try(bar, parity); n++) {
     if (pause) __nanosleep(pause);
     if ((n & 1023u) == 0u) {
       if (n == 0u) t0 = gtimer();
-      else if (gtimer() - t0 > (unsigned long long)limitNs) return;
+      else if (gtimer() - t0 > (unsigned long long)limitNs) {
+        if (told) {
+          limitNs = 1000000LL;
+          return;
+        }
+        give_up(error, sc);
+        told = true;
+        t0 = gtimer();
+      }
     }
   }
 }
@@ -136,15 +158,11 @@ __device__ __forceinline__ void bulk_s2g(void* dst, const void* src, uint32_t by
 }
 
 // true when a wait that began at t0 is to be given up: its time is over, or
-// another wait has given up.  That ends the CG (done), so that the solve's
-// later launches return at once and the host reports the timeout.
+// another wait has given up
 __device__ __noinline__ bool expired(unsigned long long t0, long long limit, int* error, CgScalars* sc) {
   if (*((volatile int*)error) != 0) return true;
   if (gtimer() - t0 <= (unsigned long long)limit) return false;
-  if (atomicExch(error, 7) == 0) {
-    sc->status = 3;
-    sc->done = 1;
-  }
+  give_up(error, sc);
   return true;
 }
 
@@ -365,7 +383,7 @@ __global__ void __launch_bounds__(kMcThreads, 1) k_mic_cluster(McArgs a) {
   auto s_p = [&](int st) { return stages + st * kStageWords + kVecWords; };
   auto s_bits = [&](int st) { return reinterpret_cast<unsigned*>(stages + st * kStageWords + 2 * kVecWords); };
   auto s_r = [&](int st) { return stages + st * kStageWords + 2 * kVecWords + kBitWords; };
-  const long long limit = 2 * a.waitNs + 1000000000LL;  // beyond what a computing warp's own waits can add up to
+  long long limit = 2 * a.waitNs + 1000000000LL;  // beyond what a computing warp's own waits can add up to
   // levels that a neighbour's word exists for: those with a cell inside the grid
   const int fLo = kBack ? 7 : 0, fHi = kBack ? nl : nx + 7;
   // gives up on behalf of the whole sweep once a wait has lasted too long
@@ -396,8 +414,8 @@ __global__ void __launch_bounds__(kMcThreads, 1) k_mic_cluster(McArgs a) {
       for (int q = 8 * fHi + lane; q < 8 * (nlp + kPad); q += 32) faceY[q] = faceZ[q] = 0u;
       // lanes whose neighbour is another warp's, or the outside (which counts as 0)
       const bool inY = ly == (kBack ? kUY - 1 : 0), inZ = lq == (kBack ? 3 : 0);
-      const unsigned outY = dnY && !a.stall && ly == (kBack ? 0 : kUY - 1);
-      const unsigned outZ = dnZ && !a.stall && lq == (kBack ? 0 : 3);
+      const unsigned outY = dnY && a.stall != 1 && ly == (kBack ? 0 : kUY - 1);
+      const unsigned outZ = dnZ && a.stall != 1 && lq == (kBack ? 0 : 3);
       // the next warps keep the word of this warp's level L at pub + stride * L
       // (it is their level L -+ 7; levels without a cell end up in the slack
       // or among words nobody reads)
@@ -437,7 +455,7 @@ __global__ void __launch_bounds__(kMcThreads, 1) k_mic_cluster(McArgs a) {
         float2* const vec = reinterpret_cast<float2*>(s_vec(st)) + lane;
         const float2* const pc = reinterpret_cast<const float2*>(s_p(st)) + lane;
         const unsigned* const cc = s_bits(st) + lane;
-        wait_bar(&s_full[u][st], (c / kStages) & 1, limit, 0);
+        wait_bar(&s_full[u][st], (c / kStages) & 1, limit, 0, a.error, sc);
         if (MODE != 0 && (regular >> ch & 1ull))
           mic_levels<MODE, true>(ms, inY, inZ, adY, adZ, outY, outZ, puY, puZ, strideZ, vec, pc, cc, readP, overdue);
         else
@@ -449,6 +467,7 @@ __global__ void __launch_bounds__(kMcThreads, 1) k_mic_cluster(McArgs a) {
     // ---- the copying warp: chunks in, kStages ahead, and their results out
     float* const out = (MODE == 0 ? S.P : S.z) + unit * nlp * 64;
     auto fetch = [&](int c) {
+      if (a.stall == 2) return;
       const int st = c % kStages;
       const long long at = (unit * nlp + (long long)(kBack ? nch - 1 - c : c) * kCH) * 32;
       const uint32_t vb = kVecWords * 4, bb = kBitWords * 4;
@@ -462,7 +481,7 @@ __global__ void __launch_bounds__(kMcThreads, 1) k_mic_cluster(McArgs a) {
       for (int c = 0; c < min(kStages, nch); c++) fetch(c);
     for (int c = 0; c < nch; c++) {
       const int st = c % kStages;
-      wait_bar(&s_done[u][st], (c / kStages) & 1, limit, 100);
+      wait_bar(&s_done[u][st], (c / kStages) & 1, limit, 100, a.error, sc);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the results, for the copy engine
       if (lane == 0) bulk_s2g(out + (long long)(kBack ? nch - 1 - c : c) * kVecWords, s_vec(st), kVecWords * 4);
       if (kBack) {
@@ -835,7 +854,7 @@ static McArgs mc_args(const MicClusterLaunch& m) {
   a.ndone = m.ndone;
   a.waitNs = m.waitNs;
   a.nlpMax = m.nlpMax;
-  a.stall = m.stall ? 1 : 0;
+  a.stall = m.stall;
   return a;
 }
 

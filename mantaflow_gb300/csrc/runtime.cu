@@ -129,8 +129,8 @@ struct mg_solver_s {
   bool useMicCluster = false;
   unsigned int epoch = 0;
   long long waitNs = kWaitNs;  // limit of each device-side MIC wait
-  bool stallNext = false;      // the next MIC solve's waits run out (test of the timeout path)
-  bool stall = false;          // ... during this solve
+  int stallNext = 0;           // the next MIC solve's waits run out (tests of the timeout path)
+  int stall = 0;               // ... during this solve
   size_t memLimit = 0;         // cap on the device memory the solver holds (0: none)
   mgpu::MgHierarchy* mg = nullptr;  // static multigrid cache (gMapMG)
   // one MG-PCG iteration captured as a CUDA graph, replayed while the
@@ -504,7 +504,7 @@ extern "C" int mg_solver_set_memory_limit(mg_solver s, size_t bytes) {
 extern "C" int mg_solver_set_wait_limit(mg_solver s, long long limitNs, int stallNextSolve) {
   if (!valid_solver(s) || limitNs < 0) return fail(MG_ERR_ARG, "mg_solver_set_wait_limit: invalid argument");
   s->waitNs = limitNs ? limitNs : kWaitNs;
-  s->stallNext = stallNextSolve != 0;
+  s->stallNext = stallNextSolve == 2 ? 2 : stallNextSolve != 0;
   return MG_OK;
 }
 
@@ -1581,7 +1581,7 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
   if (pc == kPcMic) {
     ProfScope ps(s, "mic_init");
     s->stall = s->stallNext;
-    s->stallNext = false;
+    s->stallNext = 0;
     CK(cudaMemsetAsync(s->mic.error, 0, sizeof(int), s->stream));
     if (b.Aif) launch_mic_planes(b, 0, s->stream);
     else if (s->useMicCluster) {
@@ -1676,7 +1676,7 @@ extern "C" int mg_solve_pressure_system(mg_grid rhs, mg_grid vel, mg_grid pressu
   CK(cudaMemcpyAsync(s->scHost, s->sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   if (pc == kPcMic) {
-    s->stall = false;
+    s->stall = 0;
     int err = 0;
     CK(cudaMemcpy(&err, s->mic.error, sizeof(int), cudaMemcpyDeviceToHost));
     if (err && s->useMicCluster) {

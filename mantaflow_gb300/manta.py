@@ -161,8 +161,9 @@ class Solver:
     def setWaitLimit(self, ns, stallNextSolve=False):
         """Limit of each device-side MIC(0) wavefront wait in nanoseconds (0:
         the default 200 ms).  stallNextSolve makes the next MIC(0) solve's
-        waits run out, to exercise the timeout path."""
-        check(_lib.load().mg_solver_set_wait_limit(self._h, int(ns), 1 if stallNextSolve else 0))
+        waits run out, to exercise the timeout path (2: those for the copies
+        into shared memory)."""
+        check(_lib.load().mg_solver_set_wait_limit(self._h, int(ns), int(stallNextSolve)))
 
     def __del__(self):
         h = getattr(self, "_h", None)
