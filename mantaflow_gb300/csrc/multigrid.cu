@@ -1148,11 +1148,13 @@ constexpr size_t kCgDynSmem = (size_t)kCgNb * kCgThreads * (sizeof(float) + size
 // the levels' results are bit-identical to them; vectors written inside
 // the launch are read at L2 (tail_ld).
 constexpr int kTailThreads = 512;
-// Largest level run inside the cluster, in storage slots.  With 57^3 (195 000)
-// in it a solve at 112^3 takes 2.26 ms instead of 1.89, with 41 x 50 x 36
-// (74 000) one at 161 x 199 x 143 as long as without (3.38 and 3.40 ms), with
-// the levels of 33^3 outside one at 256^3 0.25 ms longer.
-constexpr long long kTailSlots = 100000;
+// Largest level run inside the cluster, in storage slots.  A pass inside takes
+// 2.1 us and grows with the level, one outside costs a launch.  Solves with the
+// level in and out of it: 33^3 (39 000 slots) at 256^3 5.92 and 6.01 ms, 36^3
+// (47 000) at 140^3 3.01 and 3.09, 38^3 (55 000) at 150^3 2.74 and 2.73, 41 x 50
+// x 36 (74 000) at 161 x 199 x 143 3.36 and 3.21, 41^3 at 160^3 and 80^3 2.72 and
+// 2.60, 1.62 and 1.48.
+constexpr long long kTailSlots = 50000;
 constexpr int kCoarseMax = 2 * kTailThreads;  // coarsest-level vertices
 
 // A value that other CTAs of the launch write, and one that nobody writes.

@@ -50,3 +50,18 @@ def test_both_solvers_of_the_coarsest_level_agree(shape, monkeypatch):
     assert np.isfinite(p).all() and np.abs(p).max() > 0
     assert it == it2
     assert np.abs(p - q).max() <= 1e-5 * np.abs(q).max()
+
+
+@pytest.mark.parametrize("n,inside", [(256, 33), (140, 36), (160, 21)])
+def test_levels_of_the_cluster_launch(n, inside):
+    """the largest level that the cluster launch runs, by measured times: 33^3
+    and 36^3 are faster inside it, 41^3 is faster as launches of its own"""
+    import ctypes as C
+    from mantaflow_gb300 import _lib as mlib
+    s = m.Solver(name="levels", gridSize=m.vec3(n, n, n), dim=3)
+    flags = s.create(m.FlagGrid)
+    flags.initDomain()
+    flags.fillGrid()
+    lay = mlib.MultigridLayout()
+    mlib.check(mlib.load().mg_multigrid_describe(flags._h, C.byref(lay)))
+    assert lay.size[lay.tailFirst][0] == inside
