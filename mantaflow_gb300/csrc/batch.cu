@@ -67,19 +67,24 @@ Dims dims_of(int nx, int ny, int nz) {
   d.sz = d.is3d ? (long long)nx * ny : 0;
   return d;
 }
-// bytes of a 3D scene's MIC buffers: what the cluster sweeps need, or the
-// diagonal and face words of the tile sweeps
+// bytes of a 3D scene's MIC buffers: room for what any of the sweeps needs, the
+// diagonal and face words of the tile sweeps or the cluster sweeps' buffers.
+// (Which of them the GPU runs is known after mg_init only; a job's bytes are the
+// same before and after.)
 size_t mic_bytes(int nx, int ny, int nz) {
-  MicClusterScene m;
   const size_t n = (size_t)nx * ny * nz;
-  if (!mic_cluster_plan(dims_of(nx, ny, nz), &m))
-    return align256(n * sizeof(float)) +
-           align256(mic_flow_face_words(mic_tiles(nx) * mic_tiles(ny) * mic_tiles(nz)) * sizeof(unsigned long long));
-  const size_t f = mic_cluster_floats(m);
-  size_t b = align256(f * sizeof(float)) + align256(f / 2 * sizeof(unsigned)) + align256(mic_cluster_flag_bytes(m)) +
-             align256(mic_cluster_face_words(m) * sizeof(unsigned));
-  if (2 * f > 4 * n) b += 2 * align256(f * sizeof(float));  // else r and z share advection's scratch
-  return b;
+  size_t most = align256(n * sizeof(float)) +
+                align256(mic_flow_face_words(mic_tiles(nx) * mic_tiles(ny) * mic_tiles(nz)) * sizeof(unsigned long long));
+  for (int ctas = 8; ctas <= 16; ctas *= 2) {
+    MicClusterScene m;
+    if (!mic_cluster_plan_for(dims_of(nx, ny, nz), ctas, &m)) continue;
+    const size_t f = mic_cluster_floats(m);
+    size_t b = align256(f * sizeof(float)) + align256(f / 2 * sizeof(unsigned)) + align256(mic_cluster_flag_bytes(m)) +
+               align256(mic_cluster_face_words(m) * sizeof(unsigned));
+    if (2 * f > 4 * n) b += 2 * align256(f * sizeof(float));  // else r and z share advection's scratch
+    most = std::max(most, b);
+  }
+  return most;
 }
 
 // bytes of one scene's device block (3D scenes also hold the MIC diagonal

@@ -248,6 +248,7 @@ struct MicClusterLaunch {
 int mic_cluster_prepare();
 // geometry (d, nby, nbz, zper, nlp) of a scene; false: the tile sweeps run it
 bool mic_cluster_plan(const Dims& d, MicClusterScene* s);
+bool mic_cluster_plan_for(const Dims& d, int ctas, MicClusterScene* s);  // with clusters of 8 or 16 CTAs
 size_t mic_cluster_floats(const MicClusterScene& s);
 size_t mic_cluster_flag_bytes(const MicClusterScene& s);
 size_t mic_cluster_face_words(const MicClusterScene& s);

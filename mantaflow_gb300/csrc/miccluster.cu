@@ -824,16 +824,17 @@ int mic_cluster_prepare() {
 
 // A cluster spans the y range (16 lines per CTA) and as many z-blocks as
 // then fit; the slots of every level fit the shared memory.
-bool mic_cluster_plan(const Dims& d, MicClusterScene* s) {
-  if (!d.is3d || !g_mcCluster) return false;
+bool mic_cluster_plan_for(const Dims& d, int ctas, MicClusterScene* s) {
+  if (!d.is3d || !ctas) return false;
   s->d = d;
   s->nby = (d.ny + kBlk - 1) / kBlk;
   s->nbz = (d.nz + kBlk - 1) / kBlk;
   s->nlp = mc_levels(d.nx);
-  if (s->nby > g_mcCluster || s->nlp > 64 * kCH || mc_smem(s->nlp) > (size_t)kMcMaxSmem) return false;
-  s->zper = std::min(s->nbz, g_mcCluster / s->nby);
+  if (s->nby > ctas || s->nlp > 64 * kCH || mc_smem(s->nlp) > (size_t)kMcMaxSmem) return false;
+  s->zper = std::min(s->nbz, ctas / s->nby);
   return true;
 }
+bool mic_cluster_plan(const Dims& d, MicClusterScene* s) { return mic_cluster_plan_for(d, g_mcCluster, s); }
 static size_t mc_units(const MicClusterScene& s) { return (size_t)s.nby * s.nbz * kMcWarps; }
 size_t mic_cluster_floats(const MicClusterScene& s) { return mc_units(s) * s.nlp * 64; }
 size_t mic_cluster_flag_bytes(const MicClusterScene& s) { return mc_units(s) * (s.nlp / kCH); }
