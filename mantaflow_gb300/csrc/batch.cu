@@ -620,6 +620,19 @@ int engine_refine_buffers(Engine& e) {
   return changed ? engine_tables(e) : MG_OK;
 }
 
+// Whatever is queued on the side streams, the engine's stream waits for, also
+// where a solve ends early: what follows touches the scenes again.
+struct SideJoin {
+  Engine& e;
+  int used = 0;  // side streams
+  ~SideJoin() {
+    for (int q = 0; q < used; q++) {
+      cudaEventRecord(e.join[q], e.side[q]);
+      cudaStreamWaitEvent(e.stream, e.join[q], 0);
+    }
+  }
+};
+
 // One batched GridCg solve (pressure.cpp:407-419) of every scene not
 // skipped, each to its own accuracy: PcMIC in 3D with (int)(cgMaxIterFac *
 // max size) iterations at most; in 2D GridCg drops MIC (conjugategrad.cpp:
@@ -646,9 +659,10 @@ int engine_cg(Engine& e, BatchMic& mic, const std::vector<float>& acc, const std
   CKB(cudaMemcpyAsync(e.dDone, &nskip, sizeof(int), cudaMemcpyHostToDevice, st));
   launch_b_pcg_init(e.dTiles, nt, e.dScenes, st);
   // the cluster scenes' solves, beside everything below
+  SideJoin side{e};
   const int nside = std::min((int)e.groups.size(), kSideStreams);
   if (nside) CKB(cudaEventRecord(e.fork, st));
-  for (int q = 0; q < nside; q++) CKB(cudaStreamWaitEvent(e.side[q], e.fork, 0));
+  for (; side.used < nside; side.used++) CKB(cudaStreamWaitEvent(e.side[side.used], e.fork, 0));
   for (size_t q = 0; q < e.groups.size(); q++) {
     const ClusterGroup& g = e.groups[q];
     CKB(launch_cg_cluster(g.plan, e.dCluster + g.first, CgClusterScene{}, g.count, g.a0, e.side[q % kSideStreams]));
@@ -781,6 +795,7 @@ int engine_cg(Engine& e, BatchMic& mic, const std::vector<float>& acc, const std
   }
   *sweepsOut = sweeps;
   for (int q = 0; q < nside; q++) CKB(cudaStreamWaitEvent(st, e.join[q], 0));
+  side.used = 0;
   CKB(cudaStreamSynchronize(st));
   return MG_OK;
 }

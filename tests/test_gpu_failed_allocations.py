@@ -1,5 +1,6 @@
 """An allocation of the pressure solver's state that fails: the call reports it
-and the next call on the same solver starts anew and is right.
+and the next call on the same solver starts anew and is right.  In a batch: when
+the call returns, no solve of another stream is still at work on the scenes.
 
 The failure is made on the host: the library's objects are linked once more,
 with cudaMalloc wrapped by a function that answers cudaErrorMemoryAllocation
@@ -86,6 +87,45 @@ print("failed", failed)
 """
 
 
+BATCH = r"""
+import ctypes, sys, time
+import numpy as np
+from mantaflow_gb300 import _lib
+L = _lib.load(sys.argv[1])
+L.fail_after.argtypes = [ctypes.c_long]
+from mantaflow_gb300 import batch as mb
+from mantaflow_gb300._lib import MantaError
+
+# 2D scenes of hundreds of iterations on the side streams, a 3D one beside them
+sizes = [(511, 512, 1), (500, 480, 1), (300, 420, 1), (24, 24, 24)]
+
+
+def batch():
+    return mb.BatchedPlumes(sizes, [(0, -4e-3, 0)] * len(sizes), range(len(sizes)), cgAccuracy=1e-5)
+
+
+failed = 0
+for k in range(40):
+    b = batch()
+    L.fail_after(k)
+    try:
+        b.step()
+    except MantaError as e:
+        assert "memory" in str(e), str(e)
+    else:
+        break
+    finally:
+        L.fail_after(-1)
+    failed += 1
+    first = [b.download(q, mb.PRESSURE) for q in range(len(sizes))]
+    time.sleep(0.2)
+    for q in range(len(sizes)):
+        assert np.array_equal(first[q], b.download(q, mb.PRESSURE)), "allocation %d: scene %d was still being solved" % (k, q)
+    b.close()
+print("failed", failed)
+"""
+
+
 @pytest.fixture(scope="module")
 def library(tmp_path_factory):
     d = tmp_path_factory.mktemp("alloc")
@@ -105,3 +145,10 @@ def test_next_call_starts_anew(library, shape, mic, least):
                        env={**os.environ, "MANTA_GB300_MIC": mic, "PYTHONPATH": ROOT})
     assert r.returncode == 0, r.stderr[-2000:]
     assert int(r.stdout.split()[-1]) >= least  # the state's allocations, each failed once
+
+
+def test_batch_leaves_nothing_running(library):
+    r = subprocess.run([sys.executable, "-c", BATCH, library], cwd=ROOT, capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "PYTHONPATH": ROOT})
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert int(r.stdout.split()[-1]) >= 7  # scenes, scalars, cluster and MIC scenes, tiles, sweep list, jobs: each failed once
