@@ -419,7 +419,8 @@ int mg_batch_download(mg_batch b, int scene, int what, void* host, size_t bytes)
 int mg_batch_noise(unsigned long long seed, int step, long long cells, float* out);
 int mg_batch_info(mg_batch b, int* count, long long* cells, long long* tiles, size_t* bytes);
 /* the CG sweep tile height the batch's autotuner chose over its first solves
- * (0 before) and the four timings (ms per lag sweeps, 8/16/32/64 rows) */
+ * (0 before; the smallest where no scene's solve sweeps over tiles, and then
+ * nothing is timed) and the four timings (ms per lag sweeps, 8/16/32/64 rows) */
 int mg_batch_tuning(mg_batch b, int* sweepRows, float* ms);
 int mg_batch_sync(mg_batch b);
 

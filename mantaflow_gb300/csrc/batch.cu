@@ -205,6 +205,7 @@ struct Engine {
   size_t activeCap = 0;
   bool dirty = true;
   int rowsK = -1;      // the tuned tile height; -1 while tuning
+  bool untiled = false;  // the last solve had no sweeps over tiles: nothing to tune
   int tuneK = 0;       // the height timed next
   int tuneSpoilt = 0;  // timings dropped because a scene finished during them
   float tuneMs[4] = {0.f, 0.f, 0.f, 0.f};
@@ -725,6 +726,7 @@ int engine_cg(Engine& e, BatchMic& mic, const std::vector<float>& acc, const std
   };
   if (rebuild()) return MG_ERR_CUDA;
   const bool tuning = e.rowsK < 0;
+  e.untiled = std::find(e.onCluster.begin(), e.onCluster.end(), 0) == e.onCluster.end();
   while (active > 0 && sweeps < maxIterAll) {
     // `lag` sweeps run as one CUDA graph, captured for the current sweep list
     // and captured again when it changes
@@ -1024,7 +1026,7 @@ extern "C" int mg_batch_noise(unsigned long long seed, int step, long long cells
 
 extern "C" int mg_batch_tuning(mg_batch b, int* sweepRows, float* ms) {
   if (!b) return set_error(MG_ERR_ARG, "mg_batch_tuning: null batch");
-  if (sweepRows) *sweepRows = b->e.rowsK < 0 ? 0 : kBTY << b->e.rowsK;
+  if (sweepRows) *sweepRows = b->e.rowsK >= 0 ? kBTY << b->e.rowsK : b->e.untiled ? kBTY : 0;
   if (ms)
     for (int q = 0; q < 4; q++) ms[q] = b->e.tuneMs[q];
   return MG_OK;
