@@ -207,7 +207,7 @@ struct Engine {
   int rowsK = -1;      // the tuned tile height; -1 while tuning
   bool untiled = false;  // the last solve had no sweeps over tiles: nothing to tune
   int tuneK = 0;       // the height timed next
-  int tuneSpoilt = 0;  // timings dropped because a scene finished during them
+  int tuneSpoilt = 0;  // timings dropped: a scene finished during them, or 2D solves ran beside
   float tuneMs[4] = {0.f, 0.f, 0.f, 0.f};
   cudaEvent_t ev[2] = {nullptr, nullptr};
   int* dDone = nullptr;
@@ -621,6 +621,14 @@ int engine_refine_buffers(Engine& e) {
   return changed ? engine_tables(e) : MG_OK;
 }
 
+// the fastest of the heights that were timed (8 rows where none was)
+int best_height(const float* ms) {
+  int best = 0;
+  for (int q = 1; q < 4; q++)
+    if (ms[q] > 0.f && (ms[best] <= 0.f || ms[q] < ms[best])) best = q;
+  return best;
+}
+
 // Whatever is queued on the side streams, the engine's stream waits for, also
 // where a solve ends early: what follows touches the scenes again.
 struct SideJoin {
@@ -700,9 +708,12 @@ int engine_cg(Engine& e, BatchMic& mic, const std::vector<float>& acc, const std
     CKB(launch_mic_level(mic.mc, kMicSearch, st));
   }
   // CG sweeps over the tiles of the scenes still iterating.  Autotuner: runs
-  // of lag sweeps in which no scene finishes are timed with events, one with
-  // tiles 8, 16, 32 and 64 rows tall each, over as many solves as that takes,
-  // and the fastest is kept; results do not depend on the choice.
+  // of lag sweeps in which no scene finishes, with no 2D solve beside them any
+  // more, are timed with events, one with tiles 8, 16, 32 and 64 rows tall
+  // each, over as many solves as that takes, and the fastest is kept; after
+  // sixteen runs that came to nothing, the fastest of those timed.  Results do
+  // not depend on the choice.
+  bool alone = false;
   int kk = e.rowsK >= 0 ? e.rowsK : e.tuneK;
   int active = 0, doneSeen = -1, sweeps = 0;
   (void)nt;
@@ -755,7 +766,12 @@ int engine_cg(Engine& e, BatchMic& mic, const std::vector<float>& acc, const std
         }
         e.graphKey = key;
       }
-      if (tuning && e.rowsK < 0) CKB(cudaEventRecord(e.ev[0], st));  // after the capture, which is host time
+      if (tuning && e.rowsK < 0) {
+        CKB(cudaEventRecord(e.ev[0], st));  // after the capture, which is host time
+        alone = true;
+        for (int q = 0; q < nside; q++) alone = alone && cudaEventQuery(e.join[q]) == cudaSuccess;
+        if (!alone) cudaGetLastError();  // "not ready" is no failure
+      }
       CKB(cudaGraphLaunch(e.sweepGraph, st));
       g_launches.fetch_add(e.graphNodes, std::memory_order_relaxed);
       e.graphLaunches++;
@@ -771,16 +787,16 @@ int engine_cg(Engine& e, BatchMic& mic, const std::vector<float>& acc, const std
       int nd = 0;
       CKB(cudaMemcpyAsync(&nd, e.dDone, sizeof(int), cudaMemcpyDeviceToHost, st));
       CKB(cudaStreamSynchronize(st));
-      if (timing && nd == (doneSeen < 0 ? nskip : doneSeen)) {
+      if (timing && alone && nd == (doneSeen < 0 ? nskip : doneSeen)) {
         CKB(cudaEventElapsedTime(&e.tuneMs[kk], e.ev[0], e.ev[1]));
         if (e.tuneK < 3) {
           kk = ++e.tuneK;
           relist = true;
         } else {
-          e.rowsK = (int)(std::min_element(e.tuneMs, e.tuneMs + 4) - e.tuneMs);
+          e.rowsK = best_height(e.tuneMs);
         }
       } else if (timing && ++e.tuneSpoilt >= 16) {
-        e.rowsK = 0;  // scenes that never run lag sweeps together
+        e.rowsK = best_height(e.tuneMs);
       }
       if (e.rowsK >= 0 && kk != e.rowsK) {
         kk = e.rowsK;
