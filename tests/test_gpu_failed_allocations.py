@@ -126,6 +126,46 @@ print("failed", failed)
 """
 
 
+SPLAT = r"""
+import ctypes, sys
+import numpy as np
+from mantaflow_gb300 import _lib
+L = _lib.load(sys.argv[1])
+L.fail_after.argtypes = [ctypes.c_long]
+import mantaflow_gb300 as m
+from oracle import oracle as og
+
+rng = np.random.default_rng(4)
+s = m.Solver(name="splat", gridSize=m.vec3(21, 18, 26), dim=3)
+flags, vel, velOld = s.create(m.FlagGrid), s.create(m.MACGrid), s.create(m.MACGrid)
+flags.initDomain(boundaryWidth=0)
+flags.fillGrid()
+pos = rng.uniform(0, 18, size=(30000, 3)).astype(np.float32)
+pp = s.create(m.BasicParticleSystem)
+pp.setPositions(pos, np.zeros(len(pos), np.int32))
+pv = rng.standard_normal(pos.shape).astype(np.float32)
+pvel = pp.create(m.PdataVec3)
+m.copyArrayToPdataVec3(pv, pvel)
+pp._flush()
+f = flags.numpy()
+v0, v1 = np.zeros(f.shape + (3,), np.float32), np.zeros(f.shape + (3,), np.float32)
+og.map_parts_to_mac(f, v0, v1, pos, np.zeros(len(pos), np.int32), pv)
+launches = []
+for fail in (True, False, False):
+    if fail:
+        L.fail_after(0)
+    n0 = ctypes.c_longlong()
+    n1 = ctypes.c_longlong()
+    L.mg_launch_count(ctypes.byref(n0))
+    m.mapPartsToMAC(flags=flags, vel=vel, velOld=velOld, parts=pp, partVel=pvel)
+    L.mg_launch_count(ctypes.byref(n1))
+    launches.append(n1.value - n0.value)
+    L.fail_after(-1)
+    assert np.array_equal(vel.numpy(), v0) and np.array_equal(velOld.numpy(), v1)
+print("launches", *launches)
+"""
+
+
 @pytest.fixture(scope="module")
 def library(tmp_path_factory):
     d = tmp_path_factory.mktemp("alloc")
@@ -152,3 +192,13 @@ def test_batch_leaves_nothing_running(library):
                        env={**os.environ, "PYTHONPATH": ROOT})
     assert r.returncode == 0, r.stderr[-2000:]
     assert int(r.stdout.split()[-1]) >= 7  # scenes, scalars, cluster and MIC scenes, tiles, sweep list, jobs: each failed once
+
+
+def test_splat_without_tables(library):
+    """mapPartsToMAC in 3D whose tables cannot be had: that call sorts by cell,
+    with the same result, and the next one has the tile lists"""
+    r = subprocess.run([sys.executable, "-c", SPLAT, library], cwd=ROOT, capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "PYTHONPATH": ROOT})
+    assert r.returncode == 0, r.stderr[-2000:]
+    sorts, lists, again = (int(v) for v in r.stdout.split()[1:])
+    assert lists == again == 6 and sorts > 20
