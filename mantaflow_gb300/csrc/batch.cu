@@ -571,7 +571,7 @@ int engine_tables(Engine& e) {
     CgClusterPlan pl;
     if (b.mic || !cg_cluster_plan(b.d, b.A0f != nullptr, &pl)) continue;
     e.onCluster[q] = 1;
-    shapes[{-pl.k, -(2 * pl.ctas + (b.A0f ? 1 : 0))}].push_back({q, pl});
+    shapes[{-pl.k * pl.threads, -(2 * pl.ctas + (b.A0f ? 1 : 0))}].push_back({q, pl});
   }
   for (auto& kv : shapes) {
     ClusterGroup g{kv.second[0].second, e.hScenes[kv.second[0].first].A0f != nullptr, (int)e.hCluster.size(),

@@ -6,13 +6,13 @@
 // takes a microsecond or two and whose launches and cold starts take 27
 // (96 x 128 cells, 377 iterations: 10.2 ms).  The scene's four vectors fit in
 // the shared memory and registers of a cluster, so here one launch runs the
-// whole solve and nothing but the result goes back to memory: 1.1 ms for the
-// same solve, 2.8 us per iteration, most of it the latency of the two sums.
+// whole solve and nothing but the result goes back to memory: 0.95 ms for the
+// same solve, 2.5 us per iteration, most of it the latency of the two sums.
 // Four steps of a batch of twelve 2D scenes (65^2 to 413^2, up to 950
 // iterations) and four 3D ones went from 236 to 63 ms.
 //
-//  * CTA k of the cluster owns a strip of whole rows; thread t holds the
-//    strip's cells t, t + 512, ... (K of them): residual, A s and, up to 16
+//  * CTA k of the cluster owns a strip of whole rows; thread t of T holds the
+//    strip's cells t, t + T, ... (K of them): residual, A s and, up to 16
 //    cells per thread, search value and pressure in registers.  The search
 //    vector is also in shared memory for the neighbours, with one halo row on
 //    each side.
@@ -28,8 +28,8 @@
 // Every cell's float operations are those of the grid kernels (pressure.cu),
 // a thread sums its cells' products as theirs do, and the threads' sums are
 // added up with more bits than their doubles have.  (Three floats to a sum cost
-// a quarter of an iteration: with two, 48 bits, a 96 x 128 step takes 0.94 ms
-// instead of 1.17.  In double it is more: the FP64 pipe does two lanes a cycle.)
+// instructions: with two, 48 bits, a 96 x 128 step takes 0.94 ms instead of 1.04.
+// In double it is more: the FP64 pipe does two lanes a cycle.)
 // The split depends on the scene's size alone, so a scene computes the same
 // alone and in any batch.
 #include <cfloat>
@@ -46,10 +46,12 @@ namespace mgpu {
 
 namespace {
 
-constexpr int kCcThreads = 512;
-constexpr int kCcWarps = kCcThreads / 32;
+constexpr int kCcThreads = 512;     // of a CTA with a long strip
+constexpr int kCcSmall = 256;       // of one with up to kCcStrip cells
+constexpr int kCcStrip = 2048;
 constexpr int kCcMaxCta = 16;
 constexpr int kCcMaxK = 32;
+static_assert(kCcStrip <= 8 * kCcSmall && kCcStrip >= 4 * kCcThreads, "the cells per thread that kernel_of has");
 constexpr size_t kCcMaxSmem = 220 * 1024;
 
 // a CTA's share of a cluster sum: the sum and the largest |r| (as the float's
@@ -65,9 +67,10 @@ __device__ __forceinline__ TSum across(const TSum& a, int o) {
 
 // the sum of the threads' sums and the maximum of mx over the cluster, the same
 // bits in every thread of every CTA
-template <bool MX>
+template <int T, bool MX>
 __device__ __forceinline__ void cluster_sum(cg::cluster_group& cl, int ncta, Share* wp, Share* cp, const FSum& own,
                                             TSum& sum, int& mx) {
+  constexpr int kWarps = T / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   TSum t{own.h, own.l, 0.f};
 #pragma unroll
@@ -76,9 +79,9 @@ __device__ __forceinline__ void cluster_sum(cg::cluster_group& cl, int ncta, Sha
   if (lane == 0) wp[wid] = Share{t, mx};
   __syncthreads();
   if (wid == 0) {
-    Share v = wp[lane & (kCcWarps - 1)];
+    Share v = wp[lane & (kWarps - 1)];
 #pragma unroll
-    for (int o = kCcWarps / 2; o > 0; o >>= 1) v.s.add(across(v.s, o));
+    for (int o = kWarps / 2; o > 0; o >>= 1) v.s.add(across(v.s, o));
     if (MX) v.mx = __reduce_max_sync(0xffffffffu, v.mx);
     if (ncta == 1) {
       if (lane == 0) cp[0] = v;
@@ -103,10 +106,10 @@ __device__ __forceinline__ unsigned pack_code(int c) {
 }
 constexpr unsigned kBLowX = 16, kBLowY = 32, kBHighX = 64, kBHighY = 128;
 
-template <int K, bool A0>
-__global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterScene* tab, CgClusterScene one) {
+template <int K, int T, bool A0>
+__global__ void __launch_bounds__(T, 1) k_cg_cluster(const CgClusterScene* tab, CgClusterScene one) {
   extern __shared__ __align__(16) float smem[];
-  __shared__ Share s_wp[kCcWarps];
+  __shared__ Share s_wp[T / 32];
   __shared__ Share s_cp[2][kCcMaxCta];
   constexpr bool kRegs = K <= 16;  // search and pressure values in registers
   cg::cluster_group cl = cg::this_cluster();
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
   for (int q = 0; q < (K + 3) / 4; q++) code[q] = 0;
 #pragma unroll
   for (int q = 0; q < K; q++) {
-    const int e = tid + kCcThreads * q;
+    const int e = tid + T * q;
     r[q] = 0.f;
     t[q] = 0.f;
     if (kRegs) sv[q] = p[q] = 0.f;
@@ -152,7 +155,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
       acc.add(v * v);
     }
   }
-  for (int x = tid; x < nx; x += kCcThreads) {
+  for (int x = tid; x < nx; x += T) {
     smem[x] = low ? S.rhs[base - nx + x] : 0.f;
     if (R > 0) s_s[cells + x] = high ? S.rhs[base + cells + x] : 0.f;
     s_rlo[x] = s_rhi[x] = 0.f;
@@ -163,7 +166,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
   else cl.sync();
   float* const rloUp = high ? cl.map_shared_rank(s_rlo, rank + 1) : s_rlo;   // where the next strip keeps my last row
   float* const rhiDown = low ? cl.map_shared_rank(s_rhi, rank - 1) : s_rhi;  // where the previous one keeps my first
-  cluster_sum<false>(cl, ncta, s_wp, s_cp[1], acc, sum, mx);
+  cluster_sum<T, false>(cl, ncta, s_wp, s_cp[1], acc, sum, mx);
   float sigma = sum.rounded();
   float alpha = 0.f, beta = 0.f, dp = 0.f, res = g->resNorm;
   int it = 0, done = 0, status = 0;
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
     acc = FSum();
 #pragma unroll
     for (int q = 0; q < K; q++) {
-      const int e = tid + kCcThreads * q;
+      const int e = tid + T * q;
       if (e < cells) {
         const unsigned c = code[q >> 2] >> (8 * (q & 3));
         const float xc = kRegs ? sv[q] : s_s[e];
@@ -187,7 +190,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
         acc.add(v * xc);
       }
     }
-    cluster_sum<false>(cl, ncta, s_wp, s_cp[0], acc, sum, mx);
+    cluster_sum<T, false>(cl, ncta, s_wp, s_cp[0], acc, sum, mx);
     dp = sum.rounded();
     alpha = fabsf(dp) > 0.f ? sigma / dp : 0.f;
     const float na = -alpha;
@@ -196,7 +199,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
     mx = __float_as_int(-1.f);
 #pragma unroll
     for (int q = 0; q < K; q++) {
-      const int e = tid + kCcThreads * q;
+      const int e = tid + T * q;
       if (e < cells) {
         if (kRegs) p[q] = p[q] + alpha * sv[q];
         else s_p[e] = s_p[e] + alpha * s_s[e];
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
         if (rv == rv) mx = max(mx, __float_as_int(fabsf(rv)));  // NaN takes no part, as in fmaxf
       }
     }
-    cluster_sum<true>(cl, ncta, s_wp, s_cp[1], acc, sum, mx);
+    cluster_sum<T, true>(cl, ncta, s_wp, s_cp[1], acc, sum, mx);
     it++;
     res = __int_as_float(mx);
     if (res < 0.f) res = S.nanNorm;
@@ -228,14 +231,14 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
     // s = r + beta s (UpdateSearchVec), the halo rows with their owners' values
 #pragma unroll
     for (int q = 0; q < K; q++) {
-      const int e = tid + kCcThreads * q;
+      const int e = tid + T * q;
       if (e < cells) {
         const float v = r[q] + beta * (kRegs ? sv[q] : s_s[e]);
         if (kRegs) sv[q] = v;
         s_s[e] = v;
       }
     }
-    for (int x = tid; x < nx; x += kCcThreads) {
+    for (int x = tid; x < nx; x += T) {
       if (low) smem[x] = s_rlo[x] + beta * smem[x];
       if (high) s_s[cells + x] = s_rhi[x] + beta * s_s[cells + x];
     }
@@ -243,7 +246,7 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
   }
 #pragma unroll
   for (int q = 0; q < K; q++) {
-    const int e = tid + kCcThreads * q;
+    const int e = tid + T * q;
     if (e < cells) S.p[base + e] = kRegs ? p[q] : s_p[e];
   }
   if (rank == 0 && tid == 0) {
@@ -260,17 +263,20 @@ __global__ void __launch_bounds__(kCcThreads, 1) k_cg_cluster(const CgClusterSce
 
 typedef void (*CgClusterKernel)(const CgClusterScene*, CgClusterScene);
 template <bool A0>
-CgClusterKernel kernel_of(int k) {
+CgClusterKernel kernel_of(int threads, int k) {
+  if (threads == kCcSmall) switch (k) {
+    case 1: return k_cg_cluster<1, kCcSmall, A0>;
+    case 2: return k_cg_cluster<2, kCcSmall, A0>;
+    case 4: return k_cg_cluster<4, kCcSmall, A0>;
+    default: return k_cg_cluster<8, kCcSmall, A0>;
+  }
   switch (k) {
-    case 1: return k_cg_cluster<1, A0>;
-    case 2: return k_cg_cluster<2, A0>;
-    case 4: return k_cg_cluster<4, A0>;
-    case 8: return k_cg_cluster<8, A0>;
-    case 16: return k_cg_cluster<16, A0>;
-    default: return k_cg_cluster<32, A0>;
+    case 8: return k_cg_cluster<8, kCcThreads, A0>;
+    case 16: return k_cg_cluster<16, kCcThreads, A0>;
+    default: return k_cg_cluster<32, kCcThreads, A0>;
   }
 }
-CgClusterKernel kernel_of(int k, bool a0) { return a0 ? kernel_of<true>(k) : kernel_of<false>(k); }
+CgClusterKernel kernel_of(int threads, int k, bool a0) { return a0 ? kernel_of<true>(threads, k) : kernel_of<false>(threads, k); }
 
 int g_ccMaxCta = 0;
 
@@ -279,14 +285,14 @@ size_t cc_smem(int nx, int rows, int k, bool a0) {
   return sizeof(float) * (4 * (size_t)nx + cap * (1 + (k > 16 ? 1 : 0) + (a0 ? 1 : 0)));
 }
 
-cudaLaunchConfig_t cc_config(int ctas, int scenes, size_t smem, cudaLaunchAttribute* at, cudaStream_t s) {
+cudaLaunchConfig_t cc_config(int ctas, int threads, int scenes, size_t smem, cudaLaunchAttribute* at, cudaStream_t s) {
   at->id = cudaLaunchAttributeClusterDimension;
   at->val.clusterDim.x = ctas;
   at->val.clusterDim.y = 1;
   at->val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(ctas * scenes));
-  cfg.blockDim = dim3(kCcThreads);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = at;
@@ -298,8 +304,8 @@ cudaLaunchConfig_t cc_config(int ctas, int scenes, size_t smem, cudaLaunchAttrib
 
 int cg_cluster_prepare() {
   for (int k = 1; k <= kCcMaxK; k *= 2)
-    for (int a = 0; a < 2; a++) {
-      const CgClusterKernel f = kernel_of(k, a != 0);
+    for (int a = 0; a < 4; a++) {
+      const CgClusterKernel f = kernel_of(a & 2 ? kCcThreads : kCcSmall, k, (a & 1) != 0);
       if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCcMaxSmem) != cudaSuccess ||
           cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         return 1;
@@ -308,26 +314,29 @@ int cg_cluster_prepare() {
   g_ccMaxCta = 0;
   for (int c = kCcMaxCta; c >= 1 && !g_ccMaxCta; c /= 2) {
     cudaLaunchAttribute at[1];
-    const cudaLaunchConfig_t cfg = cc_config(c, 1, kCcMaxSmem, at, nullptr);
+    const cudaLaunchConfig_t cfg = cc_config(c, kCcThreads, 1, kCcMaxSmem, at, nullptr);
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, kernel_of(kCcMaxK, true), &cfg) == cudaSuccess && nc >= 1) g_ccMaxCta = c;
+    if (cudaOccupancyMaxActiveClusters(&nc, kernel_of(kCcThreads, kCcMaxK, true), &cfg) == cudaSuccess && nc >= 1) g_ccMaxCta = c;
   }
   cudaGetLastError();
   return 0;
 }
 
-// Strips of about 2048 cells: at 4 cells per thread an iteration's arithmetic
-// and its two barriers take about as long; the largest scenes take every CTA
-// of the largest cluster and up to 32 cells per thread.
+// Strips of about 2048 cells: an iteration's arithmetic and its two barriers
+// then take about as long.  Up to there 256 threads of 8 cells, whose sums take
+// half the instructions of 512 of 4 (steps of 64 x 64, 96 x 128 and 150 x 170
+// cells 0.55, 1.06 and 1.48 ms instead of 0.59, 1.17 and 1.61); the largest scenes take every CTA of the
+// largest cluster and up to 32 cells per thread.
 bool cg_cluster_plan(const Dims& d, bool a0, CgClusterPlan* pl) {
   if (d.is3d || !g_ccMaxCta) return false;
   int c = 1;
   auto rows = [&](int ctas) { return (d.ny + ctas - 1) / ctas; };
-  while (c < g_ccMaxCta && (long long)rows(c) * d.nx > 2048) c *= 2;
+  while (c < g_ccMaxCta && (long long)rows(c) * d.nx > kCcStrip) c *= 2;
   const long long strip = (long long)rows(c) * d.nx;
   if (strip > (long long)kCcThreads * kCcMaxK) return false;
-  int k = 1;
-  while ((long long)kCcThreads * k < strip) k *= 2;
+  pl->threads = strip <= kCcStrip ? kCcSmall : kCcThreads;
+  int k = pl->threads == kCcSmall ? 1 : 8;
+  while ((long long)pl->threads * k < strip) k *= 2;
   pl->ctas = c;
   pl->k = k;
   pl->rows = rows(c);
@@ -339,8 +348,8 @@ cudaError_t launch_cg_cluster(const CgClusterPlan& pl, const CgClusterScene* tab
                               bool a0, cudaStream_t s) {
   count_launch();
   cudaLaunchAttribute at[1];
-  const cudaLaunchConfig_t cfg = cc_config(pl.ctas, scenes, pl.smem, at, s);
-  return cudaLaunchKernelEx(&cfg, kernel_of(pl.k, a0), tab, one);
+  const cudaLaunchConfig_t cfg = cc_config(pl.ctas, pl.threads, scenes, pl.smem, at, s);
+  return cudaLaunchKernelEx(&cfg, kernel_of(pl.threads, pl.k, a0), tab, one);
 }
 
 }  // namespace mgpu

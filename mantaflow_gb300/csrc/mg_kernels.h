@@ -275,7 +275,7 @@ struct CgClusterScene {
   CgScalars* sc;
 };
 struct CgClusterPlan {
-  int ctas, k, rows;  // CTAs of the cluster, cells per thread, rows per CTA
+  int ctas, threads, k, rows;  // CTAs of the cluster, threads of a CTA, cells per thread, rows per CTA
   size_t smem;
 };
 int cg_cluster_prepare();
