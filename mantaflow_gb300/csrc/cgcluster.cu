@@ -18,9 +18,9 @@
 //    each side.
 //  * An iteration has two cluster-wide sums: (A s, s), and (r, r) with
 //    max|r|.  A CTA's share goes into a slot of its own in the shared memory
-//    of every CTA before a cluster barrier, and every warp then adds the
-//    slots in rank order, so all CTAs hold the same bits and take the same
-//    branches without a second exchange.
+//    of every CTA before a cluster barrier, and each then adds the slots in
+//    rank order, so all CTAs hold the same bits and take the same branches
+//    without a second exchange.
 //  * The neighbours' edge rows of the residual travel with the second sum;
 //    each CTA forms its halo rows of the search vector from them with the
 //    owner's own arithmetic.  That saves a third barrier per iteration.
@@ -28,7 +28,7 @@
 // Every cell's float operations are those of the grid kernels (pressure.cu),
 // a thread sums its cells' products as theirs do, and the threads' sums are
 // added up with more bits than their doubles have.  (Three floats to a sum cost
-// instructions: with two, 48 bits, a 96 x 128 step takes 0.94 ms instead of 1.04.
+// instructions: with two, 48 bits, a 96 x 128 step takes 0.94 ms instead of 1.03.
 // In double it is more: the FP64 pipe does two lanes a cycle.)
 // The split depends on the scene's size alone, so a scene computes the same
 // alone and in any batch.
@@ -54,10 +54,19 @@ constexpr int kCcMaxK = 32;
 static_assert(kCcStrip <= 8 * kCcSmall && kCcStrip >= 4 * kCcThreads, "the cells per thread that kernel_of has");
 constexpr size_t kCcMaxSmem = 220 * 1024;
 
-// a CTA's share of a cluster sum: the sum and the largest |r| (as the float's
+// a warp's share of a cluster sum: the sum and the largest |r| (as the float's
 // bits; negative: none)
 struct __align__(16) Share {
   TSum s;
+  int mx;
+};
+template <int T>
+struct SumSmem {
+  static constexpr int kAdd = T / 128;  // warps that add up
+  float2 part[T];
+  int wmx[T / 32];
+  Share share[2][kCcMaxCta * kAdd];  // of every CTA's adding warps, by sum
+  float sum;
   int mx;
 };
 
@@ -65,36 +74,62 @@ __device__ __forceinline__ TSum across(const TSum& a, int o) {
   return TSum{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o), __shfl_xor_sync(0xffffffffu, a.m, o)};
 }
 
-// the sum of the threads' sums and the maximum of mx over the cluster, the same
-// bits in every thread of every CTA
+// The sum of the threads' sums over the cluster, rounded to float, and the
+// maximum of mx, the same bits in every thread of every CTA.  Sums in three
+// floats take instructions, so a quarter of a CTA's warps add up four threads
+// each.  The cluster's shares are added up by every warp of a small CTA, by one
+// of a large one (the other way about, steps of 96 x 128 and 150 x 170 cells are
+// 3 % slower, those of 200 x 200 to 400 x 400 cells 5 %).
 template <int T, bool MX>
-__device__ __forceinline__ void cluster_sum(cg::cluster_group& cl, int ncta, Share* wp, Share* cp, const FSum& own,
-                                            TSum& sum, int& mx) {
-  constexpr int kWarps = T / 32;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  TSum t{own.h, own.l, 0.f};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t.add(across(t, o));
-  if (MX) mx = __reduce_max_sync(0xffffffffu, mx);
-  if (lane == 0) wp[wid] = Share{t, mx};
+__device__ __forceinline__ float cluster_sum(cg::cluster_group& cl, int ncta, SumSmem<T>& sm, int which, const FSum& own, int& mx) {
+  constexpr int kAdd = SumSmem<T>::kAdd;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  sm.part[t] = make_float2(own.h, own.l);
+  if (MX) {
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) sm.wmx[wid] = mx;
+  }
   __syncthreads();
-  if (wid == 0) {
-    Share v = wp[lane & (kWarps - 1)];
+  if (wid < kAdd) {
+    Share v{TSum{}, -1};
 #pragma unroll
-    for (int o = kWarps / 2; o > 0; o >>= 1) v.s.add(across(v.s, o));
-    if (MX) v.mx = __reduce_max_sync(0xffffffffu, v.mx);
+    for (int q = 0; q < 4; q++) {
+      const float2 p = sm.part[t + q * (T / 4)];
+      if (q == 0) v.s = TSum{p.x, p.y, 0.f};
+      else v.s.add(TSum{p.x, p.y, 0.f});
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v.s.add(across(v.s, o));
+    if (MX) v.mx = __reduce_max_sync(0xffffffffu, sm.wmx[lane & (T / 32 - 1)]);
     if (ncta == 1) {
-      if (lane == 0) cp[0] = v;
+      if (lane == 0) sm.share[which][wid] = v;
     } else if (lane < ncta) {
-      *cl.map_shared_rank(cp + cl.block_rank(), lane) = v;
+      *cl.map_shared_rank(&sm.share[which][cl.block_rank() * kAdd + wid], lane) = v;
     }
   }
   if (ncta == 1) __syncthreads();
   else cl.sync();
-  const Share v = cp[lane & (ncta - 1)];  // a power of two
-  sum = v.s;
-  for (int o = ncta / 2; o > 0; o >>= 1) sum.add(across(sum, o));
-  if (MX) mx = __reduce_max_sync(0xffffffffu, v.mx);
+  const int n = ncta * kAdd, lanes = min(n, 32);  // powers of two
+  float sum = 0.f;
+  if (T == kCcSmall || wid == 0) {
+    Share v = sm.share[which][lane & (lanes - 1)];
+    if (n > 32) {
+      const Share u = sm.share[which][lane + 32];
+      v.s.add(u.s);
+      v.mx = max(v.mx, u.mx);
+    }
+    for (int o = lanes / 2; o > 0; o >>= 1) v.s.add(across(v.s, o));
+    if (MX) mx = __reduce_max_sync(0xffffffffu, v.mx);
+    sum = v.s.rounded();
+  }
+  if (T == kCcSmall) return sum;
+  if (threadIdx.x == 0) {
+    sm.sum = sum;
+    sm.mx = mx;
+  }
+  __syncthreads();
+  if (MX) mx = sm.mx;
+  return sm.sum;
 }
 
 // the 2D part of a stencil code in a byte: A0 (bits 0-2), then the links
@@ -109,8 +144,7 @@ constexpr unsigned kBLowX = 16, kBLowY = 32, kBHighX = 64, kBHighY = 128;
 template <int K, int T, bool A0>
 __global__ void __launch_bounds__(T, 1) k_cg_cluster(const CgClusterScene* tab, CgClusterScene one) {
   extern __shared__ __align__(16) float smem[];
-  __shared__ Share s_wp[T / 32];
-  __shared__ Share s_cp[2][kCcMaxCta];
+  __shared__ SumSmem<T> s_sum;
   constexpr bool kRegs = K <= 16;  // search and pressure values in registers
   cg::cluster_group cl = cg::this_cluster();
   const int ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -132,7 +166,6 @@ __global__ void __launch_bounds__(T, 1) k_cg_cluster(const CgClusterScene* tab, 
 
   float r[K], t[K], sv[kRegs ? K : 1], p[kRegs ? K : 1];
   unsigned code[(K + 3) / 4];
-  TSum sum;
   int mx = -1;
   FSum acc;
 #pragma unroll
@@ -160,14 +193,12 @@ __global__ void __launch_bounds__(T, 1) k_cg_cluster(const CgClusterScene* tab, 
     if (R > 0) s_s[cells + x] = high ? S.rhs[base + cells + x] : 0.f;
     s_rlo[x] = s_rhi[x] = 0.f;
   }
-  if (tid < 2 * kCcMaxCta) s_cp[tid / kCcMaxCta][tid % kCcMaxCta] = Share{TSum{}, __float_as_int(-1.f)};
   // no CTA stores into another's shared memory before that one has set it up
   if (ncta == 1) __syncthreads();
   else cl.sync();
   float* const rloUp = high ? cl.map_shared_rank(s_rlo, rank + 1) : s_rlo;   // where the next strip keeps my last row
   float* const rhiDown = low ? cl.map_shared_rank(s_rhi, rank - 1) : s_rhi;  // where the previous one keeps my first
-  cluster_sum<T, false>(cl, ncta, s_wp, s_cp[1], acc, sum, mx);
-  float sigma = sum.rounded();
+  float sigma = cluster_sum<T, false>(cl, ncta, s_sum, 1, acc, mx);
   float alpha = 0.f, beta = 0.f, dp = 0.f, res = g->resNorm;
   int it = 0, done = 0, status = 0;
 
@@ -190,8 +221,7 @@ __global__ void __launch_bounds__(T, 1) k_cg_cluster(const CgClusterScene* tab, 
         acc.add(v * xc);
       }
     }
-    cluster_sum<T, false>(cl, ncta, s_wp, s_cp[0], acc, sum, mx);
-    dp = sum.rounded();
+    dp = cluster_sum<T, false>(cl, ncta, s_sum, 0, acc, mx);
     alpha = fabsf(dp) > 0.f ? sigma / dp : 0.f;
     const float na = -alpha;
     // p += alpha s, r -= alpha A s; (r, r) and max|r|
@@ -211,7 +241,7 @@ __global__ void __launch_bounds__(T, 1) k_cg_cluster(const CgClusterScene* tab, 
         if (rv == rv) mx = max(mx, __float_as_int(fabsf(rv)));  // NaN takes no part, as in fmaxf
       }
     }
-    cluster_sum<T, true>(cl, ncta, s_wp, s_cp[1], acc, sum, mx);
+    const float sigmaNew = cluster_sum<T, true>(cl, ncta, s_sum, 1, acc, mx);
     it++;
     res = __int_as_float(mx);
     if (res < 0.f) res = S.nanNorm;
@@ -220,7 +250,6 @@ __global__ void __launch_bounds__(T, 1) k_cg_cluster(const CgClusterScene* tab, 
       done = 1;
       break;
     }
-    const float sigmaNew = sum.rounded();
     beta = sigmaNew / sigma;
     sigma = sigmaNew;
     if (!(res < 1e35f)) {
