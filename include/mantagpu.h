@@ -397,8 +397,8 @@ int mg_batch_create(int count, const int* sizes, const float* gravity, const uns
 int mg_batch_destroy(mg_batch b);
 /* solvePressure's cgAccuracy (1e-3) and cgMaxIterFac (1.5) */
 int mg_batch_set_solver(mg_batch b, float cgAccuracy, float cgMaxIterFac);
-/* MG_PC_MIC (the default): 3D scenes precondition with MIC(0), whose
- * dataflow sweeps run over the tiles of all 3D scenes in one launch; 2D
+/* MG_PC_MIC (the default): 3D scenes precondition with MIC(0), one launch
+ * per sweep over all of them (scenes too wide for a cluster: another); 2D
  * scenes run GridCg without a preconditioner, as the reference does in 2D.
  * MG_PC_NONE: no scene is preconditioned. */
 int mg_batch_set_preconditioner(mg_batch b, int preconditioner);

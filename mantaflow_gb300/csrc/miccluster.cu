@@ -35,12 +35,16 @@
 // waits only for clusters that run or have finished.  The backward sweep runs
 // the same levels downward.
 //
-// A level takes about 115 cycles (the arithmetic's chain is 63), a chunk's
-// hand-over 80, and a warp runs about 900 cycles behind the one that feeds it.
-// Forward / backward sweep: 22 / 28 us at 64^3, 47 / 56 us at 128^3.  Whole
-// solves against the tile sweeps of micflow.cu: 64^3 smoke (50 iterations)
-// 9.2 -> 4.0 ms, 128^3 dam break (53) 21.3 -> 8.0 ms.  Grids with more than
-// 256 rows or more than about 400 cells along x do not fit and keep the tiles.
+// Eight levels take 1000 cycles forward and 1070 back where their words are
+// there, 1200 and 1300 where a pair of levels waits for one (four chunks in
+// five); between chunks pass 280 and 410, most of it the wait for the copy's
+// barrier.  A bundle runs 1900 to 2100 cycles behind the one that feeds it (seven
+// levels of skew and the words' way), 5600 to 6900 where that is in another
+// cluster.  At 128^3: 18 chunks 12 us, 27 hops 26 us and 3 between clusters 8.5 us
+// make the 46 us of a forward sweep; a backward one takes 52, at 64^3 they take 21
+// and 22.  Whole solves against the tile sweeps of micflow.cu: 64^3 smoke (50
+// iterations) 9.3 -> 3.5 ms, 128^3 dam break (53) 21.3 -> 7.7 ms.  Grids with more
+// than 256 rows or more than about 400 cells along x do not fit and keep the tiles.
 #include <cooperative_groups.h>
 
 #include <algorithm>

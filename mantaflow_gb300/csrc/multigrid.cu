@@ -623,10 +623,10 @@ __global__ void __launch_bounds__(256, 3) k_mg_residual(Lev L, int S, const CgSc
 
 // The same passes on a level with a stencil dictionary.  A level of 590 000
 // slots or fewer is bound by latency: a launch, an id, its tuple, the values.
-// With the ids fetched while the pass before ends and all values loaded at
-// once, a solve at 161 x 199 x 143 takes 3.24 instead of 3.38 ms, one at 112^3
-// 1.74 instead of 1.89, a smoke step at 256^3 7.26 instead of 7.58.  (The
-// transfers between levels and the cluster launch gain nothing from it.)
+// The ids are fetched while the pass before ends and all values loaded at
+// once, which is worth 4 % of a solve at 161 x 199 x 143 or a smoke step at 256^3
+// and 8 % of a solve at 112^3.  (The transfers between levels and the cluster
+// launch gain nothing from it.)
 template <bool IS3D>
 __global__ void __launch_bounds__(256, 4) k_mg_smooth_dict(Lev L, int ox, int oy, int oz, const CgScalars* sc) {
   constexpr int S = IS3D ? 14 : 5;
@@ -1234,9 +1234,10 @@ __device__ __forceinline__ void coarse_dots(CoarseSmem& sm, int warps, int slot,
 // Each iteration is a chain of two dot products and three barriers, so what
 // counts is latency: spread over the cluster, with two cluster barriers, it
 // took 4.6 us for 288 vertices and 50 iterations to a solve (240 of the 345 us
-// of a launch); here 2 us (3 us for 729 vertices).  A thread has K vertices, t and t + threads, in an
-// order with the longest axis last, so that a neighbour is a fixed, short step
-// away in the search vector.  Absent neighbours have coefficient zero.
+// of a launch); here 2.2 us, for 512 vertices 2.7 and for 729, two to a thread,
+// 4.0.  A thread has K vertices, t and t + threads, in an order with the longest
+// axis last, so that a neighbour is a fixed, short step away in the search vector.
+// Absent neighbours have coefficient zero.
 // Vectors, dot products and scalars are double-float pairs on the FP32 pipe
 // (the stencil product is a compensated sum of exact float products); the
 // iterates follow an IEEE-double CG to ~1e-14 relative.
@@ -1505,8 +1506,7 @@ struct TailVertex {
 // could have had before: while a colour's results travel to the other CTAs
 // (a barrier of the cluster takes 1100 cycles by itself), the next colour's
 // stencils are fetched, and every pass issues all its loads before the first
-// use: 2.1 us a pass, before 3.5.  With the coarsest level's solver this took a
-// launch from 400 to 205 us, a solve at 161 x 199 x 143 from 4.51 to 3.38 ms.
+// use: 2.1 us a pass, where loads waited for in turn took 3.5.
 template <bool IS3D>
 __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const Lev* __restrict__ levs, int first, int last, int S,
                                                              float accuracy, const CgScalars* sc) {

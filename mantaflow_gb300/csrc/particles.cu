@@ -444,13 +444,13 @@ __global__ void __launch_bounds__(256) k_p2g_gather(Dims d, int comp, SortedPart
 // shared memory, about 20 instructions for a particle's 24 faces.  The weights
 // come from a batch of 32 particles whose lanes prepared one each.
 //
-// At 128^3 with 16.0 M particles mapPartsToMAC took 5.5 ms with a radix sort
-// and eight-way merges per component (3.2 ms of it in the merges, about 100
-// instructions per contribution); now 1.5 ms: lists 0.11 + 0.16, sort 0.38,
-// splat 0.9.  The splat is bound by shared memory, ten wavefronts per particle
-// of a tile (95 % of the rate), the sort by its instructions.  With particles
-// in random order the lists' atomics and the loads by index weigh more: 10.8 M
-// in 108 x 125 x 100 take 3.3 ms (before: 5.8), in seeding order 0.95 (3.8).
+// At 128^3 with 16.0 M particles mapPartsToMAC takes 1.45 ms, lists 0.11 + 0.16,
+// sort 0.38, splat 0.9, where a radix sort and eight-way merges per component took
+// 5.5 (3.2 of it in the merges, about 100 instructions per contribution).  The
+// splat is bound by shared memory, ten wavefronts per particle of a tile (96 % of
+// the rate), the sort by its instructions.  With particles in random order the
+// lists' atomics and the loads by index weigh more: 10.8 M in 108 x 125 x 100 take
+// 3.3 ms, in seeding order 0.95 (sorted and merged: 5.8 and 3.8).
 template <int X, int Y, int Z>
 struct TileShape {
   static constexpr int x = X, y = Y, z = Z;
@@ -1011,9 +1011,9 @@ SortedParts sorted_copy(mg_particles p, const unsigned* sorted, const PartView& 
 // Whether mapPartsToMAC takes the tile lists: in 3D, with room for every
 // particle in the eight tiles that it can reach (eight of the scratch's ten
 // words), and memory for the tiles' tables.  The larger tiles from a million
-// cells on: with the small ones 128^3 takes 2.31 instead of 1.58 ms.  Below, a
-// large tile's list is too long a serial walk for the few tiles there are
-// (75 x 62 x 90: 0.52 instead of 0.45 ms with the transfer back).
+// cells on: with the small ones a call by itself at 128^3 takes 2.31 instead of
+// 1.58 ms.  Below, a large tile's list is too long a serial walk for the few tiles
+// there are (75 x 62 x 90: 0.52 instead of 0.45 ms with the transfer back).
 bool tile_lists(mg_particles p) {
   if (p->tileMem) return true;
   Tiles& s = p->tiles;
