@@ -156,7 +156,7 @@ __device__ __forceinline__ void maccormack_real_cell(const Dims& d, const int* _
     pz = (k + 0.5f) - vc.z * (-dt);
   } else {
     const float p0x = i + 0.5f, p0y = j + 0.5f, p0z = k + 0.5f;
-    const V3 vi = interp_mac(d, vel, p0x - (vc.x * (-dt)) * 0.5f, p0y - (vc.y * (-dt)) * 0.5f, p0z - (vc.z * (-dt)) * 0.5f);
+    const V3 vi = interp_mac<false, true>(d, vel, p0x - (vc.x * (-dt)) * 0.5f, p0y - (vc.y * (-dt)) * 0.5f, p0z - (vc.z * (-dt)) * 0.5f);
     px = p0x - vi.x * (-dt);
     py = p0y - vi.y * (-dt);
     pz = p0z - vi.z * (-dt);
@@ -165,7 +165,7 @@ __device__ __forceinline__ void maccormack_real_cell(const Dims& d, const int* _
 #pragma unroll
   for (int c = 0; c < CH; c++) {
     const float* f = fwd + c * d.n;
-    const float bwd = kOrderSpace == 1 ? interp(d, f, px, py, pz) : interp_cubic<CH == 3>(d, f, px, py, pz);
+    const float bwd = kOrderSpace == 1 ? interp<true>(d, f, px, py, pz) : interp_cubic<CH == 3>(d, f, px, py, pz);
     fw[c] = __ldg(f + idx);
     float v = fw[c];
     if (fluid) {
@@ -210,10 +210,10 @@ __global__ void __launch_bounds__(256, 6) k_maccormack_cell(Dims d, const int* _
 // trilinear on the component's plane; orderSpace 2 is interpolCubicMAC's
 // component (interpolHigh.h:171-178), the Vec3 Catmull-Rom sample half a
 // cell further along the component's axis (0 for z in 2D).
-template <int kOS>
+template <int kOS, bool kClamp = false>
 __device__ __forceinline__ float sample_mac_comp(const Dims& d, const float* __restrict__ plane, int c, float x, float y,
                                                  float z) {
-  if (kOS == 1) return interp(d, plane, x, y, z);
+  if (kOS == 1) return interp<kClamp>(d, plane, x, y, z);
   if (c == 0) return interp_cubic<true>(d, plane, x + 0.5f, y, z);
   if (c == 1) return interp_cubic<true>(d, plane, x, y + 0.5f, z);
   if (!d.is3d) return 0.f;
@@ -221,16 +221,16 @@ __device__ __forceinline__ float sample_mac_comp(const Dims& d, const float* __r
 }
 
 // SemiLagrangeMAC (advection.cpp:44-77), src sampled per component.
-template <int kTrace, int kOS>
+template <int kTrace, int kOS, bool kClamp = false>
 __device__ __forceinline__ void sl_mac_cell(const Dims& d, CMac vel, CMac src, int i, int j, int k, float dt, float* out) {
   const long long idx = ix(d, i, j, k);
   if (kTrace == 1) {
     const V3 ax = mac_at_x(d, vel, idx);
-    out[0] = sample_mac_comp<kOS>(d, src.u, 0, (i + 0.5f) - ax.x * dt, (j + 0.5f) - ax.y * dt, (k + 0.5f) - ax.z * dt);
+    out[0] = sample_mac_comp<kOS, kClamp>(d, src.u, 0, (i + 0.5f) - ax.x * dt, (j + 0.5f) - ax.y * dt, (k + 0.5f) - ax.z * dt);
     const V3 ay = mac_at_y(d, vel, idx);
-    out[1] = sample_mac_comp<kOS>(d, src.v, 1, (i + 0.5f) - ay.x * dt, (j + 0.5f) - ay.y * dt, (k + 0.5f) - ay.z * dt);
+    out[1] = sample_mac_comp<kOS, kClamp>(d, src.v, 1, (i + 0.5f) - ay.x * dt, (j + 0.5f) - ay.y * dt, (k + 0.5f) - ay.z * dt);
     const V3 az = mac_at_z(d, vel, idx);
-    out[2] = sample_mac_comp<kOS>(d, src.w, 2, (i + 0.5f) - az.x * dt, (j + 0.5f) - az.y * dt, (k + 0.5f) - az.z * dt);
+    out[2] = sample_mac_comp<kOS, kClamp>(d, src.w, 2, (i + 0.5f) - az.x * dt, (j + 0.5f) - az.y * dt, (k + 0.5f) - az.z * dt);
   } else {
     // the midpoint trace samples src, as the reference does
     const float p0x = i + 0.5f, p0y = j + 0.5f, p0z = k + 0.5f;
@@ -240,8 +240,8 @@ __device__ __forceinline__ void sl_mac_cell(const Dims& d, CMac vel, CMac src, i
       const float qy = c == 1 ? (float)j : j + 0.5f;
       const float qz = c == 2 ? (float)k : k + 0.5f;
       const V3 a = c == 0 ? mac_at_x(d, src, idx) : (c == 1 ? mac_at_y(d, src, idx) : mac_at_z(d, src, idx));
-      const V3 vi = interp_mac(d, src, qx - (a.x * dt) * 0.5f, qy - (a.y * dt) * 0.5f, qz - (a.z * dt) * 0.5f);
-      out[c] = sample_mac_comp<kOS>(d, src.c(c), c, p0x - vi.x * dt, p0y - vi.y * dt, p0z - vi.z * dt);
+      const V3 vi = interp_mac<false, kClamp>(d, src, qx - (a.x * dt) * 0.5f, qy - (a.y * dt) * 0.5f, qz - (a.z * dt) * 0.5f);
+      out[c] = sample_mac_comp<kOS, kClamp>(d, src.c(c), c, p0x - vi.x * dt, p0y - vi.y * dt, p0z - vi.z * dt);
     }
   }
 }
@@ -327,11 +327,11 @@ __device__ __forceinline__ void maccormack_mac_cell(const Dims& d, const int* __
     if (kTrace == 1) {
       // SemiLagrangeMAC(fwd, -dt), as sl_mac_cell<1> forms it
       const float mdt = -dt;
-      bwd[0] = sample_mac_comp<kOS>(d, fwd.u, 0, (i + 0.5f) - ax.x * mdt, (j + 0.5f) - ax.y * mdt, (k + 0.5f) - ax.z * mdt);
-      bwd[1] = sample_mac_comp<kOS>(d, fwd.v, 1, (i + 0.5f) - ay.x * mdt, (j + 0.5f) - ay.y * mdt, (k + 0.5f) - ay.z * mdt);
-      bwd[2] = sample_mac_comp<kOS>(d, fwd.w, 2, (i + 0.5f) - az.x * mdt, (j + 0.5f) - az.y * mdt, (k + 0.5f) - az.z * mdt);
+      bwd[0] = sample_mac_comp<kOS, true>(d, fwd.u, 0, (i + 0.5f) - ax.x * mdt, (j + 0.5f) - ax.y * mdt, (k + 0.5f) - ax.z * mdt);
+      bwd[1] = sample_mac_comp<kOS, true>(d, fwd.v, 1, (i + 0.5f) - ay.x * mdt, (j + 0.5f) - ay.y * mdt, (k + 0.5f) - ay.z * mdt);
+      bwd[2] = sample_mac_comp<kOS, true>(d, fwd.w, 2, (i + 0.5f) - az.x * mdt, (j + 0.5f) - az.y * mdt, (k + 0.5f) - az.z * mdt);
     } else {
-      sl_mac_cell<kTrace, kOS>(d, vel, fwd, i, j, k, -dt, bwd);
+      sl_mac_cell<kTrace, kOS, true>(d, vel, fwd, i, j, k, -dt, bwd);
     }
   }
   float fw[3], val[3];

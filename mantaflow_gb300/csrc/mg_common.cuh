@@ -103,12 +103,10 @@ struct Wts {
   float s0, s1, t0, t1, f0, f1;
 };
 
-// One axis: the position clamped to [0, last] gives the reference's clamped
-// index and weights (at the upper end min(last, last - 1) and weight 1) without
-// a branch; min and max that pass on a NaN, whose weights are NaN there too.
-// With this and clamps of one instruction a value, MacCormack advection of a
-// velocity at 256^3 takes 603 us instead of 735.
-__device__ __forceinline__ void build_axis(float p, float last, int lastIndex, int& i, float& w0, float& w1) {
+// One axis without a branch: the position clamped to [0, last] gives the
+// reference's clamped index and weights (at the upper end min(last, last - 1) and
+// weight 1); min and max that pass on a NaN, whose weights are NaN there too.
+__device__ __forceinline__ void clamp_axis(float p, float last, int lastIndex, int& i, float& w0, float& w1) {
   float c;
   asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(c) : "f"(p));
   asm("min.NaN.f32 %0, %1, %2;" : "=f"(c) : "f"(c), "f"(last));
@@ -116,26 +114,50 @@ __device__ __forceinline__ void build_axis(float p, float last, int lastIndex, i
   w1 = c - (float)i;
   w0 = 1.f - w1;
 }
-template <bool kShift>
+// kClamp: by clamp_axis, for the MacCormack passes, which instructions bound
+// (with clamps of one instruction a value, a velocity at 256^3 takes 603 us instead
+// of 735).  The passes that wait for their gathers keep the selections, whose index
+// is there earlier and takes fewer registers: first-order advection of a Vec3 at
+// 200^3 takes 103 us with them and 133 without, mapMACToParts of 16 M particles in
+// order 181 and 197, first-order advection of a velocity at 32^3 27.5 and 28.8.
+template <bool kShift, bool kClamp = false>
 __device__ __forceinline__ Wts build_index(const Dims& d, float x, float y, float z) {
   Wts w;
-  build_axis(kShift ? x : x - 0.5f, (float)(d.nx - 1), d.nx - 2, w.xi, w.s0, w.s1);
-  build_axis(kShift ? y : y - 0.5f, (float)(d.ny - 1), d.ny - 2, w.yi, w.t0, w.t1);
+  const float px = kShift ? x : x - 0.5f;
+  const float py = kShift ? y : y - 0.5f;
   const float pz = kShift ? z : z - 0.5f;
+  if (kClamp) {
+    clamp_axis(px, (float)(d.nx - 1), d.nx - 2, w.xi, w.s0, w.s1);
+    clamp_axis(py, (float)(d.ny - 1), d.ny - 2, w.yi, w.t0, w.t1);
+    if (d.nz > 1) {
+      clamp_axis(pz, (float)(d.nz - 1), d.nz - 2, w.zi, w.f0, w.f1);
+    } else {  // no clamp at the upper end
+      w.zi = (int)pz;
+      w.f1 = pz - (float)w.zi;
+      w.f0 = 1.f - w.f1;
+      if (pz < 0.f) { w.zi = 0; w.f0 = 1.f; w.f1 = 0.f; }
+    }
+    return w;
+  }
+  w.xi = (int)px; w.yi = (int)py; w.zi = (int)pz;
+  w.s1 = px - (float)w.xi; w.s0 = 1.f - w.s1;
+  w.t1 = py - (float)w.yi; w.t0 = 1.f - w.t1;
+  w.f1 = pz - (float)w.zi; w.f0 = 1.f - w.f1;
+  if (px < 0.f) { w.xi = 0; w.s0 = 1.f; w.s1 = 0.f; }
+  if (py < 0.f) { w.yi = 0; w.t0 = 1.f; w.t1 = 0.f; }
+  if (pz < 0.f) { w.zi = 0; w.f0 = 1.f; w.f1 = 0.f; }
+  if (w.xi >= d.nx - 1) { w.xi = d.nx - 2; w.s0 = 0.f; w.s1 = 1.f; }
+  if (w.yi >= d.ny - 1) { w.yi = d.ny - 2; w.t0 = 0.f; w.t1 = 1.f; }
   if (d.nz > 1) {
-    build_axis(pz, (float)(d.nz - 1), d.nz - 2, w.zi, w.f0, w.f1);
-  } else {  // no clamp at the upper end
-    w.zi = (int)pz;
-    w.f1 = pz - (float)w.zi;
-    w.f0 = 1.f - w.f1;
-    if (pz < 0.f) { w.zi = 0; w.f0 = 1.f; w.f1 = 0.f; }
+    if (w.zi >= d.nz - 1) { w.zi = d.nz - 2; w.f0 = 0.f; w.f1 = 1.f; }
   }
   return w;
 }
 
 // interpol<T> for one float plane (util/interpol.h:68-78)
+template <bool kClamp = false>
 __device__ __forceinline__ float interp(const Dims& d, const float* __restrict__ a, float x, float y, float z) {
-  const Wts w = build_index<false>(d, x, y, z);
+  const Wts w = build_index<false, kClamp>(d, x, y, z);
   const int X = 1, Y = (int)d.sy, Z = (int)d.sz;
   const int b = w.xi + Y * w.yi + Z * w.zi;
   const float* p = a + b;
@@ -148,10 +170,10 @@ __device__ __forceinline__ float interp(const Dims& d, const float* __restrict__
 // kSlab: in 2D, read the z = 0 slab whatever z is (for arbitrary particle
 // positions; the reference's 2D particles stay in 0 <= z < 1, where this
 // changes nothing)
-template <bool kSlab = false>
+template <bool kSlab = false, bool kClamp = false>
 __device__ __forceinline__ V3 interp_mac(const Dims& d, CMac m, float x, float y, float z) {
-  Wts w = build_index<false>(d, x, y, z);
-  Wts s = build_index<true>(d, x, y, z);
+  Wts w = build_index<false, kClamp>(d, x, y, z);
+  Wts s = build_index<true, kClamp>(d, x, y, z);
   if (kSlab && !d.is3d) w.zi = s.zi = 0;
   const int X = 1, Y = (int)d.sy, Z = (int)d.sz;
   V3 r;
