@@ -193,6 +193,9 @@ struct Engine {
   size_t clusterCap = 0;
   cudaStream_t side[kSideStreams] = {};
   cudaEvent_t fork = nullptr, join[kSideStreams] = {};
+  // the cluster sweeps beside sweeps by tiles
+  cudaStream_t sweepSide = nullptr;
+  cudaEvent_t sweepFork = nullptr, sweepJoin = nullptr;
   std::vector<BTile> tiles1;
   std::vector<BTile> tilesDam;  // the 32 x 8 tiles of the dam-break scenes
   BTile* dTilesDam = nullptr;
@@ -216,6 +219,7 @@ struct Engine {
     if (stream) cudaStreamSynchronize(stream);
     for (auto st : side)
       if (st) cudaStreamSynchronize(st);
+    if (sweepSide) cudaStreamSynchronize(sweepSide);
     for (auto* m : members) {
       cudaFree(m->mem);
       cudaFree(m->refMem);
@@ -240,6 +244,9 @@ struct Engine {
       if (side[q]) cudaStreamDestroy(side[q]);
     }
     if (fork) cudaEventDestroy(fork);
+    if (sweepFork) cudaEventDestroy(sweepFork);
+    if (sweepJoin) cudaEventDestroy(sweepJoin);
+    if (sweepSide) cudaStreamDestroy(sweepSide);
     if (sweepGraph) cudaGraphExecDestroy(sweepGraph);
     if (ev[0]) cudaEventDestroy(ev[0]);
     if (ev[1]) cudaEventDestroy(ev[1]);
@@ -253,6 +260,9 @@ int engine_init(Engine& e, float dt) {
   CKB(cudaEventCreate(&e.ev[0]));
   CKB(cudaEventCreate(&e.ev[1]));
   CKB(cudaEventCreateWithFlags(&e.fork, cudaEventDisableTiming));
+  CKB(cudaStreamCreateWithFlags(&e.sweepSide, cudaStreamNonBlocking));
+  CKB(cudaEventCreateWithFlags(&e.sweepFork, cudaEventDisableTiming));
+  CKB(cudaEventCreateWithFlags(&e.sweepJoin, cudaEventDisableTiming));
   for (int q = 0; q < kSideStreams; q++) {
     CKB(cudaStreamCreateWithFlags(&e.side[q], cudaStreamNonBlocking));
     CKB(cudaEventCreateWithFlags(&e.join[q], cudaEventDisableTiming));
@@ -843,6 +853,9 @@ int engine_step(Engine& e, mg_batch_stats* stats) {
   mic.error = e.dMicCounter + 1;
   mic.epochDev = (unsigned int*)(e.dMicCounter + 2);
   mic.spinLimit = 200000000LL;
+  mic.side = e.sweepSide;
+  mic.fork = e.sweepFork;
+  mic.join = e.sweepJoin;
   mic.mc = MicClusterLaunch{};
   mic.mc.scenes = e.dMc;
   mic.mc.nscenes = (int)e.hMc.size();

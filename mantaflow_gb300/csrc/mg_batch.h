@@ -114,6 +114,10 @@ struct BatchMic {
   unsigned int* epochDev;  // device word, advanced on the device before each sweep
   long long spinLimit;
   MicClusterLaunch mc;  // the scenes of the cluster sweeps
+  // where both kinds of sweeps run, the cluster sweeps' chain runs on a stream
+  // of its own, forked and joined once per CG sweep
+  cudaStream_t side;
+  cudaEvent_t fork, join;
 };
 // doInit's preconditioner application for the MIC scenes: P, z = M^-1 r,
 // sigma = dot(z, r), search = z

@@ -2046,11 +2046,17 @@ static void pcg_iteration(const BTile* t, int nt, int byTile, const BScene* s, i
   const dim3 b(kBTX, kBTY, 1);
   count_launch();
   k_b_pcg_spmv<R><<<nt, b, 0, st>>>(t, s);
+  const bool both = mic && mic->mc.njobs > 0 && byTile > 0;
+  if (both) {
+    cudaEventRecord(mic->fork, st);
+    cudaStreamWaitEvent(mic->side, mic->fork, 0);
+  }
   if (mic && mic->mc.njobs > 0) {
-    launch_mic_level(mic->mc, kMicAxpy, st);
-    launch_mic_cluster(mic->mc, 1, st);
-    launch_mic_cluster(mic->mc, 2, st);
-    launch_mic_level(mic->mc, kMicUpdate, st);
+    cudaStream_t cs = both ? mic->side : st;
+    launch_mic_level(mic->mc, kMicAxpy, cs);
+    launch_mic_cluster(mic->mc, 1, cs);
+    launch_mic_cluster(mic->mc, 2, cs);
+    launch_mic_level(mic->mc, kMicUpdate, cs);
   }
   if (byTile == 0) return;
   count_launch();
@@ -2065,6 +2071,10 @@ static void pcg_iteration(const BTile* t, int nt, int byTile, const BScene* s, i
   }
   count_launch();
   k_b_pcg_update<R><<<byTile, b, 0, st>>>(t, s);
+  if (both) {
+    cudaEventRecord(mic->join, mic->side);
+    cudaStreamWaitEvent(st, mic->join, 0);
+  }
 }
 void launch_b_pcg_iteration(const BTile* t, int nt, int byTile, const BScene* s, int rows, int* ndone, const BatchMic* mic,
                             cudaStream_t st) {
