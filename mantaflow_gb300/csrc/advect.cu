@@ -18,7 +18,7 @@ namespace mgpu {
 
 // ---------------------------------------------------------------- scalar SL
 // SemiLagrange (advection.cpp:25-41) for CH float planes (1: Real, 3: Vec3)
-template <int CH, int kOrderSpace, int kTrace>
+template <int CH, int kOrderSpace, int kTrace, bool kClamp>
 __device__ __forceinline__ void sl_real_cell(const Dims& d, CMac vel, const float* __restrict__ src, float* __restrict__ dst,
                                                  float dt, int i, int j, int k) {
   const long long idx = ix(d, i, j, k);
@@ -36,7 +36,7 @@ __device__ __forceinline__ void sl_real_cell(const Dims& d, CMac vel, const floa
     pz = (k + 0.5f) - vc.z * dt;
   } else {
     const float p0x = i + 0.5f, p0y = j + 0.5f, p0z = k + 0.5f;
-    const V3 vi = interp_mac(d, vel, p0x - (vc.x * dt) * 0.5f, p0y - (vc.y * dt) * 0.5f, p0z - (vc.z * dt) * 0.5f);
+    const V3 vi = interp_mac<false, kClamp>(d, vel, p0x - (vc.x * dt) * 0.5f, p0y - (vc.y * dt) * 0.5f, p0z - (vc.z * dt) * 0.5f);
     px = p0x - vi.x * dt;
     py = p0y - vi.y * dt;
     pz = p0z - vi.z * dt;
@@ -44,18 +44,18 @@ __device__ __forceinline__ void sl_real_cell(const Dims& d, CMac vel, const floa
 #pragma unroll
   for (int c = 0; c < CH; c++) {
     const float* s = src + c * d.n;
-    dst[c * d.n + idx] = kOrderSpace == 1 ? interp(d, s, px, py, pz) : interp_cubic<CH == 3>(d, s, px, py, pz);
+    dst[c * d.n + idx] = kOrderSpace == 1 ? interp<kClamp>(d, s, px, py, pz) : interp_cubic<CH == 3>(d, s, px, py, pz);
   }
 }
 
-template <int CH, int kOrderSpace, int kTrace>
+template <int CH, int kOrderSpace, int kTrace, bool kClamp>
 __global__ void __launch_bounds__(256) k_sl_cell(Dims d, CMac vel, const float* __restrict__ src, float* __restrict__ dst,
                                                  float dt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
   if (i >= d.nx || j >= d.ny) return;
-  sl_real_cell<CH, kOrderSpace, kTrace>(d, vel, src, dst, dt, i, j, k);
+  sl_real_cell<CH, kOrderSpace, kTrace, kClamp>(d, vel, src, dst, dt, i, j, k);
 }
 
 // doClampComponent (advection.cpp:144-186) over CH planes.  Returns true
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(256, 6) k_maccormack_cell(Dims d, const int* _
 // trilinear on the component's plane; orderSpace 2 is interpolCubicMAC's
 // component (interpolHigh.h:171-178), the Vec3 Catmull-Rom sample half a
 // cell further along the component's axis (0 for z in 2D).
-template <int kOS, bool kClamp = false>
+template <int kOS, bool kClamp>
 __device__ __forceinline__ float sample_mac_comp(const Dims& d, const float* __restrict__ plane, int c, float x, float y,
                                                  float z) {
   if (kOS == 1) return interp<kClamp>(d, plane, x, y, z);
@@ -221,7 +221,7 @@ __device__ __forceinline__ float sample_mac_comp(const Dims& d, const float* __r
 }
 
 // SemiLagrangeMAC (advection.cpp:44-77), src sampled per component.
-template <int kTrace, int kOS, bool kClamp = false>
+template <int kTrace, int kOS, bool kClamp>
 __device__ __forceinline__ void sl_mac_cell(const Dims& d, CMac vel, CMac src, int i, int j, int k, float dt, float* out) {
   const long long idx = ix(d, i, j, k);
   if (kTrace == 1) {
@@ -246,24 +246,24 @@ __device__ __forceinline__ void sl_mac_cell(const Dims& d, CMac vel, CMac src, i
   }
 }
 
-template <int kTrace, int kOS>
+template <int kTrace, int kOS, bool kClamp>
 __device__ __forceinline__ void sl_mac_grid_cell(const Dims& d, CMac vel, CMac src, Mac dst, float dt, int i, int j, int k) {
   const long long idx = ix(d, i, j, k);
   const bool inner = i >= 1 && i < d.nx - 1 && j >= 1 && j < d.ny - 1 && (!d.is3d || (k >= 1 && k < d.nz - 1));
   float out[3] = {0.f, 0.f, 0.f};
-  if (inner) sl_mac_cell<kTrace, kOS>(d, vel, src, i, j, k, dt, out);
+  if (inner) sl_mac_cell<kTrace, kOS, kClamp>(d, vel, src, i, j, k, dt, out);
   dst.u[idx] = out[0];
   dst.v[idx] = out[1];
   dst.w[idx] = out[2];
 }
 
-template <int kTrace, int kOS>
+template <int kTrace, int kOS, bool kClamp>
 __global__ void __launch_bounds__(256) k_sl_mac(Dims d, CMac vel, CMac src, Mac dst, float dt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
   if (i >= d.nx || j >= d.ny) return;
-  sl_mac_grid_cell<kTrace, kOS>(d, vel, src, dst, dt, i, j, k);
+  sl_mac_grid_cell<kTrace, kOS, kClamp>(d, vel, src, dst, dt, i, j, k);
 }
 
 // doClampComponentMAC (advection.cpp:191-235)
@@ -509,8 +509,8 @@ __global__ void __launch_bounds__(256) k_b_advect_fwd(const BTile* __restrict__ 
   BATCH_CELL
   if (sc.kind != 0) return;  // plume scenes only
   const CMac v = bcmac(sc.vel[cur], d.n);
-  sl_real_cell<1, 1, 1>(d, v, sc.dens[cur], sc.fwd + 3 * d.n, sc.dt, i, j, k);
-  sl_mac_grid_cell<1, 1>(d, v, v, bmac(sc.fwd, d.n), sc.dt, i, j, k);
+  sl_real_cell<1, 1, 1, true>(d, v, sc.dens[cur], sc.fwd + 3 * d.n, sc.dt, i, j, k);
+  sl_mac_grid_cell<1, 1, true>(d, v, v, bmac(sc.fwd, d.n), sc.dt, i, j, k);
 }
 // MacCormack correction and clamp of both into the next buffers
 __global__ void __launch_bounds__(256) k_b_advect_mc(const BTile* __restrict__ tiles, const BScene* __restrict__ S, int cur) {
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(256) k_b_outflow_copy(const BTile* __restrict_
 __global__ void __launch_bounds__(256) k_b_dam_advect_phi(const BTile* __restrict__ tiles, const BScene* __restrict__ S,
                                                           int cur) {
   BATCH_CELL
-  sl_real_cell<1, 1, 1>(d, bcmac(sc.vel[cur], d.n), sc.dens[cur], sc.dens[1 - cur], sc.dt, i, j, k);
+  sl_real_cell<1, 1, 1, true>(d, bcmac(sc.vel[cur], d.n), sc.dens[cur], sc.dens[1 - cur], sc.dt, i, j, k);
 }
 // dam break: advectSemiLagrange(vel, order 1) into the next buffer (a closed
 // box has no outflow cells, so applyOutflowBC changes nothing)
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(256) k_b_dam_advect_vel(const BTile* __restric
                                                           int cur) {
   BATCH_CELL
   const CMac v = bcmac(sc.vel[cur], d.n);
-  sl_mac_grid_cell<1, 1>(d, v, v, bmac(sc.vel[1 - cur], d.n), sc.dt, i, j, k);
+  sl_mac_grid_cell<1, 1, true>(d, v, v, bmac(sc.vel[1 - cur], d.n), sc.dt, i, j, k);
 }
 #undef BATCH_CELL
 
@@ -572,10 +572,18 @@ void launch_b_advect_velocity(const BTile* t, int nt, const BScene* s, int cur, 
 // ------------------------------------------------------------- launchers
 static const dim3 kBlk(32, 8, 1);
 
+// Below 64^3 cells a first pass is one wave whose chain counts, and takes the index
+// by selections (a MAC call at 32^3 27.5 us with it, 28.8 without; at 300 x 200 in
+// 2D 22.1 and 22.7; MacCormack of a Real at 48 x 50 x 52 10.4 and 10.9).  They are
+// alike at 64^3 and 100^3, and the branch-free one is faster from 128^3 on (Real
+// 14.7 and 13.8 us, MAC 39.5 and 38.9; at 256^3 244 and 238), but for a Vec3.
+static bool one_wave(const Dims& d) { return d.n < 64 * 64 * 64; }
+
 template <int CH, int OS, int TR>
 static void launch_sl(const Dims& d, CMac vel, const float* src, float* dst, float dt, cudaStream_t s) {
   count_launch();
-  k_sl_cell<CH, OS, TR><<<grid3(d, kBlk), kBlk, 0, s>>>(d, vel, src, dst, dt);
+  const auto k = CH == 1 && !one_wave(d) ? k_sl_cell<CH, OS, TR, CH == 1> : k_sl_cell<CH, OS, TR, false>;
+  k<<<grid3(d, kBlk), kBlk, 0, s>>>(d, vel, src, dst, dt);
 }
 template <int CH, int OS, int TR>
 static void launch_mc(const Dims& d, const int* flags, CMac vel, const float* orig, const float* fwd, float* dst, float dt,
@@ -613,17 +621,16 @@ void launch_advect_maccormack(const Dims& d, int ch, const int* flags, CMac vel,
   else dispatch_mc<3>(d, flags, vel, orig, fwd, dst, dt, strength, clampMode, orderSpace, orderTrace, s);
 }
 
+template <bool kClamp>
+static auto sl_mac(int orderSpace, int orderTrace) {
+  return orderSpace == 1 ? orderTrace == 1 ? k_sl_mac<1, 1, kClamp> : k_sl_mac<2, 1, kClamp>
+                         : orderTrace == 1 ? k_sl_mac<1, 2, kClamp> : k_sl_mac<2, 2, kClamp>;
+}
 void launch_advect_sl_mac(const Dims& d, CMac vel, CMac src, Mac dst, float dt, int orderSpace, int orderTrace,
                          cudaStream_t s) {
   count_launch();
-  const dim3 g = grid3(d, kBlk);
-  if (orderSpace == 1) {
-    if (orderTrace == 1) k_sl_mac<1, 1><<<g, kBlk, 0, s>>>(d, vel, src, dst, dt);
-    else k_sl_mac<2, 1><<<g, kBlk, 0, s>>>(d, vel, src, dst, dt);
-  } else {
-    if (orderTrace == 1) k_sl_mac<1, 2><<<g, kBlk, 0, s>>>(d, vel, src, dst, dt);
-    else k_sl_mac<2, 2><<<g, kBlk, 0, s>>>(d, vel, src, dst, dt);
-  }
+  const auto k = one_wave(d) ? sl_mac<false>(orderSpace, orderTrace) : sl_mac<true>(orderSpace, orderTrace);
+  k<<<grid3(d, kBlk), kBlk, 0, s>>>(d, vel, src, dst, dt);
 }
 
 // the modes that the clamp tells apart: 1, 2 and neither

@@ -114,12 +114,11 @@ __device__ __forceinline__ void clamp_axis(float p, float last, int lastIndex, i
   w1 = c - (float)i;
   w0 = 1.f - w1;
 }
-// kClamp: by clamp_axis, for the MacCormack passes, which instructions bound
-// (with clamps of one instruction a value, a velocity at 256^3 takes 603 us instead
-// of 735).  The passes that wait for their gathers keep the selections, whose index
-// is there earlier and takes fewer registers: first-order advection of a Vec3 at
-// 200^3 takes 103 us with them and 133 without, mapMACToParts of 16 M particles in
-// order 181 and 197, first-order advection of a velocity at 32^3 27.5 and 28.8.
+// kClamp: by clamp_axis, which takes fewer instructions (with clamps of one
+// instruction a value, MacCormack advection of a velocity at 256^3 takes 603 us
+// instead of 735).  By selections the index is there earlier and takes fewer
+// registers: first-order advection of a Vec3 at 200^3 takes 103 us with them and
+// 133 without.
 template <bool kShift, bool kClamp = false>
 __device__ __forceinline__ Wts build_index(const Dims& d, float x, float y, float z) {
   Wts w;

@@ -855,19 +855,25 @@ __global__ void __launch_bounds__(32) k_tile_splat(Tiles s, PartView p, float* v
 // old, flipVelocityUpdate (knMapLinearMACGridToVec3_FLIP, :659-668):
 //   pvel = flipRatio * (pvel + (v - vOld)) + (1.0 - flipRatio) * v
 // where the second product is formed in double and rounded to float.
+// The branch-free index (kClamp): 16 M particles at 128^3 that the flow has mixed
+// take 842 us with it and 960 with selections (FLIP 1678 and 1818), particles in
+// the grid's order 199 and 182 (359 and 342).  A few thousand particles take the
+// selections (4000 at 16^3 5.2 us and 6.2, 20 000 at 32^3 4.3 and 4.7).
+constexpr long long kFewParticles = 1 << 16;
+template <bool kClamp>
 __global__ void k_mac_to_parts(Dims d, PartView p, long long n, CMac vel, CMac old, float flipRatio, float* pu,
                                float* pv, float* pw) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n || part_skip(p, i)) return;
   const float x = p.x[i], y = p.y[i], z = p.z[i];
-  const V3 v = interp_mac<true>(d, vel, x, y, z);
+  const V3 v = interp_mac<true, kClamp>(d, vel, x, y, z);
   if (!old.u) {
     pu[i] = v.x;
     pv[i] = v.y;
     pw[i] = v.z;
     return;
   }
-  const V3 o = interp_mac<true>(d, old, x, y, z);
+  const V3 o = interp_mac<true, kClamp>(d, old, x, y, z);
   const float dlx = v.x - o.x, dly = v.y - o.y, dlz = v.z - o.z;
   const double keep = 1.0 - (double)flipRatio;
   pu[i] = flipRatio * (pu[i] + dlx) + (float)(keep * (double)v.x);
@@ -876,17 +882,19 @@ __global__ void k_mac_to_parts(Dims d, PartView p, long long n, CMac vel, CMac o
 }
 
 // mapGridToParts(Vec3) (knMapFromGrid, flip.cpp:625-631): every active
-// particle, interpol<T> per component
+// particle, interpol<T> per component; by the branch-free index at every count (a
+// Real, 2 M particles at 64^3 in the grid's order: 12.5 us and 13.4 by selections;
+// 200 000 there 4.8 and 4.4; mixed, and below 65 536, alike)
 __global__ void k_grid_to_parts(Dims d, PartView p, long long n, const float* __restrict__ g0,
                                 const float* __restrict__ g1, const float* __restrict__ g2, float* t0, float* t1,
                                 float* t2) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n || (p.flag[i] & kPDelete) != 0) return;
   const float x = p.x[i], y = p.y[i], z = p.z[i];
-  t0[i] = interp(d, g0, x, y, z);
+  t0[i] = interp<true>(d, g0, x, y, z);
   if (g1) {
-    t1[i] = interp(d, g1, x, y, z);
-    t2[i] = interp(d, g2, x, y, z);
+    t1[i] = interp<true>(d, g1, x, y, z);
+    t2[i] = interp<true>(d, g2, x, y, z);
   }
 }
 
@@ -1341,8 +1349,9 @@ static int mac_to_parts(const char* what, mg_grid flags, mg_grid vel, mg_grid ve
   const CMac cv{v, v + d.n, v + 2 * d.n};
   const CMac co = vo ? CMac{vo, vo + d.n, vo + 2 * d.n} : CMac{nullptr, nullptr, nullptr};
   count_launch();
-  k_mac_to_parts<<<blocks_of(parts->n), 256, 0, parts->st>>>(d, view_of(parts, ptype, exclude), parts->n, cv, co,
-                                                              flipRatio, partVel->c[0], partVel->c[1], partVel->c[2]);
+  const auto k = parts->n < kFewParticles ? k_mac_to_parts<false> : k_mac_to_parts<true>;
+  k<<<blocks_of(parts->n), 256, 0, parts->st>>>(d, view_of(parts, ptype, exclude), parts->n, cv, co, flipRatio,
+                                                partVel->c[0], partVel->c[1], partVel->c[2]);
   return launch_status(what);
 }
 
